@@ -219,7 +219,7 @@ bf_status bf_graph_info_get(const bf_graph* h, bf_graph_info* o) {
   o->n_down = g.n_down;
   o->max_depth = g.max_depth;
   o->k_lanes = g.k_lanes;
-  o->device_bytes = g.device_bytes;
+  o->device_bytes = g.device_bytes + g.panels.bytes;
   return BF_OK;
 }
 
@@ -405,7 +405,18 @@ bf_status bf_schedule_levels(const bf_graph* h, uint32_t cap, uint64_t* items, u
     set_error("bf_schedule_levels: null argument");
     return BF_ERR_INVALID;
   }
-  const Sched& sc = h->g.ctx.sc;
+  // (a panel schedule's tables are computed when asked for: the device work
+  // and the schedule belong to the graph, under its lock)
+  Graph* g = const_cast<Graph*>(&h->g);
+  std::lock_guard<std::mutex> lk(g->mu);
+  Sched& sc = g->ctx.sc;
+  if (sc.valid && sc.panel && sc.lvl_item.empty()) {
+    if (cudaSetDevice(g->device) != cudaSuccess)
+      return cuda_status(cudaGetLastError(), "cudaSetDevice");
+    bf_status rc = schedule_tables(g, g->ctx, sc, g->stream);
+    if (rc == BF_OK) rc = check_device_error(g, g->stream);
+    if (rc) return rc;
+  }
   if (!sc.valid || sc.lvl_item.size() < 2 || sc.lvl_row.size() != sc.lvl_item.size() ||
       sc.lvl_edge.size() != sc.lvl_item.size()) {
     set_error("bf_schedule_levels: no target-restricted schedule built yet");

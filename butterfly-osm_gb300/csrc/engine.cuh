@@ -140,8 +140,35 @@ constexpr uint32_t PLAIN_K = 32;
 constexpr uint32_t UPWARD_SMEM_PATH = 2048;
 constexpr uint32_t UPWARD_WARPS = 4;
 
+// Panels of the pull DAG (panel.cu): up to 16 consecutive ranks of one run with
+// their in-edges as a dense weight tile over a list of source ranks.
+constexpr uint32_t PANEL_ROWS = 16;
+struct Panels {
+  uint32_t n = 0;                   // panels (0: none built)
+  uint32_t n_levels = 0;            // levels of the panel DAG
+  uint64_t max_label = 0;           // bound on every finite label of a sweep
+  std::vector<uint32_t> lvl_first;  // level -> first panel, n_levels + 1
+  uint4* d_a = nullptr;             // {highest rank, rows | stride << 8 | bucket << 16,
+                                    //  sources, level}
+  uint2* d_b = nullptr;             // {first source, first weight}
+  uint32_t* d_of = nullptr;         // [n] highest rank -> panel
+  uint32_t* d_hibits = nullptr;     // [n bits] highest ranks of panels
+  uint32_t* d_src = nullptr;        // source ranks
+  uint32_t* d_w = nullptr;          // tiles [source][row], then triangles [row][row]
+  uint64_t bytes = 0;
+};
+
 // A sweep schedule (target-restricted or full graph) with its cached CUDA graph.
 struct Sched {
+  // panel form (panel.cu): items of each level, rows in rank order; the work
+  // items and edge records below are then not built
+  bool panel = false;
+  bool fell_back = false;           // built as items: the budget holds no panel rows
+  std::vector<uint32_t> lvl_pan;    // level -> first panel item
+  uint4* d_pitem = nullptr;         // [2 per item]
+  size_t cap_pitem = 0;
+  bool counted = false;             // n_live / n_edges hold the rows that reach a target
+  uint32_t n_live = 0;
   bool valid = false;
   uint64_t key = 0;              // hash of the targets and split settings (a pre-check)
   std::vector<uint32_t> tgt;     // the targets the schedule was built for (compared exactly)
@@ -171,6 +198,7 @@ struct Sched {
   bool g_pdl = false;
   const uint32_t* g_hub = nullptr;
   bool g_hinted = false;
+  bool g_sat = false;
   // captured single-lane bounded sweep (full schedule), with its geometry
   cudaGraphExec_t one_exec = nullptr;
   const void* one_slab = nullptr;
@@ -201,6 +229,8 @@ struct Sched {
 
 struct SchedScratch;  // device schedule builder scratch (schedule.cu)
 void free_sched_scratch(SchedScratch* s);
+struct PanelScratch;  // panel schedule builder scratch (panel.cu)
+void free_panel_scratch(PanelScratch* s);
 
 // Execution context of the batched engine: schedules, the distance slab and
 // scratch of one in-flight computation. The C-ABI calls use the graph's
@@ -229,6 +259,9 @@ struct Ctx {
   void* h_stage = nullptr;         // page-locked staging arena for schedule uploads
   size_t stage_bytes = 0;
   SchedScratch* sd = nullptr;      // device schedule builder scratch
+  PanelScratch* ps = nullptr;      // panel schedule builder scratch
+  cudaStream_t cnt = nullptr;      // side stream: exact row counts of a panel schedule
+  cudaEvent_t cnt_fork = nullptr;
   // level program of the persistent isochrone sweep (full schedule)
   std::vector<uint2> iso_prog;
   uint2* d_iso_prog = nullptr;
@@ -286,6 +319,8 @@ struct Graph {
   std::vector<uint32_t> pos_of;     // rank -> slab position (plain engine)
   std::vector<uint32_t> lvl_start;  // level -> first position, n_levels + 1
   std::vector<uint32_t> rank_at;    // slab position -> rank
+
+  Panels panels;                    // blocked pull DAG of the matrix sweeps
 
   // device: elimination tree / upward
   uint32_t* d_parent = nullptr;   // [n] etree parent rank (NONE at roots)
@@ -448,16 +483,36 @@ __global__ void k_extract(const uint32_t* __restrict__ slab, uint32_t slab_strid
 
 // engine_batched.cu
 bf_status batched_prepare(Graph* g, uint32_t split_edges);
+// items: the caller reads work items and edge records (else a restricted
+// schedule may come in the panel form, which only sweep_levels reads).
 bf_status build_schedule(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt, uint64_t T, bool all,
-                         cudaStream_t st, const uint32_t* d_tgt = nullptr);
+                         cudaStream_t st, const uint32_t* d_tgt = nullptr, bool items = false);
+// panel.cu
+bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
+                       const std::vector<uint64_t>& off, const std::vector<uint32_t>& src,
+                       const std::vector<uint32_t>& w, uint64_t max_up);
+void free_panels(Panels& P);
+bf_status build_schedule_panels(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt,
+                                const uint32_t* d_tgt, uint64_t T, uint64_t key, cudaStream_t st);
+bool panels_saturate(const Graph* g, uint64_t max_seed);
+cudaError_t sweep_panels(Graph* g, Sched& sc, uint32_t* slab, uint32_t Kp, unsigned tpb, bool sat,
+                         cudaStream_t st, uint64_t* launches, const uint32_t* seeded);
 // schedule.cu: the target-restricted schedule of h_tgt (host) / d_tgt (the
 // same targets on the device, or null) built on the device
 bf_status build_schedule_device(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt,
                                 const uint32_t* d_tgt, uint64_t T, uint64_t key, cudaStream_t st);
+// Rows and edges that reach the schedule's targets (a panel schedule sweeps a
+// few more), counted on the context's side stream from here; finish_counts
+// waits for them and stores them in the schedule.
+bf_status start_counts(Graph* g, Ctx& c, Sched& sc, const uint32_t* d_tgt, uint64_t T,
+                       cudaStream_t st);
+bf_status finish_counts(Graph* g, Ctx& c, Sched& sc);
+// Per-level item, edge and row tables of a schedule in the panel form.
+bf_status schedule_tables(Graph* g, Ctx& c, Sched& sc, cudaStream_t st);
 bf_status hub_rows_device(Graph* g, Sched& sc, uint32_t H, cudaStream_t st);
 bf_status sweep_levels(Graph* g, Sched& sc, uint32_t* slab, uint32_t Kp, unsigned lane_blocks,
                        unsigned tpb, cudaStream_t st, uint64_t* launches,
-                       const uint32_t* seeded);
+                       const uint32_t* seeded, uint64_t max_seed = 0);
 // Reset the slab for a wave and mark its seeded rows (the ancestor paths of
 // the wave's sources) so the sweep reads a row's old value only when seeded.
 void launch_mark_paths(Graph* g, const uint32_t* d_src, uint64_t k, const uint32_t* cidx,

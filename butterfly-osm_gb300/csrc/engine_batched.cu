@@ -120,7 +120,10 @@ __global__ void k_scatter_pairs(const uint2* __restrict__ pr, uint64_t m,
 // map is patched in place: entries of the previous schedule are reset to
 // NONE and the new ones set.
 bf_status build_schedule(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt, uint64_t T, bool all,
-                         cudaStream_t st, const uint32_t* d_tgt) {
+                         cudaStream_t st, const uint32_t* d_tgt, bool want_items) {
+  // restricted schedules are built on the device unless turned off: as panels
+  // (panel.cu) where the caller only sweeps, else as items (schedule.cu)
+  const bool panels = !all && T && g->tune.dev_sched && g->panels.n && !want_items;
   const uint32_t SPLIT = std::max<uint32_t>(1, g->tune.split);
   const uint32_t SMALL_ROWS = g->tune.small_rows;
   const uint32_t SMALL_SPLIT = std::max<uint32_t>(1, std::min(SPLIT, g->tune.small_split));
@@ -128,7 +131,7 @@ bf_status build_schedule(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt, uin
                        ((uint64_t)SPLIT << 56) ^ ((uint64_t)SMALL_SPLIT << 48) ^
                        ((uint64_t)SMALL_ROWS << 20);
   // reuse only for the same split settings and exactly the same targets
-  if (sc.valid && sc.key == key && sc.T == T &&
+  if (sc.valid && sc.key == key && sc.T == T && (sc.panel || sc.fell_back) == panels &&
       (all || (sc.tgt.size() == T && (T == 0 || std::memcmp(sc.tgt.data(), h_tgt, T * 4) == 0)))) {
     ++sc.uses;
     return BF_OK;
@@ -143,8 +146,19 @@ bf_status build_schedule(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt, uin
     cudaGraphExecDestroy(sc.one_exec);
     sc.one_exec = nullptr;
   }
-  // restricted schedules are built on the device (schedule.cu) unless turned
-  // off; the totals it reads back carry edges in 32 bits
+  sc.fell_back = false;
+  if (panels) {
+    bf_status s = build_schedule_panels(g, c, sc, h_tgt, d_tgt, T, key, st);
+    if (s) return s;
+    // a budget that holds 32 lanes of the rows that reach a target, but not
+    // of the somewhat more rows of the panels: sweep the former
+    if (ctx_budget(g, c) / ((uint64_t)std::max<uint32_t>(sc.n_r, 1) * 4 + T * 8) >= 32)
+      return BF_OK;
+    sc.valid = false;
+    sc.fell_back = true;
+  }
+  sc.panel = false;
+  // the totals the item builder reads back carry edges in 32 bits
   if (!all && T && g->tune.dev_sched && g->n_down < 0xFFFFFFFFull)
     return build_schedule_device(g, c, sc, h_tgt, d_tgt, T, key, st);
   sc.dev_built = false;
@@ -571,12 +585,13 @@ __global__ void __launch_bounds__(128)
 // Reset to INF the rows that are read before being fully written: rows that
 // get seeds (seeded bits), rows without in-edges and rows whose in-edges are
 // split over items (combined by atomicMin). All other rows are fully written
-// by the sweep before anything reads them. One block per 32-row group.
+// by the sweep before anything reads them (of a panel schedule: all rows, so
+// split is null). One block per 32-row group.
 __global__ void __launch_bounds__(256)
     k_init_rows(const uint32_t* __restrict__ seeded, const uint32_t* __restrict__ split,
                 uint32_t words, uint32_t* __restrict__ slab, uint32_t Kp) {
   for (uint32_t gw = blockIdx.x; gw < words; gw += gridDim.x) {
-    uint32_t m = seeded[gw] | split[gw];
+    uint32_t m = seeded[gw] | (split ? split[gw] : 0u);
     while (m) {
       const uint32_t b = __ffs(m) - 1;
       m &= m - 1;
@@ -605,7 +620,7 @@ __global__ void __launch_bounds__(128)
   if (threadIdx.x != 0) return;
   const uint32_t sa = static_cast<uint32_t>(__cvta_generic_to_shared(infbuf));
   for (uint32_t gw = blockIdx.x; gw < words; gw += gridDim.x) {
-    uint32_t m = seeded[gw] | split[gw];
+    uint32_t m = seeded[gw] | (split ? split[gw] : 0u);
     while (m) {
       const uint32_t b = __ffs(m) - 1;
       m &= m - 1;
@@ -694,7 +709,7 @@ uint64_t ctx_budget(Graph* g, Ctx& c) {
 
 static void free_sched(Sched& sc) {
   void* p[] = {sc.d_cidx, sc.d_item, sc.d_erec, sc.d_elen, sc.d_trow, sc.d_split, sc.d_hub,
-               sc.d_lvl, sc.d_uses, sc.d_hub_h, sc.d_lvl_erec};
+               sc.d_lvl, sc.d_uses, sc.d_hub_h, sc.d_lvl_erec, sc.d_pitem};
   for (void* q : p)
     if (q) cudaFree(q);
   if (sc.gexec) cudaGraphExecDestroy(sc.gexec);
@@ -715,6 +730,9 @@ void free_ctx(Ctx& c) {
   if (c.d_count) cudaFree(c.d_count);
   if (c.h_stage) cudaFreeHost(c.h_stage);
   free_sched_scratch(c.sd);
+  free_panel_scratch(c.ps);
+  if (c.cnt_fork) cudaEventDestroy(c.cnt_fork);
+  if (c.cnt) cudaStreamDestroy(c.cnt);
   for (auto& e : c.ev)
     if (e) cudaEventDestroy(e);
   if (c.fork) cudaEventDestroy(c.fork);
@@ -726,6 +744,8 @@ void free_ctx(Ctx& c) {
 bf_status init_ctx(Ctx& c) {
   for (auto& e : c.ev) BF_CUDA(cudaEventCreate(&e));
   BF_CUDA(cudaStreamCreateWithFlags(&c.aux, cudaStreamNonBlocking));
+  BF_CUDA(cudaStreamCreateWithFlags(&c.cnt, cudaStreamNonBlocking));
+  BF_CUDA(cudaEventCreateWithFlags(&c.cnt_fork, cudaEventDisableTiming));
   BF_CUDA(cudaEventCreateWithFlags(&c.fork, cudaEventDisableTiming));
   BF_CUDA(cudaEventCreateWithFlags(&c.join, cudaEventDisableTiming));
   return BF_OK;
@@ -766,15 +786,17 @@ bf_status hub_rows(Graph* g, Sched& sc, uint64_t row_bytes, cudaStream_t st, con
 // CUDA graph instead of being issued one by one.
 bf_status sweep_levels(Graph* g, Sched& sc, uint32_t* slab, uint32_t Kp, unsigned lane_blocks,
                        unsigned tpb, cudaStream_t st, uint64_t* launches,
-                       const uint32_t* seeded) {
+                       const uint32_t* seeded, uint64_t max_seed) {
   const bool pdl = g->tune.pdl != 0;
+  const bool sat = sc.panel && panels_saturate(g, max_seed);
   // cache hints only pay when the slab is well beyond L2 (otherwise
   // evict-first would drop lines that the sweep reads again)
-  const bool hinted = (uint64_t)std::max<uint32_t>(sc.n_r, 1) * Kp * 4 > 4 * g->l2_bytes;
+  const bool hinted = !sc.panel && (uint64_t)std::max<uint32_t>(sc.n_r, 1) * Kp * 4 > 4 * g->l2_bytes;
   const uint32_t* hub = nullptr;
   bf_status hs;
   if (hinted && (hs = hub_rows(g, sc, (uint64_t)Kp * 4, st, &hub))) return hs;
   auto issue = [&](cudaStream_t s, uint64_t* count) -> cudaError_t {
+    if (sc.panel) return sweep_panels(g, sc, slab, Kp, tpb, sat, s, count, seeded);
     for (uint32_t l = 0; l < g->n_levels; ++l) {
       const uint32_t i0 = sc.lvl_item[l], i1 = sc.lvl_item[l + 1];
       if (i1 == i0) continue;
@@ -788,7 +810,7 @@ bf_status sweep_levels(Graph* g, Sched& sc, uint32_t* slab, uint32_t Kp, unsigne
   };
   const bool geom = sc.g_kp == Kp && sc.g_lb == lane_blocks && sc.g_tpb == tpb &&
                     sc.g_slab == slab && sc.g_stream == st && sc.g_seeded == seeded &&
-                    sc.g_pdl == pdl && sc.g_hub == hub && sc.g_hinted == hinted;
+                    sc.g_pdl == pdl && sc.g_hub == hub && sc.g_hinted == hinted && sc.g_sat == sat;
   if (sc.gexec && !geom) {
     cudaGraphExecDestroy(sc.gexec);
     sc.gexec = nullptr;
@@ -819,12 +841,14 @@ bf_status sweep_levels(Graph* g, Sched& sc, uint32_t* slab, uint32_t Kp, unsigne
       sc.g_pdl = pdl;
       sc.g_hub = hub;
       sc.g_hinted = hinted;
+      sc.g_sat = sat;
     }
   }
   if (sc.gexec && g->tune.graphs) {
     BF_CUDA(cudaGraphLaunch(sc.gexec, st));
-    for (uint32_t l = 0; l < g->n_levels; ++l)
-      if (sc.lvl_item[l + 1] != sc.lvl_item[l]) ++*launches;
+    const std::vector<uint32_t>& first = sc.panel ? sc.lvl_pan : sc.lvl_item;
+    for (size_t l = 0; l + 1 < first.size(); ++l)
+      if (first[l + 1] != first[l]) ++*launches;
   } else {
     BF_CUDA(issue(st, launches));
   }
@@ -884,7 +908,7 @@ bf_status prepare_rows(Graph* g, Ctx& c, Sched& sc, const uint32_t* d_src, uint6
   // only rows the sweep does not overwrite whole need INF first (seeded,
   // split and in-edge-free rows; 10k x 10k: 2.8 against 3.5 ms for a reset
   // of the whole slab beside the upward pass)
-  launch_init_rows(c.d_seeded, sc.d_split, words, c.d_slab, Kp, st);
+  launch_init_rows(c.d_seeded, sc.panel ? nullptr : sc.d_split, words, c.d_slab, Kp, st);
   BF_CUDA(cudaGetLastError());
   *launches += 2;
   return BF_OK;
@@ -929,7 +953,7 @@ bf_status batched_wave(Graph* g, Ctx& c, const uint32_t* d_src, uint64_t kw, uin
     // only rows the sweep does not overwrite whole need INF first: seeded
     // rows (read back by their item), split rows (atomicMin targets) and rows
     // without in-edges (read, never written) - sc.d_split marks the last two
-    launch_init_rows(c.d_seeded, sc.d_split, words, c.d_slab, Kp, st);
+    launch_init_rows(c.d_seeded, sc.panel ? nullptr : sc.d_split, words, c.d_slab, Kp, st);
     BF_CUDA(cudaStreamWaitEvent(st, c.join, 0));
     if ((s = launch_scatter_seeds(g, c.d_cseed, kw, d_src, c.d_slab, Kp, st,
                                   pre_stride ? pre_stride : kw, pre_col, sc.d_cidx)))
@@ -982,6 +1006,7 @@ bf_status batched_matrix(Graph* g, Ctx& c, const uint32_t* d_src, uint64_t S, co
     stats->schedule_ms +=
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tb).count();
   Sched& sc = c.sc;
+  if (stats && (s = start_counts(g, c, sc, d_tgt, T, st))) return s;
   const uint64_t rows = std::max<uint32_t>(sc.n_r, 1);
   // lanes per wave: all sources if the slab fits the budget, else waves
   uint64_t max_lanes = ctx_budget(g, c) / (rows * 4);
@@ -1020,9 +1045,10 @@ bf_status batched_matrix(Graph* g, Ctx& c, const uint32_t* d_src, uint64_t S, co
     }
   }
   if (stats) {
+    if ((s = finish_counts(g, c, sc))) return s;
     stats->n_batches += (S + wave - 1) / wave;
     stats->waves += (S + wave - 1) / wave;
-    stats->swept_nodes = sc.n_r;
+    stats->swept_nodes = sc.n_live;
     stats->swept_edges = sc.n_edges;
     stats->lanes = Kp;
     stats->kernel_launches += launches;

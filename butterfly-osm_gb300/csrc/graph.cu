@@ -18,6 +18,7 @@
 //     sources of v's DOWN in-edges) and a slab position per node, ordered by
 //     (level, rank), so every level is a contiguous position range.
 //   * the pull CSR (DownReverseAdjFlat) re-indexed by slab position.
+//   * the panels of the pull DAG (panel.cu).
 
 #include <algorithm>
 #include <cstring>
@@ -282,6 +283,17 @@ static bf_status build_graph_impl(const bf_cch_csr* csr, const bf_config* cfg, G
       up_rec[p++] = make_uint2(depth[u] - depth[v], w);
     }
   }
+  // the longest UP path (a bound on every seed of a sweep), for the panels
+  uint64_t max_up = 0;
+  {
+    std::vector<uint64_t> up(n, 0);
+    for (uint32_t u = n; u-- > 0;) {
+      for (uint64_t k = uo[u]; k < uo[u + 1]; ++k)
+        if (csr->up_weights[k] != INF)
+          up[u] = std::max(up[u], up[csr->up_targets[k]] + csr->up_weights[k]);
+      max_up = std::max(max_up, up[u]);
+    }
+  }
   last_src.clear();
   last_src.shrink_to_fit();
   rec_at.clear();
@@ -354,6 +366,7 @@ static bf_status build_graph_impl(const bf_cch_csr* csr, const bf_config* cfg, G
   if ((s = dev_upload(&g->d_lvl_start, g->lvl_start.data(), g->lvl_start.size(), g))) return s;
   uint32_t zero = 0;
   if ((s = dev_upload(&g->d_err, &zero, 1, g))) return s;
+  if ((s = build_panels(g, run_end, in_off_r, in_src_r, in_w_r, max_up))) return s;
   g->rank_at = std::move(rank_at);
   g->h_in_off = std::move(in_off);
   g->h_in_rec = std::move(in_rec);
@@ -374,6 +387,7 @@ void free_graph(Graph* g) {
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (g->h_set_stage) cudaFreeHost(g->h_set_stage);
+  free_panels(g->panels);
   free_ctx(g->ctx);
   for (auto& e : g->ev)
     if (e) cudaEventDestroy(e);

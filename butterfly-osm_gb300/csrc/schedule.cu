@@ -48,9 +48,10 @@ namespace {
 // Peeling rounds at most (10 000 targets on the country graph take 38).
 constexpr uint32_t PEEL_ROUNDS = 4096;
 // meta words: three rotating frontier sizes, the row count, the candidate
-// count, peeling rounds run and frontier left, the grid-barrier words
+// count, peeling rounds run and frontier left, the grid-barrier words, the
+// totals of start_counts (two 64-bit counters)
 constexpr uint32_t META_NR = 3, META_NC = 4, META_ROUNDS = 5, META_LEFT = 6, META_BAR = 8,
-                   META_WORDS = 16;
+                   META_TOT = 12, META_WORDS = 16;
 constexpr uint32_t HUB_BINS = 65536;
 
 // Grow a device array to `need` elements (1/8 more with `slack`: arrays
@@ -578,6 +579,8 @@ struct SchedScratch {
   size_t cap_alive = 0, cap_ist = 0, cap_cnt = 0, cap_front = 0, cap_wpre = 0, cap_rowpos = 0,
          cap_rdeg = 0, cap_rpre = 0, cap_b64 = 0, cap_b32 = 0, cap_lvlrow = 0, cap_lvli = 0,
          cap_hist = 0, cap_meta = 0, cap_tgt = 0, cap_clist = 0;
+  unsigned long long* h_counts = nullptr;  // page-locked: rows and edges of start_counts
+  bool counting = false;      // start_counts has work on the side stream
   unsigned peel_blocks = 0;  // co-resident blocks of the peeling launch
   size_t back_words = 0;
 };
@@ -589,17 +592,17 @@ void free_sched_scratch(SchedScratch* s) {
   for (void* q : p)
     if (q) cudaFree(q);
   if (s->h_back) cudaFreeHost(s->h_back);
+  if (s->h_counts) cudaFreeHost(s->h_counts);
   delete s;
 }
 
-bf_status build_schedule_device(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt,
-                                const uint32_t* d_tgt, uint64_t T, uint64_t key,
-                                cudaStream_t st) {
-  const uint32_t n = g->n, L = g->n_levels;
-  const uint32_t W = (n + 31) / 32;
-  const uint32_t SPLIT = std::max<uint32_t>(1, g->tune.split);
-  const uint32_t SMALL_SPLIT = std::max<uint32_t>(1, std::min(SPLIT, g->tune.small_split));
-  SplitCfg cfg{SPLIT, SMALL_SPLIT, g->tune.small_rows, SPLIT + 1};
+namespace {
+
+// Scratch of the row selection (select_rows), and the targets on the device
+// (uploaded when d_tgt is null).
+bf_status select_scratch(Graph* g, Ctx& c, const uint32_t* h_tgt, const uint32_t** d_tgt,
+                         uint64_t T, cudaStream_t st) {
+  const uint32_t n = g->n, W = (n + 31) / 32;
   if (!c.sd) {
     c.sd = new (std::nothrow) SchedScratch();
     if (!c.sd) {
@@ -608,52 +611,29 @@ bf_status build_schedule_device(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_t
     }
   }
   SchedScratch& s = *c.sd;
-  const uint64_t nb_rows = (n + SCAN_BLOCK - 1) / SCAN_BLOCK + 1;
-  const uint64_t nb_words = (W + 1 + SCAN_BLOCK - 1) / SCAN_BLOCK + 1;
   bf_status rc;
   if ((rc = ensure_dev(&s.alive, s.cap_alive, W + 1, g)) ||
       (rc = ensure_dev(&s.clist, s.cap_clist, n, g)) ||
       (rc = ensure_dev(&s.ist, s.cap_ist, W + 1, g)) ||
       (rc = ensure_dev(&s.cnt, s.cap_cnt, n, g)) ||
       (rc = ensure_dev(&s.front, s.cap_front, 2 * (size_t)n, g)) ||
-      (rc = ensure_dev(&s.wpre, s.cap_wpre, W + 2, g)) ||
-      (rc = ensure_dev(&s.rowpos, s.cap_rowpos, n, g)) ||
-      (rc = ensure_dev(&s.rdeg, s.cap_rdeg, n, g)) ||
-      (rc = ensure_dev(&s.rpre, s.cap_rpre, (size_t)n + 1, g)) ||
-      (rc = ensure_dev(&s.bsum64, s.cap_b64, nb_rows + 1, g)) ||
-      (rc = ensure_dev(&s.bsum32, s.cap_b32, nb_words + 1, g)) ||
-      (rc = ensure_dev(&s.lvlrow, s.cap_lvlrow, (size_t)L + 1, g)) ||
-      (rc = ensure_dev(&s.lvl_item, s.cap_lvli, (size_t)L + 1, g)) ||
-      (rc = ensure_dev(&s.hist, s.cap_hist, (size_t)L * cfg.s1, g)) ||
-      (rc = ensure_dev(&s.meta, s.cap_meta, META_WORDS, g)) ||
-      (rc = ensure_dev(&sc.d_split, sc.cap_split, (size_t)W + 1, g)) ||
-      (rc = ensure_dev(&sc.d_cidx, sc.cap_cidx, n, g)))
+      (rc = ensure_dev(&s.meta, s.cap_meta, META_WORDS, g)))
     return rc;
-  if (!g->d_lvl_start) {
-    set_error("device schedule: level table missing");
-    return BF_ERR_DEVICE;
-  }
-  const size_t back = 4 + 3 * ((size_t)L + 1);
-  if (back > s.back_words) {
-    if (s.h_back) cudaFreeHost(s.h_back);
-    s.h_back = nullptr;
-    s.back_words = 0;
-    if (cudaHostAlloc((void**)&s.h_back, back * 4, cudaHostAllocDefault) != cudaSuccess) {
-      cudaGetLastError();
-      set_error("cannot allocate the schedule read-back buffer");
-      return BF_ERR_OOM;
-    }
-    s.back_words = back;
-  }
-  if (!d_tgt) {
+  if (!*d_tgt) {
     if ((rc = ensure_dev(&s.tgt, s.cap_tgt, T, g))) return rc;
     if (T) BF_CUDA(cudaMemcpyAsync(s.tgt, h_tgt, T * 4, cudaMemcpyHostToDevice, st));
-    d_tgt = s.tgt;
+    *d_tgt = s.tgt;
   }
+  return BF_OK;
+}
+
+// Steps 1 and 2: the rows that reach a target, as the bitmap s.alive.
+bf_status select_rows(Graph* g, SchedScratch& s, const uint32_t* d_tgt, uint64_t T,
+                      cudaStream_t st) {
+  const uint32_t n = g->n, W = (n + 31) / 32;
   BF_CUDA(cudaMemsetAsync(s.alive, 0, (size_t)(W + 1) * 4, st));
   BF_CUDA(cudaMemsetAsync(s.ist, 0, (size_t)(W + 1) * 4, st));
   BF_CUDA(cudaMemsetAsync(s.meta, 0, META_WORDS * 4, st));
-  BF_CUDA(cudaMemsetAsync(s.hist, 0, (size_t)L * cfg.s1 * 4, st));
   // 1. ancestors of the targets
   uint32_t* d_nc = s.meta + META_NC;
   if (T)
@@ -678,6 +658,74 @@ bf_status build_schedule_device(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_t
                             (const uint2*)g->d_in_rec, s.cnt, s.alive, (const uint32_t*)s.ist,
                             hook ? 2000000ll : BARRIER_TIMEOUT_CYCLES, hook ? 1u : NONE,
                             g->d_err));
+  return BF_OK;
+}
+
+// Live rows and their in-edges, over the candidates.
+__global__ void __launch_bounds__(256)
+    k_sd_totals(const uint32_t* __restrict__ clist, const uint32_t* __restrict__ nc_p,
+                const uint64_t* __restrict__ in_off, const uint32_t* __restrict__ alive,
+                unsigned long long* __restrict__ tot) {
+  const uint32_t nc = *nc_p;
+  unsigned long long rows = 0, edges = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += gridDim.x * blockDim.x) {
+    const uint32_t p = clist[i];
+    if (!bit_of(alive, p)) continue;
+    ++rows;
+    edges += in_off[p + 1] - in_off[p];
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    rows += __shfl_down_sync(0xFFFFFFFFu, rows, o);
+    edges += __shfl_down_sync(0xFFFFFFFFu, edges, o);
+  }
+  if ((threadIdx.x & 31) == 0 && rows) {
+    atomicAdd(&tot[0], rows);
+    atomicAdd(&tot[1], edges);
+  }
+}
+
+// Steps 1 to 3 and the read-back: per-level tables, row and item offsets.
+bf_status compact_schedule(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt,
+                           const uint32_t* d_tgt, uint64_t T, cudaStream_t st) {
+  const uint32_t n = g->n, L = g->n_levels;
+  const uint32_t W = (n + 31) / 32;
+  const uint32_t SPLIT = std::max<uint32_t>(1, g->tune.split);
+  const uint32_t SMALL_SPLIT = std::max<uint32_t>(1, std::min(SPLIT, g->tune.small_split));
+  SplitCfg cfg{SPLIT, SMALL_SPLIT, g->tune.small_rows, SPLIT + 1};
+  bf_status rc;
+  if ((rc = select_scratch(g, c, h_tgt, &d_tgt, T, st))) return rc;
+  SchedScratch& s = *c.sd;
+  const uint64_t nb_rows = (n + SCAN_BLOCK - 1) / SCAN_BLOCK + 1;
+  const uint64_t nb_words = (W + 1 + SCAN_BLOCK - 1) / SCAN_BLOCK + 1;
+  if ((rc = ensure_dev(&s.wpre, s.cap_wpre, W + 2, g)) ||
+      (rc = ensure_dev(&s.rowpos, s.cap_rowpos, n, g)) ||
+      (rc = ensure_dev(&s.rdeg, s.cap_rdeg, n, g)) ||
+      (rc = ensure_dev(&s.rpre, s.cap_rpre, (size_t)n + 1, g)) ||
+      (rc = ensure_dev(&s.bsum64, s.cap_b64, nb_rows + 1, g)) ||
+      (rc = ensure_dev(&s.bsum32, s.cap_b32, nb_words + 1, g)) ||
+      (rc = ensure_dev(&s.lvlrow, s.cap_lvlrow, (size_t)L + 1, g)) ||
+      (rc = ensure_dev(&s.lvl_item, s.cap_lvli, (size_t)L + 1, g)) ||
+      (rc = ensure_dev(&s.hist, s.cap_hist, (size_t)L * cfg.s1, g)) ||
+      (rc = ensure_dev(&sc.d_split, sc.cap_split, (size_t)W + 1, g)))
+    return rc;
+  if (!g->d_lvl_start) {
+    set_error("device schedule: level table missing");
+    return BF_ERR_DEVICE;
+  }
+  const size_t back = 4 + 3 * ((size_t)L + 1);
+  if (back > s.back_words) {
+    if (s.h_back) cudaFreeHost(s.h_back);
+    s.h_back = nullptr;
+    s.back_words = 0;
+    if (cudaHostAlloc((void**)&s.h_back, back * 4, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      set_error("cannot allocate the schedule read-back buffer");
+      return BF_ERR_OOM;
+    }
+    s.back_words = back;
+  }
+  if ((rc = select_rows(g, s, d_tgt, T, st))) return rc;
+  BF_CUDA(cudaMemsetAsync(s.hist, 0, (size_t)L * cfg.s1 * 4, st));
   // 3. compaction
   const unsigned nbw = (unsigned)((W + 1 + SCAN_BLOCK - 1) / SCAN_BLOCK);
   PopVal pv{s.alive};
@@ -718,9 +766,81 @@ bf_status build_schedule_device(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_t
     set_error("device schedule: inconsistent counts");
     return BF_ERR_DEVICE;
   }
+  sc.lvl_item.assign(s.h_back + 4, s.h_back + 4 + L + 1);
+  sc.lvl_row.assign(s.h_back + 4 + (L + 1), s.h_back + 4 + 2 * (L + 1));
+  sc.lvl_edge.assign(s.h_back + 4 + 2 * (L + 1), s.h_back + 4 + 3 * (L + 1));
+  return BF_OK;
+}
+
+}  // namespace
+
+bf_status schedule_tables(Graph* g, Ctx& c, Sched& sc, cudaStream_t st) {
+  bf_status rc = finish_counts(g, c, sc);
+  if (rc) return rc;
+  return compact_schedule(g, c, sc, sc.tgt.data(), nullptr, sc.T, st);
+}
+
+bf_status start_counts(Graph* g, Ctx& c, Sched& sc, const uint32_t* d_tgt, uint64_t T,
+                       cudaStream_t st) {
+  if (!sc.panel) {
+    sc.n_live = sc.n_r;
+    return BF_OK;
+  }
+  if (sc.counted) return BF_OK;
+  bf_status rc;
+  // after the caller's stream (the targets may still be on their way)
+  BF_CUDA(cudaEventRecord(c.cnt_fork, st));
+  BF_CUDA(cudaStreamWaitEvent(c.cnt, c.cnt_fork, 0));
+  if ((rc = select_scratch(g, c, sc.tgt.data(), &d_tgt, T, c.cnt))) return rc;
+  SchedScratch& s = *c.sd;
+  if (!s.h_counts &&
+      cudaHostAlloc((void**)&s.h_counts, 16, cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    s.h_counts = nullptr;
+    set_error("cannot allocate the row-count read-back buffer");
+    return BF_ERR_OOM;
+  }
+  if ((rc = select_rows(g, s, d_tgt, T, c.cnt))) return rc;
+  unsigned long long* tot = reinterpret_cast<unsigned long long*>(s.meta + META_TOT);
+  k_sd_totals<<<152, 256, 0, c.cnt>>>(s.clist, s.meta + META_NC, g->d_in_off, s.alive, tot);
+  BF_CUDA(cudaGetLastError());
+  BF_CUDA(cudaMemcpyAsync(s.h_counts, tot, 16, cudaMemcpyDeviceToHost, c.cnt));
+  s.counting = true;
+  return BF_OK;
+}
+
+bf_status finish_counts(Graph* g, Ctx& c, Sched& sc) {
+  (void)g;
+  if (!c.sd || !c.sd->counting) return BF_OK;
+  c.sd->counting = false;
+  BF_CUDA(cudaStreamSynchronize(c.cnt));
+  sc.n_live = (uint32_t)c.sd->h_counts[0];
+  sc.n_edges = c.sd->h_counts[1];
+  sc.counted = true;
+  return BF_OK;
+}
+
+bf_status build_schedule_device(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt,
+                                const uint32_t* d_tgt, uint64_t T, uint64_t key,
+                                cudaStream_t st) {
+  const uint32_t n = g->n, L = g->n_levels;
+  const uint32_t SPLIT = std::max<uint32_t>(1, g->tune.split);
+  const uint32_t SMALL_SPLIT = std::max<uint32_t>(1, std::min(SPLIT, g->tune.small_split));
+  SplitCfg cfg{SPLIT, SMALL_SPLIT, g->tune.small_rows, SPLIT + 1};
   sc.valid = false;
+  bf_status rc;
+  if ((rc = finish_counts(g, c, sc)) || (rc = compact_schedule(g, c, sc, h_tgt, d_tgt, T, st)))
+    return rc;
+  SchedScratch& s = *c.sd;
+  if (!d_tgt) d_tgt = s.tgt;
+  uint32_t* d_nr = s.meta + META_NR;
+  const uint32_t n_r = s.h_back[0];
+  uint64_t tot;
+  std::memcpy(&tot, s.h_back + 1, 8);
+  const uint64_t n_e = tot & 0xFFFFFFFFull, n_i = tot >> 32;
   const bool two = g->has_len;
-  if ((rc = ensure_dev(&sc.d_item, sc.cap_items, n_i, g, true)) ||
+  if ((rc = ensure_dev(&sc.d_cidx, sc.cap_cidx, n, g)) ||
+      (rc = ensure_dev(&sc.d_item, sc.cap_items, n_i, g, true)) ||
       (rc = ensure_dev(&sc.d_erec, sc.cap_edges, n_e + 2, g, true)) ||
       (two && (rc = ensure_dev(&sc.d_elen, sc.cap_elen, n_e, g, true))) ||
       (rc = ensure_dev(&sc.d_trow, sc.cap_t, T, g, true)) ||
@@ -740,9 +860,6 @@ bf_status build_schedule_device(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_t
   BF_CUDA(cudaMemcpyAsync(sc.d_lvl, s.lvl_item, ((size_t)L + 1) * 4, cudaMemcpyDeviceToDevice,
                           st));
   BF_CUDA(cudaGetLastError());
-  sc.lvl_item.assign(s.h_back + 4, s.h_back + 4 + L + 1);
-  sc.lvl_row.assign(s.h_back + 4 + (L + 1), s.h_back + 4 + 2 * (L + 1));
-  sc.lvl_edge.assign(s.h_back + 4 + 2 * (L + 1), s.h_back + 4 + 3 * (L + 1));
   sc.n_r = n_r;
   sc.n_items = n_i;
   sc.n_edges = n_e;

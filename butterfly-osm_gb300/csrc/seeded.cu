@@ -171,6 +171,12 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
   tr.erase(std::unique(tr.begin(), tr.end()), tr.end());
   if ((rc = build_schedule(g, c, c.sc, tr.data(), tr.size(), false, s))) return rc;
   Sched& sc = c.sc;
+  if (st) {
+    const uint32_t* none = nullptr;
+    if ((rc = start_counts(g, c, sc, none, nt ? tr.size() : 0, s))) return rc;
+  }
+  uint64_t max_seed = 0;
+  for (uint64_t k = 0; k < ns; ++k) max_seed = std::max<uint64_t>(max_seed, src_seeds[k].cost);
   const uint64_t rows = std::max<uint32_t>(sc.n_r, 1);
   uint64_t max_lanes = ctx_budget(g, c) / (rows * 4 + (uint64_t)T * 4 * 2);
   max_lanes = max_lanes >= 32 ? max_lanes & ~31ull : 0;
@@ -212,7 +218,8 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
         return rc;
       ++launches;
     }
-    if ((rc = sweep_levels(g, sc, c.d_slab, Kp, lane_blocks, tpb, s, &launches, c.d_seeded)))
+    if ((rc = sweep_levels(g, sc, c.d_slab, Kp, lane_blocks, tpb, s, &launches, c.d_seeded,
+                           max_seed)))
       return rc;
     dim3 eg((unsigned)((T + 31) / 32), (unsigned)((kw + 31) / 32)), eb(32, 8);
     k_seeded_extract<<<eg, eb, 0, s>>>(c.d_slab, Kp, sc.d_cidx, d_to.as<uint64_t>(),
@@ -242,10 +249,11 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
   if (n_conflicts) *n_conflicts = cells.size();
   for (uint64_t i = 0; i < cells.size() && i < conflict_cap; ++i) conflicts[i] = cells[i];
   if (st) {
+    if ((rc = finish_counts(g, c, sc))) return rc;
     st->n_batches += (S + wave - 1) / wave;
     st->waves += (S + wave - 1) / wave;
     st->kernel_launches += launches;
-    st->swept_nodes = sc.n_r;
+    st->swept_nodes = sc.n_live;
     st->swept_edges = sc.n_edges;
     st->lanes = Kp;
   }

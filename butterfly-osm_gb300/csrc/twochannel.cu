@@ -401,7 +401,7 @@ bf_status matrix_seeded_2ch(Graph* g, Ctx& c, const bf_seed2* src_seeds, const u
   for (uint64_t k = 0; k < nt; ++k) tr[k] = tgt_seeds[k].rank;
   std::sort(tr.begin(), tr.end());
   tr.erase(std::unique(tr.begin(), tr.end()), tr.end());
-  if ((rc = build_schedule(g, c, c.sc, tr.data(), tr.size(), false, s))) return rc;
+  if ((rc = build_schedule(g, c, c.sc, tr.data(), tr.size(), false, s, nullptr, true))) return rc;
   Sched& sc = c.sc;
   const uint64_t rows = std::max<uint32_t>(sc.n_r, 1);
   uint64_t max_lanes = ctx_budget(g, c) / (rows * 8 + (uint64_t)T * 4 * 2 * 2);

@@ -228,8 +228,9 @@ bf_status bf_autotune_isochrones(bf_graph* g, const uint32_t* d_origins,
 
 /* Per level of the last target-restricted schedule of the graph's C-ABI
  * matrix calls: work items, edge records and rows (first min(cap, levels)
- * entries; *n_levels = levels). For profiling: the k-th launch of a sweep
- * processes the k-th level with items. No reference counterpart. */
+ * entries; *n_levels = levels), of the schedule as work items. A schedule
+ * swept as panels (fewer levels, each a launch) has its table computed by
+ * this call. No reference counterpart. */
 bf_status bf_schedule_levels(const bf_graph* g, uint32_t cap, uint64_t* items, uint64_t* edges,
                              uint64_t* rows, uint32_t* n_levels);
 

@@ -1,0 +1,125 @@
+"""Panel sweeps (up to 16 consecutive ranks of one run swept as a dense tile)
+against the CPU oracle and the item sweep (tolerance 0: u32 min-plus), at the
+edges of panels, of weight-tile strides, of staged source chunks and of lane
+blocks, and with labels beyond the one-instruction relaxation's range."""
+import numpy as np
+import pytest
+
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+INF = 0xFFFFFFFF
+
+
+def _cch(n, up, seed, w_lo, w_hi, drop):
+    """CCH from UP neighbour lists; every edge also goes DOWN with its own
+    weight, each direction dropped (INF) with probability `drop`, except the
+    steps r -> r + 1 that make the runs."""
+    rng = np.random.default_rng(seed)
+    src = np.array([u for u in range(n) for _ in up[u]], np.int64)
+    tgt = np.array([v for u in range(n) for v in up[u]], np.int64)
+    w = rng.integers(w_lo, w_hi, (2, len(src)), dtype=np.uint64)
+    w[:, (rng.random(len(src)) < drop) & (tgt != src + 1)] = INF
+    lone = rng.random((2, len(src))) < drop
+    lone[:, tgt == src + 1] = False
+    w[lone] = INF
+    off = np.zeros((2, n + 1), np.uint64)
+    off[0, 1:] = np.cumsum(np.bincount(src, minlength=n))
+    off[1, 1:] = np.cumsum(np.bincount(tgt, minlength=n))
+    o = np.lexsort((src, tgt))
+    return dict(n=n, up_off=off[0], up_tgt=tgt.astype(np.uint32), up_w=w[0].astype(np.uint32),
+                down_off=off[1], down_tgt=src[o].astype(np.uint32),
+                down_w=w[1][o].astype(np.uint32))
+
+
+def _band(n, width):
+    """One run of n ranks, each joined to the next `width`."""
+    return [list(range(u + 1, min(n, u + 1 + width))) for u in range(n)]
+
+
+def _fan():
+    """A run whose 16 rows pull from disjoint ancestors (its tile is split),
+    under a run of 700 ranks."""
+    up = [[u + 1] + list(range(16 + 40 * u, 56 + 40 * u)) for u in range(16)]
+    up[15] = sorted(set(up[15]))
+    return [sorted(set(x)) for x in up] + [
+        list(range(u + 1, min(716, u + 4))) for u in range(16, 716)]
+
+
+GRAPHS = {
+    # run lengths at and beside the panel and stride edges
+    **{"band%d" % n: (_band(n, n), 1, 60) for n in (1, 2, 3, 5, 9, 13, 16, 17, 33)},
+    "sources300": (_band(330, 330), 1, 1000),  # over 256 sources above a panel
+    "fan": (_fan(), 1, 500),
+    # labels up to and past 2^31, and sums that saturate
+    "long": (_band(40, 12), 1 << 26, 1 << 28),
+    "saturating": (_band(40, 12), 1 << 29, 0xFFFFFFF0),
+}
+
+
+@pytest.mark.parametrize("name", sorted(GRAPHS))
+def test_panels_small_graphs(built, name):
+    import bfphast
+    up, lo, hi = GRAPHS[name]
+    n = len(up)
+    cch = _cch(n, up, 7, lo, hi, 0.2)
+    c = orc.Cch.from_dict(cch)
+    g, items = bfphast.Graph.from_cch(cch), bfphast.Graph.from_cch(cch)
+    items.set_tune(device_schedule=0)
+    rng = np.random.default_rng(n)
+    for S, T in ((1, 1), (4, n), (33, 5), (65, n), (129, 3), (600, n)):
+        src = rng.integers(0, n, S).astype(np.uint32)
+        tgt = rng.integers(0, n, T).astype(np.uint32)
+        want, _ = c.matrix(src, tgt)
+        got, st = g.matrix(src, tgt, stats=True)
+        assert np.array_equal(got, want), (S, T)
+        ref, si = items.matrix(src, tgt, stats=True)
+        assert np.array_equal(ref, want), (S, T)
+        assert (st["swept_nodes"], st["swept_edges"]) == (si["swept_nodes"], si["swept_edges"])
+        sets = [[(int(s), int(rng.integers(0, 1 << 31)))] for s in src[:9]]
+        tsets = [[(int(t), 0)] for t in tgt[:9]]
+        got = g.matrix_seeded(sets, tsets)  # seed costs past the short range
+        assert np.array_equal(got, orc.table_phast_lopsided(c, sets, tsets, INF)[0]), (S, T)
+
+
+@pytest.mark.parametrize("S", [130, 512, 516, 1030])
+def test_panels_wide_levels(built, grid100, S):
+    """Every node a target: levels of thousands of panels, lane blocks of 512
+    and what is left of them, every block size."""
+    import bfphast
+    _, cch = grid100
+    n = cch["n"]
+    g = bfphast.Graph.from_cch(cch)
+    rng = np.random.default_rng(S)
+    src = rng.integers(0, n, S).astype(np.uint32)
+    tgt = np.arange(n, dtype=np.uint32)
+    pick = rng.choice(S, 12, replace=False)
+    c = orc.Cch.from_dict(cch)
+    want = np.stack([c.phast_query(int(s)) for s in src[pick]])
+    for tpb in (32, 64, 128, 256):
+        g.set_tune(threads_per_block=tpb)
+        assert np.array_equal(g.matrix(src, tgt)[pick], want), tpb
+
+
+def test_panels_budget_falls_back_to_items(built, country_small):
+    """A budget for 32 lanes of the rows that reach a target, but not of the
+    targets' ancestors, is still served (by the item sweep)."""
+    import bfphast
+    _, cch = country_small
+    n = cch["n"]
+    c = orc.Cch.from_dict(cch)
+    rng = np.random.default_rng(2)
+    src = rng.integers(0, n, 40).astype(np.uint32)
+    tgt = rng.choice(n, 500, replace=False).astype(np.uint32)
+    want, _ = c.matrix(src, tgt)
+    served = 0
+    for mb in range(12, 60, 2):
+        g = bfphast.Graph.from_cch(cch, hbm_budget=mb << 20)
+        try:
+            for _ in range(2):
+                assert np.array_equal(g.matrix(src, tgt), want), mb
+            served += 1
+        except bfphast.BfError as e:
+            assert e.status == bfphast.BF_ERR_OOM and not served, mb
+        g.close()
+    assert served
