@@ -148,13 +148,17 @@ struct Panels {
   uint32_t n_levels = 0;            // levels of the panel DAG
   uint64_t max_label = 0;           // bound on every finite label of a sweep
   std::vector<uint32_t> lvl_first;  // level -> first panel, n_levels + 1
-  uint4* d_a = nullptr;             // {highest rank, rows | stride << 8 | bucket << 16,
-                                    //  sources, level}
+  uint4* d_a = nullptr;             // {highest rank, rows | stride << 8, sources, -}
   uint2* d_b = nullptr;             // {first source, first weight}
   uint32_t* d_of = nullptr;         // [n] highest rank -> panel
   uint32_t* d_hibits = nullptr;     // [n bits] highest ranks of panels
+  uint32_t* d_lvl = nullptr;        // device copy of lvl_first
   uint32_t* d_src = nullptr;        // source ranks
-  uint32_t* d_w = nullptr;          // tiles [source][row], then triangles [row][row]
+  uint32_t* d_w = nullptr;          // tiles [source][row], each followed by its panel's
+                                    // triangle [row][row]; `absent` where there is no edge
+  uint32_t absent = 0xFFFFFFFFu;
+  uint16_t* d_em = nullptr;         // per source: the rows it has an edge into
+  uint16_t* d_tm = nullptr;         // by rank: the rows of its own panel it has an edge into
   uint64_t bytes = 0;
 };
 
@@ -165,8 +169,9 @@ struct Sched {
   bool panel = false;
   bool fell_back = false;           // built as items: the budget holds no panel rows
   std::vector<uint32_t> lvl_pan;    // level -> first panel item
-  uint4* d_pitem = nullptr;         // [2 per item]
-  size_t cap_pitem = 0;
+  uint4* d_pitem = nullptr;
+  uint32_t* d_prow = nullptr;       // slab rows of the items' sources
+  size_t cap_pitem = 0, cap_prow = 0;
   bool counted = false;             // n_live / n_edges hold the rows that reach a target
   uint32_t n_live = 0;
   bool valid = false;
@@ -412,12 +417,12 @@ inline void parallel_for(uint64_t n, F&& f) {
 // One level launch; with `pdl` it is a programmatic dependent of the
 // previous launch on the stream (the kernels wait before reading rows).
 template <class... P, class... A>
-inline cudaError_t launch_level(void (*kern)(P...), dim3 grid, unsigned tpb, bool pdl,
-                                cudaStream_t s, A... args) {
+inline cudaError_t launch_level_smem(void (*kern)(P...), dim3 grid, unsigned tpb, size_t smem,
+                                     bool pdl, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(tpb);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -425,6 +430,12 @@ inline cudaError_t launch_level(void (*kern)(P...), dim3 grid, unsigned tpb, boo
   cfg.attrs = at;
   cfg.numAttrs = pdl ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+template <class... P, class... A>
+inline cudaError_t launch_level(void (*kern)(P...), dim3 grid, unsigned tpb, bool pdl,
+                                cudaStream_t s, A... args) {
+  return launch_level_smem(kern, grid, tpb, 0, pdl, s, args...);
 }
 
 // Cooperative launch of a persistent sweep kernel on `blocks` blocks.
@@ -495,8 +506,10 @@ void free_panels(Panels& P);
 bf_status build_schedule_panels(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt,
                                 const uint32_t* d_tgt, uint64_t T, uint64_t key, cudaStream_t st);
 bool panels_saturate(const Graph* g, uint64_t max_seed);
-cudaError_t sweep_panels(Graph* g, Sched& sc, uint32_t* slab, uint32_t Kp, unsigned tpb, bool sat,
-                         cudaStream_t st, uint64_t* launches, const uint32_t* seeded);
+uint32_t panel_fill(const Graph* g, uint64_t max_seed);
+uint32_t unreachable_from(const Graph* g, const Sched& sc, uint64_t max_seed);
+cudaError_t sweep_panels(Graph* g, Sched& sc, uint32_t* slab, uint32_t Kp, bool sat, cudaStream_t st,
+                         uint64_t* launches, const uint32_t* seeded);
 // schedule.cu: the target-restricted schedule of h_tgt (host) / d_tgt (the
 // same targets on the device, or null) built on the device
 bf_status build_schedule_device(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt,
@@ -504,9 +517,8 @@ bf_status build_schedule_device(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_t
 // Rows and edges that reach the schedule's targets (a panel schedule sweeps a
 // few more), counted on the context's side stream from here; finish_counts
 // waits for them and stores them in the schedule.
-bf_status start_counts(Graph* g, Ctx& c, Sched& sc, const uint32_t* d_tgt, uint64_t T,
-                       cudaStream_t st);
-bf_status finish_counts(Graph* g, Ctx& c, Sched& sc);
+bf_status start_counts(Graph* g, Ctx& c, Sched& sc, cudaStream_t st);
+bf_status finish_counts(Ctx& c, Sched& sc);
 // Per-level item, edge and row tables of a schedule in the panel form.
 bf_status schedule_tables(Graph* g, Ctx& c, Sched& sc, cudaStream_t st);
 bf_status hub_rows_device(Graph* g, Sched& sc, uint32_t H, cudaStream_t st);
@@ -518,9 +530,9 @@ bf_status sweep_levels(Graph* g, Sched& sc, uint32_t* slab, uint32_t Kp, unsigne
 void launch_mark_paths(Graph* g, const uint32_t* d_src, uint64_t k, const uint32_t* cidx,
                        uint32_t* seeded, cudaStream_t st);
 void launch_init_rows(const uint32_t* seeded, const uint32_t* split, uint32_t words,
-                      uint32_t* slab, uint32_t Kp, cudaStream_t st);
+                      uint32_t* slab, uint32_t Kp, cudaStream_t st, uint32_t fill = INF);
 bf_status prepare_rows(Graph* g, Ctx& c, Sched& sc, const uint32_t* d_src, uint64_t kw,
-                       uint32_t Kp, cudaStream_t st, uint64_t* launches);
+                       uint32_t Kp, cudaStream_t st, uint64_t* launches, uint64_t max_seed = 0);
 bf_status sweep_levels_gated(Graph* g, Sched& sc, uint32_t* slab, uint32_t Kp, unsigned lane_blocks,
                              unsigned tpb, uint32_t* active, const uint32_t* thr, uint32_t kw,
                              cudaStream_t st, uint64_t* launches,

@@ -582,14 +582,15 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// Reset to INF the rows that are read before being fully written: rows that
+// Reset to `fill` (INF, or a panel sweep's own "unreachable") the rows that
+// are read before being fully written: rows that
 // get seeds (seeded bits), rows without in-edges and rows whose in-edges are
 // split over items (combined by atomicMin). All other rows are fully written
 // by the sweep before anything reads them (of a panel schedule: all rows, so
 // split is null). One block per 32-row group.
 __global__ void __launch_bounds__(256)
     k_init_rows(const uint32_t* __restrict__ seeded, const uint32_t* __restrict__ split,
-                uint32_t words, uint32_t* __restrict__ slab, uint32_t Kp) {
+                uint32_t words, uint32_t* __restrict__ slab, uint32_t Kp, uint32_t fill) {
   for (uint32_t gw = blockIdx.x; gw < words; gw += gridDim.x) {
     uint32_t m = seeded[gw] | (split ? split[gw] : 0u);
     while (m) {
@@ -597,7 +598,7 @@ __global__ void __launch_bounds__(256)
       m &= m - 1;
       uint32_t* row = slab + (size_t)(gw * 32 + b) * Kp;
       for (uint32_t l = threadIdx.x * 4; l < Kp; l += blockDim.x * 4)
-        *reinterpret_cast<uint4*>(row + l) = make_uint4(INF, INF, INF, INF);
+        *reinterpret_cast<uint4*>(row + l) = make_uint4(fill, fill, fill, fill);
     }
   }
 }
@@ -610,10 +611,11 @@ __global__ void __launch_bounds__(256)
 // boundary of the (16-byte aligned) slab and is a multiple of 16 bytes long.
 __global__ void __launch_bounds__(128)
     k_init_rows_bulk(const uint32_t* __restrict__ seeded, const uint32_t* __restrict__ split,
-                     uint32_t words, uint32_t* __restrict__ slab, uint32_t Kp, uint32_t ch) {
+                     uint32_t words, uint32_t* __restrict__ slab, uint32_t Kp, uint32_t ch,
+                     uint32_t fill) {
   extern __shared__ __align__(128) uint4 infbuf[];
   for (uint32_t i = threadIdx.x; i < ch / 4; i += blockDim.x)
-    infbuf[i] = make_uint4(INF, INF, INF, INF);
+    infbuf[i] = make_uint4(fill, fill, fill, fill);
   // generic-proxy writes of the run made visible to the bulk copies
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
@@ -709,7 +711,7 @@ uint64_t ctx_budget(Graph* g, Ctx& c) {
 
 static void free_sched(Sched& sc) {
   void* p[] = {sc.d_cidx, sc.d_item, sc.d_erec, sc.d_elen, sc.d_trow, sc.d_split, sc.d_hub,
-               sc.d_lvl, sc.d_uses, sc.d_hub_h, sc.d_lvl_erec, sc.d_pitem};
+               sc.d_lvl, sc.d_uses, sc.d_hub_h, sc.d_lvl_erec, sc.d_pitem, sc.d_prow};
   for (void* q : p)
     if (q) cudaFree(q);
   if (sc.gexec) cudaGraphExecDestroy(sc.gexec);
@@ -796,7 +798,7 @@ bf_status sweep_levels(Graph* g, Sched& sc, uint32_t* slab, uint32_t Kp, unsigne
   bf_status hs;
   if (hinted && (hs = hub_rows(g, sc, (uint64_t)Kp * 4, st, &hub))) return hs;
   auto issue = [&](cudaStream_t s, uint64_t* count) -> cudaError_t {
-    if (sc.panel) return sweep_panels(g, sc, slab, Kp, tpb, sat, s, count, seeded);
+    if (sc.panel) return sweep_panels(g, sc, slab, Kp, sat, s, count, seeded);
     for (uint32_t l = 0; l < g->n_levels; ++l) {
       const uint32_t i0 = sc.lvl_item[l], i1 = sc.lvl_item[l + 1];
       if (i1 == i0) continue;
@@ -888,18 +890,20 @@ void launch_mark_paths(Graph* g, const uint32_t* d_src, uint64_t k, const uint32
 }
 
 void launch_init_rows(const uint32_t* seeded, const uint32_t* split, uint32_t words,
-                      uint32_t* slab, uint32_t Kp, cudaStream_t st) {
+                      uint32_t* slab, uint32_t Kp, cudaStream_t st, uint32_t fill) {
   const uint32_t grid = std::min<uint32_t>(words, 152 * 32);
   if (Kp >= 1024 && Kp % 4 == 0 && (reinterpret_cast<uintptr_t>(slab) & 15) == 0) {
     const uint32_t ch = std::min<uint32_t>(Kp, 8192);  // 32 KB of shared memory at most
-    k_init_rows_bulk<<<grid, 128, ch * 4, st>>>(seeded, split, words, slab, Kp, ch);
+    k_init_rows_bulk<<<grid, 128, ch * 4, st>>>(seeded, split, words, slab, Kp, ch, fill);
     return;
   }
-  k_init_rows<<<grid, Kp >= 1024 ? 256 : 64, 0, st>>>(seeded, split, words, slab, Kp);
+  k_init_rows<<<grid, Kp >= 1024 ? 256 : 64, 0, st>>>(seeded, split, words, slab, Kp,
+                                                           fill);
 }
 
 bf_status prepare_rows(Graph* g, Ctx& c, Sched& sc, const uint32_t* d_src, uint64_t kw,
-                       uint32_t Kp, cudaStream_t st, uint64_t* launches) {
+                       uint32_t Kp, cudaStream_t st, uint64_t* launches,
+                       uint64_t max_seed) {
   const uint32_t words = (std::max<uint32_t>(sc.n_r, 1) + 31) / 32;
   bf_status s;
   if ((s = ensure(&c.d_seeded, c.cap_seeded, words, g))) return s;
@@ -908,7 +912,8 @@ bf_status prepare_rows(Graph* g, Ctx& c, Sched& sc, const uint32_t* d_src, uint6
   // only rows the sweep does not overwrite whole need INF first (seeded,
   // split and in-edge-free rows; 10k x 10k: 2.8 against 3.5 ms for a reset
   // of the whole slab beside the upward pass)
-  launch_init_rows(c.d_seeded, sc.panel ? nullptr : sc.d_split, words, c.d_slab, Kp, st);
+  launch_init_rows(c.d_seeded, sc.panel ? nullptr : sc.d_split, words, c.d_slab, Kp, st,
+                   sc.panel ? panel_fill(g, max_seed) : INF);
   BF_CUDA(cudaGetLastError());
   *launches += 2;
   return BF_OK;
@@ -953,7 +958,8 @@ bf_status batched_wave(Graph* g, Ctx& c, const uint32_t* d_src, uint64_t kw, uin
     // only rows the sweep does not overwrite whole need INF first: seeded
     // rows (read back by their item), split rows (atomicMin targets) and rows
     // without in-edges (read, never written) - sc.d_split marks the last two
-    launch_init_rows(c.d_seeded, sc.panel ? nullptr : sc.d_split, words, c.d_slab, Kp, st);
+    launch_init_rows(c.d_seeded, sc.panel ? nullptr : sc.d_split, words, c.d_slab, Kp, st,
+                   sc.panel ? panel_fill(g, 0) : INF);
     BF_CUDA(cudaStreamWaitEvent(st, c.join, 0));
     if ((s = launch_scatter_seeds(g, c.d_cseed, kw, d_src, c.d_slab, Kp, st,
                                   pre_stride ? pre_stride : kw, pre_col, sc.d_cidx)))
@@ -1006,7 +1012,7 @@ bf_status batched_matrix(Graph* g, Ctx& c, const uint32_t* d_src, uint64_t S, co
     stats->schedule_ms +=
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tb).count();
   Sched& sc = c.sc;
-  if (stats && (s = start_counts(g, c, sc, d_tgt, T, st))) return s;
+  if (stats && (s = start_counts(g, c, sc, st))) return s;
   const uint64_t rows = std::max<uint32_t>(sc.n_r, 1);
   // lanes per wave: all sources if the slab fits the budget, else waves
   uint64_t max_lanes = ctx_budget(g, c) / (rows * 4);
@@ -1020,6 +1026,9 @@ bf_status batched_matrix(Graph* g, Ctx& c, const uint32_t* d_src, uint64_t S, co
   const uint32_t Kp = (uint32_t)((wave + 3) & ~3ull);
   if ((s = ensure_slab(g, c, (size_t)rows * Kp * 4))) return s;
   uint64_t launches = pre_launches;
+  // cells from the sweep's "unreachable" up become INF like those above the
+  // threshold
+  const uint32_t cut = std::min(threshold, unreachable_from(g, sc, 0) - 1);
   float t_up = 0, t_dn = 0, t_ex = 0;
   for (uint64_t s0 = 0; s0 < S; s0 += wave) {
     const uint64_t kw = std::min<uint64_t>(wave, S - s0);
@@ -1028,7 +1037,7 @@ bf_status batched_matrix(Graph* g, Ctx& c, const uint32_t* d_src, uint64_t S, co
       return s;
     if (stats) BF_CUDA(cudaEventRecord(c.ev[2], st));
     dim3 eg((unsigned)((T + 31) / 32), (unsigned)((kw + 31) / 32)), eb(32, 8);
-    k_extract_lanes<<<eg, eb, 0, st>>>(c.d_slab, Kp, sc.d_trow, T, (uint32_t)kw, threshold,
+    k_extract_lanes<<<eg, eb, 0, st>>>(c.d_slab, Kp, sc.d_trow, T, (uint32_t)kw, cut,
                                        d_out + s0 * T);
     BF_CUDA(cudaGetLastError());
     ++launches;
@@ -1045,7 +1054,7 @@ bf_status batched_matrix(Graph* g, Ctx& c, const uint32_t* d_src, uint64_t S, co
     }
   }
   if (stats) {
-    if ((s = finish_counts(g, c, sc))) return s;
+    if ((s = finish_counts(c, sc))) return s;
     stats->n_batches += (S + wave - 1) / wave;
     stats->waves += (S + wave - 1) / wave;
     stats->swept_nodes = sc.n_live;

@@ -48,10 +48,9 @@ namespace {
 // Peeling rounds at most (10 000 targets on the country graph take 38).
 constexpr uint32_t PEEL_ROUNDS = 4096;
 // meta words: three rotating frontier sizes, the row count, the candidate
-// count, peeling rounds run and frontier left, the grid-barrier words, the
-// totals of start_counts (two 64-bit counters)
+// count, peeling rounds run and frontier left, the grid-barrier words
 constexpr uint32_t META_NR = 3, META_NC = 4, META_ROUNDS = 5, META_LEFT = 6, META_BAR = 8,
-                   META_TOT = 12, META_WORDS = 16;
+                   META_WORDS = 16;
 constexpr uint32_t HUB_BINS = 65536;
 
 // Grow a device array to `need` elements (1/8 more with `slack`: arrays
@@ -579,8 +578,6 @@ struct SchedScratch {
   size_t cap_alive = 0, cap_ist = 0, cap_cnt = 0, cap_front = 0, cap_wpre = 0, cap_rowpos = 0,
          cap_rdeg = 0, cap_rpre = 0, cap_b64 = 0, cap_b32 = 0, cap_lvlrow = 0, cap_lvli = 0,
          cap_hist = 0, cap_meta = 0, cap_tgt = 0, cap_clist = 0;
-  unsigned long long* h_counts = nullptr;  // page-locked: rows and edges of start_counts
-  bool counting = false;      // start_counts has work on the side stream
   unsigned peel_blocks = 0;  // co-resident blocks of the peeling launch
   size_t back_words = 0;
 };
@@ -592,7 +589,6 @@ void free_sched_scratch(SchedScratch* s) {
   for (void* q : p)
     if (q) cudaFree(q);
   if (s->h_back) cudaFreeHost(s->h_back);
-  if (s->h_counts) cudaFreeHost(s->h_counts);
   delete s;
 }
 
@@ -659,29 +655,6 @@ bf_status select_rows(Graph* g, SchedScratch& s, const uint32_t* d_tgt, uint64_t
                             hook ? 2000000ll : BARRIER_TIMEOUT_CYCLES, hook ? 1u : NONE,
                             g->d_err));
   return BF_OK;
-}
-
-// Live rows and their in-edges, over the candidates.
-__global__ void __launch_bounds__(256)
-    k_sd_totals(const uint32_t* __restrict__ clist, const uint32_t* __restrict__ nc_p,
-                const uint64_t* __restrict__ in_off, const uint32_t* __restrict__ alive,
-                unsigned long long* __restrict__ tot) {
-  const uint32_t nc = *nc_p;
-  unsigned long long rows = 0, edges = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += gridDim.x * blockDim.x) {
-    const uint32_t p = clist[i];
-    if (!bit_of(alive, p)) continue;
-    ++rows;
-    edges += in_off[p + 1] - in_off[p];
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    rows += __shfl_down_sync(0xFFFFFFFFu, rows, o);
-    edges += __shfl_down_sync(0xFFFFFFFFu, edges, o);
-  }
-  if ((threadIdx.x & 31) == 0 && rows) {
-    atomicAdd(&tot[0], rows);
-    atomicAdd(&tot[1], edges);
-  }
 }
 
 // Steps 1 to 3 and the read-back: per-level tables, row and item offsets.
@@ -775,49 +748,7 @@ bf_status compact_schedule(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt,
 }  // namespace
 
 bf_status schedule_tables(Graph* g, Ctx& c, Sched& sc, cudaStream_t st) {
-  bf_status rc = finish_counts(g, c, sc);
-  if (rc) return rc;
   return compact_schedule(g, c, sc, sc.tgt.data(), nullptr, sc.T, st);
-}
-
-bf_status start_counts(Graph* g, Ctx& c, Sched& sc, const uint32_t* d_tgt, uint64_t T,
-                       cudaStream_t st) {
-  if (!sc.panel) {
-    sc.n_live = sc.n_r;
-    return BF_OK;
-  }
-  if (sc.counted) return BF_OK;
-  bf_status rc;
-  // after the caller's stream (the targets may still be on their way)
-  BF_CUDA(cudaEventRecord(c.cnt_fork, st));
-  BF_CUDA(cudaStreamWaitEvent(c.cnt, c.cnt_fork, 0));
-  if ((rc = select_scratch(g, c, sc.tgt.data(), &d_tgt, T, c.cnt))) return rc;
-  SchedScratch& s = *c.sd;
-  if (!s.h_counts &&
-      cudaHostAlloc((void**)&s.h_counts, 16, cudaHostAllocDefault) != cudaSuccess) {
-    cudaGetLastError();
-    s.h_counts = nullptr;
-    set_error("cannot allocate the row-count read-back buffer");
-    return BF_ERR_OOM;
-  }
-  if ((rc = select_rows(g, s, d_tgt, T, c.cnt))) return rc;
-  unsigned long long* tot = reinterpret_cast<unsigned long long*>(s.meta + META_TOT);
-  k_sd_totals<<<152, 256, 0, c.cnt>>>(s.clist, s.meta + META_NC, g->d_in_off, s.alive, tot);
-  BF_CUDA(cudaGetLastError());
-  BF_CUDA(cudaMemcpyAsync(s.h_counts, tot, 16, cudaMemcpyDeviceToHost, c.cnt));
-  s.counting = true;
-  return BF_OK;
-}
-
-bf_status finish_counts(Graph* g, Ctx& c, Sched& sc) {
-  (void)g;
-  if (!c.sd || !c.sd->counting) return BF_OK;
-  c.sd->counting = false;
-  BF_CUDA(cudaStreamSynchronize(c.cnt));
-  sc.n_live = (uint32_t)c.sd->h_counts[0];
-  sc.n_edges = c.sd->h_counts[1];
-  sc.counted = true;
-  return BF_OK;
 }
 
 bf_status build_schedule_device(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt,
@@ -829,8 +760,7 @@ bf_status build_schedule_device(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_t
   SplitCfg cfg{SPLIT, SMALL_SPLIT, g->tune.small_rows, SPLIT + 1};
   sc.valid = false;
   bf_status rc;
-  if ((rc = finish_counts(g, c, sc)) || (rc = compact_schedule(g, c, sc, h_tgt, d_tgt, T, st)))
-    return rc;
+  if ((rc = compact_schedule(g, c, sc, h_tgt, d_tgt, T, st))) return rc;
   SchedScratch& s = *c.sd;
   if (!d_tgt) d_tgt = s.tgt;
   uint32_t* d_nr = s.meta + META_NR;

@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(256)
     k_seeded_extract(const uint32_t* __restrict__ slab, uint32_t Kp,
                      const uint32_t* __restrict__ cidx, const uint64_t* __restrict__ toff,
                      const uint2* __restrict__ tseed, uint64_t T, uint32_t kw, uint32_t threshold,
-                     uint32_t* __restrict__ out) {
+                     uint32_t far, uint32_t* __restrict__ out) {
   __shared__ uint32_t tile[32][33];
   const uint64_t t0 = (uint64_t)blockIdx.x * 32;
   const uint32_t l0 = blockIdx.y * 32;
@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(256)
       for (uint64_t k = toff[t]; k < toff[t + 1]; ++k) {
         const uint2 sd = tseed[k];  // {rank, part}
         const uint32_t f = slab[(size_t)cidx[sd.x] * Kp + l0 + lane];
-        if (f == INF) continue;
+        if (f >= far) continue;  // unreachable
         best = min(best, f > sd.y ? f - sd.y : 0u);
       }
     }
@@ -171,10 +171,7 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
   tr.erase(std::unique(tr.begin(), tr.end()), tr.end());
   if ((rc = build_schedule(g, c, c.sc, tr.data(), tr.size(), false, s))) return rc;
   Sched& sc = c.sc;
-  if (st) {
-    const uint32_t* none = nullptr;
-    if ((rc = start_counts(g, c, sc, none, nt ? tr.size() : 0, s))) return rc;
-  }
+  if (st && (rc = start_counts(g, c, sc, s))) return rc;
   uint64_t max_seed = 0;
   for (uint64_t k = 0; k < ns; ++k) max_seed = std::max<uint64_t>(max_seed, src_seeds[k].cost);
   const uint64_t rows = std::max<uint32_t>(sc.n_r, 1);
@@ -211,7 +208,7 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
       }
     uint32_t* du = d_units.as<uint32_t>();
     if (nu) BF_CUDA(cudaMemcpyAsync(du, units.data(), units.size() * 4, cudaMemcpyHostToDevice, s));
-    if ((rc = prepare_rows(g, c, sc, du, nu, Kp, s, &launches))) return rc;
+    if ((rc = prepare_rows(g, c, sc, du, nu, Kp, s, &launches, max_seed))) return rc;
     if (nu) {
       if ((rc = launch_upward(g, du, nu, INF, sc.d_cidx, c.d_slab, Kp, nullptr, s, nullptr,
                               du + nu, du + 2 * nu)))
@@ -224,7 +221,7 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
     dim3 eg((unsigned)((T + 31) / 32), (unsigned)((kw + 31) / 32)), eb(32, 8);
     k_seeded_extract<<<eg, eb, 0, s>>>(c.d_slab, Kp, sc.d_cidx, d_to.as<uint64_t>(),
                                        d_ts.as<uint2>(), T, (uint32_t)kw, threshold,
-                                       d_out.as<uint32_t>());
+                                       unreachable_from(g, sc, max_seed), d_out.as<uint32_t>());
     BF_CUDA(cudaGetLastError());
     ++launches;
     BF_CUDA(cudaMemcpyAsync(out + s0 * T, d_out.p, kw * T * 4, cudaMemcpyDeviceToHost, s));
@@ -249,7 +246,7 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
   if (n_conflicts) *n_conflicts = cells.size();
   for (uint64_t i = 0; i < cells.size() && i < conflict_cap; ++i) conflicts[i] = cells[i];
   if (st) {
-    if ((rc = finish_counts(g, c, sc))) return rc;
+    if ((rc = finish_counts(c, sc))) return rc;
     st->n_batches += (S + wave - 1) / wave;
     st->waves += (S + wave - 1) / wave;
     st->kernel_launches += launches;

@@ -205,7 +205,7 @@ bf_status run_matrix_batch(Server* sv, Slot& sl, std::vector<Job*>& jobs) {
       if (a >= b || jobs[i]->tgt.empty()) continue;
       const uint64_t T = jobs[i]->tgt.size();
       launch_extract_lanes(c.d_slab + (a - w0), Kp, d_trow + t_off[i], T, (uint32_t)(b - a),
-                           jobs[i]->r.threshold, d_out + o_off[i] + (a - lane_off[i]) * T, st);
+                           std::min(jobs[i]->r.threshold, unreachable_from(g, c.sc, 0) - 1), d_out + o_off[i] + (a - lane_off[i]) * T, st);
     }
     BF_CUDA(cudaGetLastError());
   }
