@@ -150,7 +150,7 @@ struct Panels {
   std::vector<uint32_t> lvl_first;  // level -> first panel, n_levels + 1
   uint4* d_a = nullptr;             // {highest rank, rows | stride << 8, sources, -}
   uint2* d_b = nullptr;             // {first source, first weight}
-  uint32_t* d_of = nullptr;         // [n] highest rank -> panel
+  uint32_t* d_of = nullptr;         // [n] rank -> panel
   uint32_t* d_hibits = nullptr;     // [n bits] highest ranks of panels
   uint32_t* d_lvl = nullptr;        // device copy of lvl_first
   uint32_t* d_src = nullptr;        // source ranks
@@ -159,6 +159,12 @@ struct Panels {
   uint32_t absent = 0xFFFFFFFFu;
   uint16_t* d_em = nullptr;         // per source: the rows it has an edge into
   uint16_t* d_tm = nullptr;         // by rank: the rows of its own panel it has an edge into
+  // UP edges of a panel, likewise: {depth of the highest rank, rows | stride << 8,
+  // targets, next panel of the root path}, {highest rank, first target, first
+  // weight, row at which the path enters the next panel}
+  uint4* d_up = nullptr;
+  uint32_t* d_up_end = nullptr;     // target depths
+  uint32_t* d_up_w = nullptr;       // tiles [target][row], each with its triangle [from][to]
   uint64_t bytes = 0;
 };
 
@@ -304,7 +310,6 @@ struct Graph {
   uint32_t n = 0;
   uint64_t n_up = 0, n_down = 0;
   uint32_t n_levels = 0, max_depth = 0;
-  uint32_t max_runs = 0;  // most runs of consecutive ranks on one root path
   uint32_t engine = BF_ENGINE_BATCHED;
   uint32_t k_lanes = 0;
   std::atomic<uint64_t> device_bytes{0};
@@ -477,6 +482,14 @@ bf_status launch_upward(Graph* g, const uint32_t* d_src, uint64_t k, uint32_t th
                         cudaStream_t st, const uint32_t* lane_thr = nullptr,
                         const uint32_t* unit_cost = nullptr, const uint32_t* unit_lane = nullptr,
                         uint32_t mode = 0);
+// upward.cu: the same over panels, where their path labels fit shared memory
+bool upward_by_panels(const Graph* g);
+bf_status upward_kernel_init();
+bf_status launch_upward_panels(Graph* g, const uint32_t* d_src, uint64_t k, uint32_t threshold,
+                               const uint32_t* pos_map, uint32_t* seed, uint32_t stride,
+                               uint32_t* flag, cudaStream_t st, const uint32_t* lane_thr,
+                               const uint32_t* unit_cost, const uint32_t* unit_lane,
+                               uint32_t mode);
 // Output of the upward pass: the u32 slab, a 16-bit slab (isochrone lanes), or
 // a compact per-source buffer of k x (max_depth + 1) {row, dist} entries that
 // launch_scatter_seeds writes into the slab later (so the pass can overlap
@@ -500,8 +513,10 @@ bf_status build_schedule(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt, uin
                          cudaStream_t st, const uint32_t* d_tgt = nullptr, bool items = false);
 // panel.cu
 bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
+                       const std::vector<uint32_t>& parent, const std::vector<uint32_t>& depth,
                        const std::vector<uint64_t>& off, const std::vector<uint32_t>& src,
-                       const std::vector<uint32_t>& w, uint64_t max_up);
+                       const std::vector<uint32_t>& w, const std::vector<uint64_t>& up_off,
+                       const std::vector<uint2>& up_rec, uint64_t max_up);
 void free_panels(Panels& P);
 bf_status build_schedule_panels(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt,
                                 const uint32_t* d_tgt, uint64_t T, uint64_t key, cudaStream_t st);

@@ -244,19 +244,6 @@ static bf_status build_graph_impl(const bf_cch_csr* csr, const bf_config* cfg, G
     run_end[r] = (parent[r] == r + 1) ? run_end[r + 1] : r;
   }
   g->max_depth = maxd;
-  // runs of consecutive ranks on the longest (in runs) root path: r's path
-  // continues r + 1's run, or starts a run below its parent's path
-  {
-    std::vector<uint32_t> runs(n, 0);
-    uint32_t maxr = 0;
-    for (uint32_t r = n; r-- > 0;) {
-      if (parent[r] == NONE) runs[r] = 1;
-      else if (parent[r] == r + 1) runs[r] = runs[r + 1];
-      else runs[r] = runs[parent[r]] + 1;
-      maxr = std::max(maxr, runs[r]);
-    }
-    g->max_runs = maxr;
-  }
   // UP records, one per (source, target)
   std::vector<uint2> up_rec(g->n_up);
   std::vector<uint32_t> up_l(two ? g->n_up : 0);
@@ -366,7 +353,8 @@ static bf_status build_graph_impl(const bf_cch_csr* csr, const bf_config* cfg, G
   if ((s = dev_upload(&g->d_lvl_start, g->lvl_start.data(), g->lvl_start.size(), g))) return s;
   uint32_t zero = 0;
   if ((s = dev_upload(&g->d_err, &zero, 1, g))) return s;
-  if ((s = build_panels(g, run_end, in_off_r, in_src_r, in_w_r, max_up))) return s;
+  if ((s = build_panels(g, run_end, parent, depth, in_off_r, in_src_r, in_w_r, up_off, up_rec,
+                        max_up))) return s;
   g->rank_at = std::move(rank_at);
   g->h_in_off = std::move(in_off);
   g->h_in_rec = std::move(in_rec);

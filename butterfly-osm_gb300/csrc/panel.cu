@@ -62,61 +62,94 @@ constexpr uint32_t FAR = 0x7FFFFFFFu;
 struct HostPanel {
   uint32_t hi, k, nu, chunk;
   uint64_t u0, w0;  // within the chunk
+  uint32_t up_n;    // the same of the UP tile
+  uint64_t up_u0, up_w0;
+};
+
+// A direction's edges by rank: the other ends of v's edges are e in
+// [off[v], off[v + 1]), given by their depth in the elimination tree (all lie on
+// v's root path, so the depth names them) or by their rank.
+struct Edges {
+  const uint64_t* off;
+  const uint32_t *end, *w;
 };
 
 struct Chunk {
   std::vector<HostPanel> pan;
   std::vector<uint32_t> src, w;
   std::vector<uint16_t> em;  // per source: the rows it has an edge into
+  std::vector<uint32_t> up_end, up_w;
 };
 
-// Panels of rows (lo .. hi] of one run, split in two where the dense tile
-// would hold more than four times the edges it stands for (rows of one run
-// that pull from different ancestors), so the tiles never exceed a small
-// multiple of the graph.
-void emit_panels(uint32_t lo, uint32_t hi, uint32_t ci, const uint64_t* off, const uint32_t* src,
-                 const uint32_t* w, Chunk& out, std::vector<uint32_t>& uni, uint16_t* tm) {
-  const uint32_t k = hi - lo + 1, ks = stride_of(k);
+// The other ends outside the panel (`outside`), each once, ascending. False: a
+// dense tile of k rows would hold more than four times the edges it stands for.
+template <class F>
+bool outer_ends(uint32_t lo, uint32_t hi, const Edges& g, F outside, std::vector<uint32_t>& uni) {
   uni.clear();
   uint64_t edges = 0;
   for (uint32_t v = lo; v <= hi; ++v)
-    for (uint64_t e = off[v]; e < off[v + 1]; ++e)
-      if (src[e] > hi) {
-        uni.push_back(src[e]);
+    for (uint64_t e = g.off[v]; e < g.off[v + 1]; ++e)
+      if (outside(g.end[e])) {
+        uni.push_back(g.end[e]);
         ++edges;
       }
   std::sort(uni.begin(), uni.end());
   uni.erase(std::unique(uni.begin(), uni.end()), uni.end());
-  if (k > 1 && uni.size() * (uint64_t)k > 4 * edges + 64) {
+  return hi == lo || uni.size() * (uint64_t)(hi - lo + 1) <= 4 * edges + 64;
+}
+
+// Panels of rows [lo, hi] of one run, split in two where a tile would be mostly
+// empty (rows of one run with edges to different ancestors), so the tiles never
+// exceed a small multiple of the graph.
+void emit_panels(uint32_t lo, uint32_t hi, uint32_t ci, const Edges& dn, const Edges& up,
+                 const uint32_t* depth, Chunk& out, std::vector<uint32_t>* uni, uint16_t* tm) {
+  const uint32_t k = hi - lo + 1, ks = stride_of(k), top = depth[hi];
+  const bool dense_dn = outer_ends(lo, hi, dn, [=](uint32_t r) { return r > hi; }, uni[0]);
+  const bool dense_up = outer_ends(lo, hi, up, [=](uint32_t d) { return d < top; }, uni[1]);
+  if (!dense_dn || !dense_up) {
     const uint32_t mid = lo + k / 2;  // rows mid .. hi, then lo .. mid - 1
-    emit_panels(mid, hi, ci, off, src, w, out, uni, tm);
-    emit_panels(lo, mid - 1, ci, off, src, w, out, uni, tm);
+    emit_panels(mid, hi, ci, dn, up, depth, out, uni, tm);
+    emit_panels(lo, mid - 1, ci, dn, up, depth, out, uni, tm);
     return;
   }
-  const uint32_t nu = (uint32_t)uni.size();
-  HostPanel p{hi, k, nu, ci, out.src.size(), out.w.size()};
-  out.src.insert(out.src.end(), uni.begin(), uni.end());
-  out.em.resize(out.em.size() + nu, 0);
+  // [other end][row] tiles, each followed by its [row][row] triangle; starts
+  // are multiples of four words so that rows of a tile load as 16-byte vectors
+  auto tile = [&](std::vector<uint32_t>& ends, std::vector<uint32_t>& w, const std::vector<uint32_t>& u) {
+    ends.insert(ends.end(), u.begin(), u.end());
+    const size_t at = w.size();
+    w.resize(at + u.size() * ks + (size_t)ks * ks, INF);
+    return w.data() + at;
+  };
+  HostPanel p{hi,           k, (uint32_t)uni[0].size(), ci, out.src.size(), out.w.size(),
+              (uint32_t)uni[1].size(), out.up_end.size(), out.up_w.size()};
+  uint32_t* t = tile(out.src, out.w, uni[0]);
+  uint32_t* tri = t + (size_t)p.nu * ks;
+  uint32_t* ut = tile(out.up_end, out.up_w, uni[1]);
+  uint32_t* utri = ut + (size_t)p.up_n * ks;
+  out.em.resize(out.em.size() + p.nu, 0);
   uint16_t* em = out.em.data() + p.u0;
-  // [source][row] tile, then the [row][row] triangle; starts are multiples
-  // of four words so that rows of a tile load as 16-byte vectors
-  const size_t words = ((size_t)nu * ks + (size_t)ks * ks + 3) & ~(size_t)3;
-  out.w.resize(out.w.size() + words, INF);
-  uint32_t* t = out.w.data() + p.w0;
-  uint32_t* tri = t + (size_t)nu * ks;
+  auto find = [](const std::vector<uint32_t>& u, uint32_t x) {
+    return (size_t)(std::lower_bound(u.begin(), u.end(), x) - u.begin());
+  };
   for (uint32_t j = 0; j < k; ++j) {
     const uint32_t v = hi - j;
-    for (uint64_t e = off[v]; e < off[v + 1]; ++e) {
+    for (uint64_t e = dn.off[v]; e < dn.off[v + 1]; ++e) {
+      const uint32_t s = dn.end[e];
       uint32_t* at;
-      if (src[e] > hi) {
-        const size_t q = std::lower_bound(uni.begin(), uni.end(), src[e]) - uni.begin();
+      if (s > hi) {
+        const size_t q = find(uni[0], s);
         at = t + q * ks + j;
         em[q] |= (uint16_t)(1u << j);
       } else {
-        at = tri + (size_t)(hi - src[e]) * ks + j;
-        tm[src[e]] |= (uint16_t)(1u << j);
+        at = tri + (size_t)(hi - s) * ks + j;
+        tm[s] |= (uint16_t)(1u << j);
       }
-      *at = std::min(*at, w[e]);
+      *at = std::min(*at, dn.w[e]);
+    }
+    for (uint64_t e = up.off[v]; e < up.off[v + 1]; ++e) {
+      const uint32_t d = up.end[e];
+      uint32_t* at = d < top ? ut + find(uni[1], d) * ks + j : utri + (size_t)j * ks + (d - top);
+      *at = std::min(*at, up.w[e]);
     }
   }
   out.pan.push_back(p);
@@ -138,23 +171,36 @@ bf_status upload(T** d, const std::vector<T>& h, Panels& P) {
 }  // namespace
 
 void free_panels(Panels& P) {
-  void* q[] = {P.d_a, P.d_b, P.d_of, P.d_hibits, P.d_lvl, P.d_src, P.d_w, P.d_em, P.d_tm};
+  void* q[] = {P.d_a, P.d_b, P.d_of, P.d_hibits, P.d_lvl, P.d_src, P.d_w, P.d_em,
+               P.d_tm, P.d_up, P.d_up_end, P.d_up_w};
   for (void* x : q)
     if (x) cudaFree(x);
   P = Panels();
 }
 
-// Panels of the pull CSR by rank (in-edges of v: off, src, w; src > v) on
-// runs given by run_end. Leaves P empty (the item sweep then serves every
-// call) when the tiles do not fit 32-bit offsets or the device.
+// Panels of the DOWN edges by target rank (in-edges of v: off, src, w; src > v)
+// and the UP edges by source rank (records {depth difference, w}), on runs given
+// by run_end. Leaves P empty (items and paths then serve every call) when the
+// tiles do not fit 32-bit offsets or the device.
 bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
+                       const std::vector<uint32_t>& parent, const std::vector<uint32_t>& depth,
                        const std::vector<uint64_t>& off, const std::vector<uint32_t>& src,
-                       const std::vector<uint32_t>& w, uint64_t max_up) {
+                       const std::vector<uint32_t>& w, const std::vector<uint64_t>& up_off,
+                       const std::vector<uint2>& up_rec, uint64_t max_up) {
   Panels& P = g->panels;
   const uint32_t n = g->n;
-  bf_status rc = panel_kernels_init();
-  if (rc) return rc;
-  if (!n || off[n] >= 0x20000000ull) return BF_OK;
+  bf_status rc;
+  if ((rc = panel_kernels_init()) || (rc = upward_kernel_init())) return rc;
+  if (!n || off[n] >= 0x20000000ull || up_off[n] >= 0x20000000ull) return BF_OK;
+  std::vector<uint32_t> up_end(up_off[n]), up_w(up_off[n]);
+  parallel_for((n + 65535) / 65536, [&](uint64_t c) {
+    for (uint64_t v = c << 16; v < std::min<uint64_t>(n, (c + 1) << 16); ++v)
+      for (uint64_t e = up_off[v]; e < up_off[v + 1]; ++e) {
+        up_end[e] = depth[v] - up_rec[e].x;
+        up_w[e] = up_rec[e].y;
+      }
+  });
+  const Edges dn{off.data(), src.data(), w.data()}, up{up_off.data(), up_end.data(), up_w.data()};
   // chunks of whole runs
   std::vector<uint32_t> cut{0};
   const uint32_t step = std::max<uint32_t>(4096, n / 512);
@@ -166,7 +212,7 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
   std::vector<Chunk> ch(nc);
   std::vector<uint16_t> tm(n, 0);  // by rank: the rows of its panel it has an edge into
   parallel_for(nc, [&](uint64_t c) {
-    std::vector<uint32_t> uni;
+    std::vector<uint32_t> uni[2];
     // runs from the highest rank down; a run's panels from its end down
     for (uint32_t v = cut[c + 1]; v > cut[c];) {
       const uint32_t e = v - 1;
@@ -174,24 +220,27 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
       while (a > cut[c] && run_end[a - 1] == e) --a;
       for (uint32_t hi = e;;) {
         const uint32_t lo = hi - a >= PANEL_ROWS ? hi - PANEL_ROWS + 1 : a;
-        emit_panels(lo, hi, (uint32_t)c, off.data(), src.data(), w.data(), ch[c], uni,
-                    tm.data());
+        emit_panels(lo, hi, (uint32_t)c, dn, up, depth.data(), ch[c], uni, tm.data());
         if (lo == a) break;
         hi = lo - 1;
       }
       v = a;
     }
   });
-  uint64_t np = 0, ns = 0, nw = 0;
-  std::vector<uint64_t> sbase(nc), wbase(nc);
+  uint64_t np = 0, ns = 0, nw = 0, up_ns = 0, up_nw = 0;
+  std::vector<uint64_t> sbase(nc), wbase(nc), up_sbase(nc), up_wbase(nc);
   for (uint32_t c = 0; c < nc; ++c) {
     sbase[c] = ns;
     wbase[c] = nw;
     np += ch[c].pan.size();
     ns += ch[c].src.size();
     nw += ch[c].w.size();
+    up_sbase[c] = up_ns;
+    up_wbase[c] = up_nw;
+    up_ns += ch[c].up_end.size();
+    up_nw += ch[c].up_w.size();
   }
-  if (nw >= 0xFFFFFFFFull || ns >= 0xFFFFFFFFull) return BF_OK;
+  if (std::max(nw, up_nw) >= 0xFFFFFFFFull || std::max(ns, up_ns) >= 0xFFFFFFFFull) return BF_OK;
   for (const Chunk& c : ch)
     for (const HostPanel& p : c.pan)
       if (p.nu >= MAX_SOURCES) return BF_OK;
@@ -226,6 +275,7 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
   for (uint32_t l = 0; l < L; ++l) P.lvl_first[l + 1] += P.lvl_first[l];
   std::vector<uint4> a(np);
   std::vector<uint2> b(np);
+  std::vector<uint4> up_a(2 * np);
   std::vector<uint32_t> of(n, NONE), hib((n + 31) / 32 + 1, 0);
   // panels of a level: heaviest bucket first (a level then does not end on a
   // long item that started last), from the highest rank down in each (so
@@ -244,27 +294,42 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
         const uint32_t id = at[l * (size_t)BUCKETS + bucket_of((uint64_t)p.nu * p.k)]++;
         a[id] = make_uint4(p.hi, p.k | ks << 8, p.nu, 0);
         b[id] = make_uint2((uint32_t)(sbase[c] + p.u0), (uint32_t)(wbase[c] + p.w0));
-        of[p.hi] = id;
+        up_a[2 * (size_t)id] = make_uint4(depth[p.hi], p.k | ks << 8, p.up_n, NONE);
+        up_a[2 * (size_t)id + 1] = make_uint4(p.hi, (uint32_t)(up_sbase[c] + p.up_u0),
+                                              (uint32_t)(up_wbase[c] + p.up_w0), 0);
+        for (uint32_t j = 0; j < p.k; ++j) of[p.hi - j] = id;
         hib[p.hi >> 5] |= 1u << (p.hi & 31);
       }
+  }
+  // the next panel of a root path, and the row it enters at
+  for (size_t i = 0; i < np; ++i) {
+    const uint32_t x = parent[a[i].x];
+    if (x == NONE) continue;
+    up_a[2 * i].w = of[x];
+    up_a[2 * i + 1].w = a[of[x]].x - x;
   }
   P.n = (uint32_t)np;
   // where no label of a sweep from the graph's own nodes reaches FAR, absent
   // edges weigh FAR, which the one-instruction relaxation needs
   P.absent = P.max_label < FAR ? FAR : INF;
-  std::vector<uint32_t> s(ns), t(nw);
+  std::vector<uint32_t> s(ns), t(nw), us(up_ns), ut(up_nw);
   std::vector<uint16_t> em(ns);
   parallel_for(nc, [&](uint64_t c) {
     std::copy(ch[c].src.begin(), ch[c].src.end(), s.begin() + sbase[c]);
     std::copy(ch[c].em.begin(), ch[c].em.end(), em.begin() + sbase[c]);
     std::transform(ch[c].w.begin(), ch[c].w.end(), t.begin() + wbase[c],
                    [&](uint32_t x) { return x == INF ? P.absent : x; });
-    std::vector<uint32_t>().swap(ch[c].src);
-    std::vector<uint32_t>().swap(ch[c].w);
+    std::copy(ch[c].up_end.begin(), ch[c].up_end.end(), us.begin() + up_sbase[c]);
+    std::copy(ch[c].up_w.begin(), ch[c].up_w.end(), ut.begin() + up_wbase[c]);
+    ch[c] = Chunk();
   });
-  if ((rc = upload(&P.d_a, a, P)) || (rc = upload(&P.d_b, b, P)) || (rc = upload(&P.d_of, of, P)) ||
-      (rc = upload(&P.d_hibits, hib, P)) || (rc = upload(&P.d_lvl, P.lvl_first, P)) || (rc = upload(&P.d_src, s, P)) ||
-      (rc = upload(&P.d_w, t, P)) || (rc = upload(&P.d_em, em, P)) || (rc = upload(&P.d_tm, tm, P))) {
+  if ((rc = upload(&P.d_a, a, P)) || (rc = upload(&P.d_b, b, P)) ||
+      (rc = upload(&P.d_of, of, P)) || (rc = upload(&P.d_hibits, hib, P)) ||
+      (rc = upload(&P.d_lvl, P.lvl_first, P)) || (rc = upload(&P.d_src, s, P)) ||
+      (rc = upload(&P.d_w, t, P)) || (rc = upload(&P.d_em, em, P)) ||
+      (rc = upload(&P.d_tm, tm, P)) ||
+      (rc = upload(&P.d_up, up_a, P)) || (rc = upload(&P.d_up_end, us, P)) ||
+      (rc = upload(&P.d_up_w, ut, P))) {
     free_panels(P);
     return rc == BF_ERR_OOM ? BF_OK : rc;
   }

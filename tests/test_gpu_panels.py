@@ -82,6 +82,28 @@ def test_panels_small_graphs(built, name):
         assert np.array_equal(got, orc.table_phast_lopsided(c, sets, tsets, INF)[0]), (S, T)
 
 
+@pytest.mark.parametrize("name", ["band1", "band16", "band17", "band33", "sources300", "fan"])
+def test_upward_by_panels_with_thresholds(built, name):
+    """The upward pass with a threshold per lane (16-bit lanes), with seed
+    costs, and entering a run at every row of a panel."""
+    import bfphast
+    up, lo, hi = GRAPHS[name]
+    n = len(up)
+    cch = _cch(n, up, 7, lo, hi, 0.2)
+    c = orc.Cch.from_dict(cch)
+    g = bfphast.Graph.from_cch(cch)
+    org = np.arange(n, dtype=np.uint32)
+    thr = (np.arange(n, dtype=np.uint32) * 7) % np.uint32(3 * hi)
+    bits, counts = g.isochrone_bitsets(org, thr)
+    want_bits, want_counts = c.isochrone_bitsets(org, thr)
+    assert np.array_equal(bits, want_bits) and np.array_equal(counts, want_counts)
+    for o in sorted({0, n // 3, n // 2, n - 1}):
+        for t in (0, hi, INF):
+            seeds = [(o, 3), (n // 2, 0), (min(n - 1, o + 5), hi)]
+            got, want = g.phast_bounded_seeded(seeds, t), c.bounded_seeded(seeds, t)
+            assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), (o, t)
+
+
 @pytest.mark.parametrize("S", [130, 512, 516, 1030])
 def test_panels_wide_levels(built, grid100, S):
     """Every node a target: levels of thousands of panels, lane blocks of 512
