@@ -82,7 +82,7 @@ def test_panels_small_graphs(built, name):
         assert np.array_equal(got, orc.table_phast_lopsided(c, sets, tsets, INF)[0]), (S, T)
 
 
-@pytest.mark.parametrize("name", ["band1", "band16", "band17", "band33", "sources300", "fan"])
+@pytest.mark.parametrize("name", ["band2", "band16", "band17", "band33", "sources300", "fan"])
 def test_upward_by_panels_with_thresholds(built, name):
     """The upward pass with a threshold per lane (16-bit lanes), with seed
     costs, and entering a run at every row of a panel."""
