@@ -148,6 +148,10 @@ struct Panels {
   uint32_t n_levels = 0;            // levels of the panel DAG
   uint64_t max_label = 0;           // bound on every finite label of a sweep
   std::vector<uint32_t> lvl_first;  // level -> first panel, n_levels + 1
+  std::vector<uint32_t> lvl_small;  // level -> first panel of at most four rows
+  uint64_t n_src = 0;
+  uint32_t* d_w16 = nullptr;        // d_w for 16-bit lanes: both halfwords min(w, 0x7FFF)
+  uint32_t* d_w16s = nullptr;       // the same, min(w, 0xFFFF)
   uint4* d_a = nullptr;             // {highest rank, rows | stride << 8, sources, -}
   uint2* d_b = nullptr;             // {first source, first weight}
   uint32_t* d_of = nullptr;         // [n] rank -> panel
@@ -495,7 +499,10 @@ bf_status launch_upward_panels(Graph* g, const uint32_t* d_src, uint64_t k, uint
 // launch_scatter_seeds writes into the slab later (so the pass can overlap
 // the slab reset, or run before the restricted schedule exists: with a null
 // pos_map the entries hold ranks, which the scatter maps through `cidx`).
-enum : uint32_t { UPWARD_OUT_SLAB32 = 0, UPWARD_OUT_SLAB16 = 1, UPWARD_OUT_COMPACT = 2 };
+// UPWARD_OUT_TILES16 (panel form only): 16-bit tiles of 64 lanes [tile][rank][64],
+// `stride` ranks each; flag[rank] receives the tile's bit.
+enum : uint32_t { UPWARD_OUT_SLAB32 = 0, UPWARD_OUT_SLAB16 = 1, UPWARD_OUT_COMPACT = 2,
+                  UPWARD_OUT_TILES16 = 3 };
 // Entries of sources [0, k) read at columns col0 .. col0 + k - 1 of rows
 // `stride` entries wide (stride 0: k).
 bf_status launch_scatter_seeds(Graph* g, const void* cseed, uint64_t k, const uint32_t* d_src,
@@ -520,6 +527,7 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
 void free_panels(Panels& P);
 bf_status build_schedule_panels(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt,
                                 const uint32_t* d_tgt, uint64_t T, uint64_t key, cudaStream_t st);
+void drop_panel_schedule(Graph* g, Ctx& c, Sched& sc);
 bool panels_saturate(const Graph* g, uint64_t max_seed);
 uint32_t panel_fill(const Graph* g, uint64_t max_seed);
 uint32_t unreachable_from(const Graph* g, const Sched& sc, uint64_t max_seed);
@@ -566,6 +574,14 @@ bf_status batched_wave(Graph* g, Ctx& c, const uint32_t* d_src, uint64_t kw, uin
 bf_status batched_matrix(Graph* g, Ctx& c, const uint32_t* d_src, uint64_t S, const uint32_t* d_tgt,
                          uint64_t T, uint32_t threshold, uint32_t* d_out, cudaStream_t st,
                          bf_stats* stats);
+
+// isopanel.cu
+bf_status iso_wave_panels(Graph* g, const uint32_t* d_orig, const uint32_t* d_thr, uint32_t kw,
+                          uint32_t tmax, uint32_t* slab, uint32_t* words, uint64_t* cnt,
+                          cudaStream_t st, cudaEvent_t ev, uint64_t* launches);
+bf_status iso_bits_panels(Graph* g, const uint32_t* slab, const uint32_t* words,
+                          const uint32_t* d_thr, uint32_t kw, uint32_t* bits, uint64_t w32,
+                          uint64_t* counts, const uint32_t* out_row, cudaStream_t st);
 
 // isochrone.cu
 // Settled (rank, distance) lists of bulk isochrones, filled wave by wave:

@@ -154,6 +154,8 @@ bf_status build_schedule(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt, uin
     // of the somewhat more rows of the panels: sweep the former
     if (ctx_budget(g, c) / ((uint64_t)std::max<uint32_t>(sc.n_r, 1) * 4 + T * 8) >= 32)
       return BF_OK;
+    BF_CUDA(cudaStreamSynchronize(st));
+    drop_panel_schedule(g, c, sc);
     sc.valid = false;
     sc.fell_back = true;
   }

@@ -13,6 +13,10 @@
 // k_bits stages a 256-rank x 32-lane tile of the slab in shared memory and
 // turns each lane's 256 comparisons into eight ballot words (one 32-byte
 // sector of that origin's bitset row).
+//
+// Waves with 16-bit thresholds run over panels in tiles of 64 lanes
+// (isopanel.cu); the item sweeps here serve larger thresholds, budgets below a
+// tile, and the forms that a tunable asks for.
 
 #include <algorithm>
 #include <cstring>
@@ -760,10 +764,27 @@ __global__ void __launch_bounds__(1024)
   }
 }
 
+// Where a wave keeps lane l's label of a rank.
 template <typename T>
+struct RowSlab {
+  const T* slab;
+  uint32_t Kp;
+  const uint32_t* cidx;
+  __device__ __forceinline__ uint32_t operator()(uint32_t rank, uint32_t l) const {
+    return slab[(size_t)cidx[rank] * Kp + l];
+  }
+};
+struct TileSlab {
+  const uint16_t* slab;
+  uint32_t n;
+  __device__ __forceinline__ uint32_t operator()(uint32_t rank, uint32_t l) const {
+    return slab[((size_t)(l >> 6) * n + rank) * 64 + (l & 63)];
+  }
+};
+
+template <typename S>
 __global__ void __launch_bounds__(256)
-    k_emit(const T* __restrict__ slab, uint32_t Kp, const uint32_t* __restrict__ cidx, uint32_t n,
-           const uint32_t* __restrict__ bits, uint64_t w32, const uint32_t* __restrict__ lane_row,
+    k_emit(const S label, uint32_t n, const uint32_t* __restrict__ bits, uint64_t w32, const uint32_t* __restrict__ lane_row,
            const uint32_t* __restrict__ pre, const uint64_t* __restrict__ lane_off,
            uint64_t total, uint32_t* __restrict__ out_rank, uint32_t* __restrict__ out_dist) {
   const uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -778,15 +799,15 @@ __global__ void __launch_bounds__(256)
     const uint32_t rank = (uint32_t)(w * 32 + bit);
     if (rank < n && pos < total) {
       out_rank[pos] = rank;
-      out_dist[pos] = (uint32_t)slab[(size_t)cidx[rank] * Kp + l];
+      out_dist[pos] = label(rank, l);
     }
     ++pos;
   }
 }
 
-template <typename T>
-bf_status emit_settled(const T* slab, uint32_t Kp, Graph* g, Sched& sc, const uint32_t* bits,
-                       uint64_t w32, const uint32_t* d_lane_row, const uint32_t* h_lane_row,
+template <typename S>
+bf_status emit_settled(const S label, Graph* g, const uint32_t* bits, uint64_t w32,
+                       const uint32_t* d_lane_row, const uint32_t* h_lane_row,
                        uint32_t kw, const uint64_t* d_counts, uint64_t n_all, SettledSink* sink,
                        cudaStream_t st) {
   std::vector<uint64_t> cnt(n_all);
@@ -814,8 +835,8 @@ bf_status emit_settled(const T* slab, uint32_t Kp, Graph* g, Sched& sc, const ui
   BF_CUDA(cudaMemcpyAsync(g->d_set_off, off.data(), (kw + 1) * 8, cudaMemcpyHostToDevice, st));
   k_lane_prefix<<<kw, 1024, 0, st>>>(bits, w32, d_lane_row, g->d_set_pre);
   dim3 eg((unsigned)((w32 + 255) / 256), kw);
-  k_emit<T><<<eg, 256, 0, st>>>(slab, Kp, sc.d_cidx, g->n, bits, w32, d_lane_row, g->d_set_pre,
-                                g->d_set_off, total, g->d_set_out, g->d_set_out + total);
+  k_emit<<<eg, 256, 0, st>>>(label, g->n, bits, w32, d_lane_row, g->d_set_pre, g->d_set_off, total,
+                             g->d_set_out, g->d_set_out + total);
   BF_CUDA(cudaGetLastError());
   if (sink->on_wave) {
     std::vector<uint32_t> rows(kw);
@@ -934,8 +955,6 @@ bf_status isochrone_bitsets(Graph* g, Ctx& c, const uint32_t* d_orig, const uint
                             uint64_t* d_bits, uint64_t* d_counts, cudaStream_t st,
                             bf_stats* stats, SettledSink* sink) {
   bf_status s;
-  if (!c.shared_full && (s = build_schedule(g, c, c.full, nullptr, 0, true, st))) return s;
-  Sched& sc = c.shared_full ? *c.shared_full : c.full;
   const uint64_t rows = g->n;
   const uint64_t w64 = (g->n + 63) / 64;
   const uint64_t aw = (rows + 31) / 32;  // active-bitmap words
@@ -959,7 +978,20 @@ bf_status isochrone_bitsets(Graph* g, Ctx& c, const uint32_t* d_orig, const uint
     pk[n + i] = ht[perm[i]];
     pk[2 * n + i] = perm[i];
   }
-  const size_t need = pk.size() * 4 + 2 * aw * 4 + 16;
+  // 16-bit lanes when every threshold fits below 0xFFFF (the clamp keeps
+  // distances within the thresholds exact and halves the bytes moved)
+  uint32_t tmax = 0;
+  for (uint64_t i = 0; i < n; ++i) tmax = std::max(tmax, ht[i]);
+  const bool half = g->tune.iso_half && tmax < 0xFFFFu;
+  // by panels (isopanel.cu), in tiles of 64 lanes, unless another form is asked
+  // for or the budget holds no tile
+  const uint64_t tile_bytes = rows * 128, words_bytes = 2 * rows * 4 + 2048 * 2 + 32;
+  const bool panels = half && upward_by_panels(g) && !(g->tune.persist & 2u) && !g->tune.staged &&
+                      ctx_budget(g, c) >= tile_bytes + words_bytes + pk.size() * 4 + 16;
+  Sched* sc = c.shared_full ? c.shared_full : &c.full;
+  if (!panels && !c.shared_full && (s = build_schedule(g, c, c.full, nullptr, 0, true, st)))
+    return s;
+  const size_t need = pk.size() * 4 + (panels ? words_bytes : 2 * aw * 4) + 32;
   if (need > c.iso_tmp_bytes) {
     if (c.d_iso_tmp) {
       cudaFree(c.d_iso_tmp);
@@ -978,19 +1010,16 @@ bf_status isochrone_bitsets(Graph* g, Ctx& c, const uint32_t* d_orig, const uint
   uint32_t* p_orig = c.d_iso_tmp;
   uint32_t* p_thr = p_orig + n;
   uint32_t* p_row = p_thr + n;
-  uint32_t* d_active = p_row + n;
+  // (the panel form reads its thresholds as 16-byte vectors)
+  uint32_t* d_active = p_orig + ((3 * n + 3) & ~(uint64_t)3);
   uint32_t* d_seeded = d_active + aw;
   BF_CUDA(cudaMemcpyAsync(p_orig, pk.data(), pk.size() * 4, cudaMemcpyHostToDevice, st));
-  // 16-bit lanes when every threshold fits below 0xFFFF (the clamp keeps
-  // distances within the thresholds exact and halves the bytes moved)
-  uint32_t tmax = 0;
-  for (uint64_t i = 0; i < n; ++i) tmax = std::max(tmax, ht[i]);
-  const bool half = g->tune.iso_half && tmax < 0xFFFFu;
   const uint32_t lb = half ? 2 : 4;      // bytes per lane
   const uint32_t lq = half ? 8 : 4;      // lanes per thread (one 16-byte load)
   // the slab is the only per-lane device memory here
   uint64_t max_lanes = ctx_budget(g, c) / (rows * lb);
   max_lanes = max_lanes >= 32 ? max_lanes & ~31ull : 0;
+  if (panels) max_lanes = std::min<uint64_t>(ctx_budget(g, c) / tile_bytes, 32) * 64;
   if (!max_lanes) {
     set_error("HBM budget too small for one 32-lane isochrone wave");
     return BF_ERR_OOM;
@@ -998,7 +1027,8 @@ bf_status isochrone_bitsets(Graph* g, Ctx& c, const uint32_t* d_orig, const uint
   if (g->tune.iso_lanes) max_lanes = std::min<uint64_t>(max_lanes, g->tune.iso_lanes);
   const uint64_t wave = std::min<uint64_t>(max_lanes, (n + lq - 1) & ~(uint64_t)(lq - 1));
   const uint32_t Kp = (uint32_t)((wave + lq - 1) & ~(uint64_t)(lq - 1));
-  if ((s = ensure_slab(g, c, (size_t)rows * Kp * lb))) return s;
+  if ((s = ensure_slab(g, c, panels ? (wave + 63) / 64 * tile_bytes : (size_t)rows * Kp * lb)))
+    return s;
   BF_CUDA(cudaMemsetAsync(d_counts, 0, n * 8, st));
   const unsigned tpb = std::min<uint32_t>(128, ((Kp / lq + 31) / 32) * 32);
   const unsigned lane_blocks = (Kp / lq + tpb - 1) / tpb;
@@ -1015,92 +1045,105 @@ bf_status isochrone_bitsets(Graph* g, Ctx& c, const uint32_t* d_orig, const uint
   for (uint64_t s0 = 0; s0 < n; s0 += wave) {
     const uint64_t kw = std::min<uint64_t>(wave, n - s0);
     if (stats) BF_CUDA(cudaEventRecord(c.ev[0], st));
-    BF_CUDA(cudaMemsetAsync(d_active, 0, 2 * aw * 4, st));  // active + seeded bitmaps
-    launch_mark_paths(g, p_orig + s0, kw, sc.d_cidx, d_seeded, st);
-    // rows are Kp * lb bytes = Kp * lb / 4 words
-    launch_init_rows(d_seeded, sc.d_split, (uint32_t)aw, c.d_slab, Kp * lb / 4, st);
-    launches += 2;
-    if ((s = launch_upward(g, p_orig + s0, kw, INF, sc.d_cidx, c.d_slab, Kp, d_active, st,
-                           p_thr + s0, nullptr, nullptr,
-                           half ? UPWARD_OUT_SLAB16 : UPWARD_OUT_SLAB32)))
-      return s;
-    ++launches;
-    if (stats) BF_CUDA(cudaEventRecord(c.ev[1], st));
-    if (half && (g->tune.persist & 2u) && Kp <= 4096) {
-      if ((s = iso_sweep_persistent(g, c, sc, slab16, Kp, d_active, p_thr + s0, (uint32_t)kw,
-                                    d_seeded, st)))
+    if (panels) {
+      // (lanes ascend by threshold: the wave's last has its largest)
+      if ((s = iso_wave_panels(g, p_orig + s0, p_thr + s0, (uint32_t)kw, pk[n + s0 + kw - 1],
+                               c.d_slab, d_active, stats ? c.d_count : nullptr, st,
+                               stats ? c.ev[1] : nullptr, &launches)))
+        return s;
+    } else {
+      BF_CUDA(cudaMemsetAsync(d_active, 0, 2 * aw * 4, st));  // active + seeded bitmaps
+      launch_mark_paths(g, p_orig + s0, kw, sc->d_cidx, d_seeded, st);
+      // rows are Kp * lb bytes = Kp * lb / 4 words
+      launch_init_rows(d_seeded, sc->d_split, (uint32_t)aw, c.d_slab, Kp * lb / 4, st);
+      launches += 2;
+      if ((s = launch_upward(g, p_orig + s0, kw, INF, sc->d_cidx, c.d_slab, Kp, d_active, st,
+                             p_thr + s0, nullptr, nullptr,
+                             half ? UPWARD_OUT_SLAB16 : UPWARD_OUT_SLAB32)))
         return s;
       ++launches;
-    } else if (half) {
-      const bool pdl = g->tune.pdl != 0;
-      // runs of consecutive levels of at most two rounds of one block's items
-      // go to k_sweep_run16 (one launch per run)
-      const uint32_t wpi = (Kp + 255) / 256;
-      const uint32_t small = wpi <= 32 ? 2 * (32 / wpi) : 0;
-      for (uint32_t l = 0; l < g->n_levels; ++l) {
-        const uint32_t i0 = sc.lvl_item[l], i1 = sc.lvl_item[l + 1];
-        if (i1 == i0) continue;
-        if (i1 - i0 <= small) {
-          uint32_t l1 = l + 1;
-          while (l1 < g->n_levels && sc.lvl_item[l1 + 1] - sc.lvl_item[l1] <= small) ++l1;
-          if (l1 - l >= 2) {
-            if (g->tune.staged && sc.lvl_erec_ready)
-              BF_CUDA(launch_level(k_sweep_run16_staged, dim3(1), 1024, pdl, st,
-                                   (const uint4*)sc.d_item, (const uint32_t*)sc.d_lvl,
-                                   (const uint32_t*)sc.d_lvl_erec, l, l1, (const uint2*)sc.d_erec,
-                                   slab16, Kp, d_active, (const uint32_t*)(p_thr + s0),
-                                   (uint32_t)kw, (const uint32_t*)d_seeded, g->d_err));
-            else
-              BF_CUDA(launch_level(k_sweep_run16, dim3(1), 1024, pdl, st, (const uint4*)sc.d_item,
-                                   (const uint32_t*)sc.d_lvl, l, l1, (const uint2*)sc.d_erec,
-                                   slab16, Kp, d_active, (const uint32_t*)(p_thr + s0),
-                                   (uint32_t)kw, (const uint32_t*)d_seeded, g->d_err));
+      if (stats) BF_CUDA(cudaEventRecord(c.ev[1], st));
+      if (half && (g->tune.persist & 2u) && Kp <= 4096) {
+        if ((s = iso_sweep_persistent(g, c, *sc, slab16, Kp, d_active, p_thr + s0, (uint32_t)kw,
+                                      d_seeded, st)))
+          return s;
+        ++launches;
+      } else if (half) {
+        const bool pdl = g->tune.pdl != 0;
+        // runs of consecutive levels of at most two rounds of one block's items
+        // go to k_sweep_run16 (one launch per run)
+        const uint32_t wpi = (Kp + 255) / 256;
+        const uint32_t small = wpi <= 32 ? 2 * (32 / wpi) : 0;
+        for (uint32_t l = 0; l < g->n_levels; ++l) {
+          const uint32_t i0 = sc->lvl_item[l], i1 = sc->lvl_item[l + 1];
+          if (i1 == i0) continue;
+          if (i1 - i0 <= small) {
+            uint32_t l1 = l + 1;
+            while (l1 < g->n_levels && sc->lvl_item[l1 + 1] - sc->lvl_item[l1] <= small) ++l1;
+            if (l1 - l >= 2) {
+              if (g->tune.staged && sc->lvl_erec_ready)
+                BF_CUDA(launch_level(k_sweep_run16_staged, dim3(1), 1024, pdl, st,
+                                     (const uint4*)sc->d_item, (const uint32_t*)sc->d_lvl,
+                                     (const uint32_t*)sc->d_lvl_erec, l, l1, (const uint2*)sc->d_erec,
+                                     slab16, Kp, d_active, (const uint32_t*)(p_thr + s0),
+                                     (uint32_t)kw, (const uint32_t*)d_seeded, g->d_err));
+              else
+                BF_CUDA(launch_level(k_sweep_run16, dim3(1), 1024, pdl, st, (const uint4*)sc->d_item,
+                                     (const uint32_t*)sc->d_lvl, l, l1, (const uint2*)sc->d_erec,
+                                     slab16, Kp, d_active, (const uint32_t*)(p_thr + s0),
+                                     (uint32_t)kw, (const uint32_t*)d_seeded, g->d_err));
+              ++launches;
+              l = l1 - 1;
+              continue;
+            }
+          }
+          if (Kp <= 128) {  // thread groups of Kp / 8 threads per item
+            const uint32_t G = Kp <= 8 ? 1 : Kp <= 16 ? 2 : Kp <= 32 ? 4 : Kp <= 64 ? 8 : 16;
+            const uint32_t per_block = 128 / G;
+            const uint32_t blocks = std::min<uint32_t>((i1 - i0 + per_block - 1) / per_block,
+                                                       GATED16_BLOCKS);
+            auto kern = G == 1 ? k_sweep_group16<1> : G == 2 ? k_sweep_group16<2>
+                      : G == 4 ? k_sweep_group16<4> : G == 8 ? k_sweep_group16<8>
+                                                            : k_sweep_group16<16>;
+            BF_CUDA(launch_level(kern, dim3(blocks), 128, pdl, st, (const uint4*)sc->d_item, i0, i1,
+                                 (const uint2*)sc->d_erec, slab16, Kp, d_active,
+                                 (const uint32_t*)(p_thr + s0), (uint32_t)kw,
+                                 (const uint32_t*)d_seeded, g->d_err));
             ++launches;
-            l = l1 - 1;
             continue;
           }
-        }
-        if (Kp <= 128) {  // thread groups of Kp / 8 threads per item
-          const uint32_t G = Kp <= 8 ? 1 : Kp <= 16 ? 2 : Kp <= 32 ? 4 : Kp <= 64 ? 8 : 16;
-          const uint32_t per_block = 128 / G;
-          const uint32_t blocks = std::min<uint32_t>((i1 - i0 + per_block - 1) / per_block,
-                                                     GATED16_BLOCKS);
-          auto kern = G == 1 ? k_sweep_group16<1> : G == 2 ? k_sweep_group16<2>
-                    : G == 4 ? k_sweep_group16<4> : G == 8 ? k_sweep_group16<8>
-                                                          : k_sweep_group16<16>;
-          BF_CUDA(launch_level(kern, dim3(blocks), 128, pdl, st, (const uint4*)sc.d_item, i0, i1,
-                               (const uint2*)sc.d_erec, slab16, Kp, d_active,
-                               (const uint32_t*)(p_thr + s0), (uint32_t)kw,
+          const bool own = Kp <= 256;  // four warps per block with their own items
+          const uint32_t blocks = own ? std::min<uint32_t>((i1 - i0 + 3) / 4, 152 * 12)
+                                      : std::min<uint32_t>(i1 - i0, GATED16_BLOCKS);
+          BF_CUDA(launch_level(own ? k_sweep_gated16<4> : k_sweep_gated16<1>,
+                               dim3(blocks, own ? 1 : lane_blocks), own ? 128 : tpb, pdl, st,
+                               (const uint4*)sc->d_item, i0, i1, (const uint2*)sc->d_erec, slab16,
+                               Kp, d_active, (const uint32_t*)(p_thr + s0), (uint32_t)kw,
                                (const uint32_t*)d_seeded, g->d_err));
           ++launches;
-          continue;
         }
-        const bool own = Kp <= 256;  // four warps per block with their own items
-        const uint32_t blocks = own ? std::min<uint32_t>((i1 - i0 + 3) / 4, 152 * 12)
-                                    : std::min<uint32_t>(i1 - i0, GATED16_BLOCKS);
-        BF_CUDA(launch_level(own ? k_sweep_gated16<4> : k_sweep_gated16<1>,
-                             dim3(blocks, own ? 1 : lane_blocks), own ? 128 : tpb, pdl, st,
-                             (const uint4*)sc.d_item, i0, i1, (const uint2*)sc.d_erec, slab16,
-                             Kp, d_active, (const uint32_t*)(p_thr + s0), (uint32_t)kw,
-                             (const uint32_t*)d_seeded, g->d_err));
-        ++launches;
+      } else if ((s = sweep_levels_gated(g, *sc, c.d_slab, Kp, lane_blocks, tpb, d_active,
+                                         p_thr + s0, (uint32_t)kw, st, &launches, d_seeded))) {
+        return s;
       }
-    } else if ((s = sweep_levels_gated(g, sc, c.d_slab, Kp, lane_blocks, tpb, d_active,
-                                       p_thr + s0, (uint32_t)kw, st, &launches, d_seeded))) {
-      return s;
     }
     if (stats) BF_CUDA(cudaEventRecord(c.ev[2], st));
     dim3 bgrid((unsigned)((g->n + TILE_R - 1) / TILE_R),
                (unsigned)((kw + TILE_L * LANE_TILES_PER_BLOCK - 1) / (TILE_L * LANE_TILES_PER_BLOCK)));
-    if (half) {
+    if (panels) {
+      if ((s = iso_bits_panels(g, c.d_slab, d_active, p_thr + s0, (uint32_t)kw,
+                               reinterpret_cast<uint32_t*>(d_bits), 2 * w64, d_counts, p_row + s0,
+                               st)))
+        return s;
+    } else if (half) {
       dim3 bg16((unsigned)((g->n + BT_RANKS - 1) / BT_RANKS),
                 (unsigned)((kw + BT_LANES - 1) / BT_LANES));
-      k_bits16<<<bg16, 256, 0, st>>>(slab16, Kp, sc.d_cidx, g->n, (uint32_t)kw,
+      k_bits16<<<bg16, 256, 0, st>>>(slab16, Kp, sc->d_cidx, g->n, (uint32_t)kw,
                                      reinterpret_cast<uint32_t*>(d_bits), 2 * w64,
                                      reinterpret_cast<unsigned long long*>(d_counts), d_active,
                                      p_row + s0);
     } else
-      k_bits<<<bgrid, 256, 0, st>>>(c.d_slab, Kp, sc.d_cidx, g->n, p_thr + s0,
+      k_bits<<<bgrid, 256, 0, st>>>(c.d_slab, Kp, sc->d_cidx, g->n, p_thr + s0,
                                               (uint32_t)kw, reinterpret_cast<uint32_t*>(d_bits),
                                               2 * w64,
                                               reinterpret_cast<unsigned long long*>(d_counts),
@@ -1110,18 +1153,22 @@ bf_status isochrone_bitsets(Graph* g, Ctx& c, const uint32_t* d_orig, const uint
     if (sink) {
       const uint32_t* h_rows = pk.data() + 2 * n + s0;
       const uint32_t* bits32 = reinterpret_cast<const uint32_t*>(d_bits);
-      bf_status es = half ? emit_settled(slab16, Kp, g, sc, bits32, 2 * w64, p_row + s0, h_rows,
-                                         (uint32_t)kw, d_counts, n, sink, st)
-                          : emit_settled(c.d_slab, Kp, g, sc, bits32, 2 * w64, p_row + s0, h_rows,
-                                         (uint32_t)kw, d_counts, n, sink, st);
+      bf_status es =
+          panels ? emit_settled(TileSlab{slab16, g->n}, g, bits32, 2 * w64, p_row + s0, h_rows,
+                                (uint32_t)kw, d_counts, n, sink, st)
+          : half ? emit_settled(RowSlab<uint16_t>{slab16, Kp, sc->d_cidx}, g, bits32, 2 * w64,
+                                p_row + s0, h_rows, (uint32_t)kw, d_counts, n, sink, st)
+                 : emit_settled(RowSlab<uint32_t>{c.d_slab, Kp, sc->d_cidx}, g, bits32, 2 * w64,
+                                p_row + s0, h_rows, (uint32_t)kw, d_counts, n, sink, st);
       if (es) return es;
       launches += 2;
     }
     if (stats) {
       BF_CUDA(cudaEventRecord(c.ev[3], st));
-      // outside the timed phases: count the wave's algorithmic sweep bytes
-      k_iso_count<<<(unsigned)std::min<uint64_t>((sc.n_items + 255) / 256, 152 * 8), 256, 0, st>>>(
-          (const uint4*)sc.d_item, sc.n_items, (const uint2*)sc.d_erec, d_active, Kp * lb,
+      // outside the timed phases: count the wave's algorithmic sweep bytes (the
+      // panel form counts as it sweeps)
+      if (!panels) k_iso_count<<<(unsigned)std::min<uint64_t>((sc->n_items + 255) / 256, 152 * 8), 256, 0, st>>>(
+          (const uint4*)sc->d_item, sc->n_items, (const uint2*)sc->d_erec, d_active, Kp * lb,
           reinterpret_cast<unsigned long long*>(c.d_count));
       BF_CUDA(cudaGetLastError());
       BF_CUDA(cudaEventSynchronize(c.ev[3]));
@@ -1143,14 +1190,16 @@ bf_status isochrone_bitsets(Graph* g, Ctx& c, const uint32_t* d_orig, const uint
     stats->upward_ms += t_up;
     stats->downward_ms += t_dn;
     stats->extract_ms += t_ex;
-    stats->swept_nodes = sc.n_r;
-    stats->swept_edges = sc.n_edges;
+    stats->swept_nodes = g->n;
+    stats->swept_edges = g->n_down;
     stats->lanes = Kp;
     uint64_t cnt[2] = {0, 0};
     BF_CUDA(cudaMemcpyAsync(cnt, c.d_count, 16, cudaMemcpyDeviceToHost, st));
     BF_CUDA(cudaStreamSynchronize(st));
-    // + every wave scans the schedule: 16 B per item and 8 B per edge record
-    stats->sweep_bytes += cnt[0] + waves * (16 * sc.n_items + 8 * sc.n_edges);
+    // + every wave scans the schedule: 24 B per panel, 8 B per source and its
+    // activity, or 16 B per item and 8 B per edge record
+    stats->sweep_bytes += cnt[0] + waves * (panels ? 24ull * g->panels.n + 8ull * g->panels.n_src
+                                                   : 16 * sc->n_items + 8 * sc->n_edges);
     stats->active_rows += cnt[1];
   }
   return BF_OK;

@@ -50,9 +50,11 @@ __device__ __forceinline__ uint32_t item_live(const uint4& it) { return it.y & 3
 __device__ __forceinline__ uint32_t item_stride(const uint4& it) { return (it.y >> 5) & 31u; }
 __device__ __forceinline__ uint32_t item_sources(const uint4& it) { return it.y >> 10; }
 
-// Work buckets of a level's panels.
-constexpr uint32_t BUCKETS = 4;
-uint32_t bucket_of(uint64_t work) { return work >= 2048 ? 0 : work >= 512 ? 1 : work >= 64 ? 2 : 3; }
+// Buckets of a level's panels by rows and work.
+constexpr uint32_t BUCKETS = 5;
+uint32_t bucket_of(uint32_t k, uint64_t work) {
+  return k <= 4 ? 4 : work >= 2048 ? 0 : work >= 512 ? 1 : work >= 64 ? 2 : 3;
+}
 
 // Labels at or above this stand for "unreachable" in the one-instruction form
 // of the relaxation (relax() below), which a sweep uses when no finite label
@@ -168,11 +170,37 @@ bf_status upload(T** d, const std::vector<T>& h, Panels& P) {
   return BF_OK;
 }
 
+__global__ void __launch_bounds__(256)
+    k_pack_weights(const uint32_t* __restrict__ w, uint64_t m, uint32_t absent, uint32_t cap,
+                   uint32_t* __restrict__ out) {
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
+       i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t x = w[i] == absent ? cap : min(w[i], cap);
+    out[i] = x | x << 16;
+  }
+}
+
+// The weight tiles for 16-bit lanes, from d_w.
+bf_status pack_weights(Panels& P, uint64_t m) {
+  for (uint32_t** p : {&P.d_w16, &P.d_w16s}) {
+    if (cudaMalloc((void**)p, m * 4) != cudaSuccess) {
+      cudaGetLastError();
+      *p = nullptr;
+      return BF_ERR_OOM;
+    }
+    P.bytes += m * 4;
+    k_pack_weights<<<152 * 8, 256>>>(P.d_w, m, P.absent, p == &P.d_w16 ? 0x7FFFu : 0xFFFFu, *p);
+    BF_CUDA(cudaGetLastError());
+  }
+  BF_CUDA(cudaDeviceSynchronize());
+  return BF_OK;
+}
+
 }  // namespace
 
 void free_panels(Panels& P) {
   void* q[] = {P.d_a, P.d_b, P.d_of, P.d_hibits, P.d_lvl, P.d_src, P.d_w, P.d_em,
-               P.d_tm, P.d_up, P.d_up_end, P.d_up_w};
+               P.d_tm, P.d_up, P.d_up_end, P.d_up_w, P.d_w16, P.d_w16s};
   for (void* x : q)
     if (x) cudaFree(x);
   P = Panels();
@@ -270,6 +298,8 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
   // every label of a sweep is the weight of an UP path and a DOWN path
   P.max_label = max_up + max_down;
   P.n_levels = L;
+  P.n_src = ns;
+  P.lvl_small.clear();
   P.lvl_first.assign(L + 1, 0);
   for (uint32_t l : lvl) ++P.lvl_first[l + 1];
   for (uint32_t l = 0; l < L; ++l) P.lvl_first[l + 1] += P.lvl_first[l];
@@ -278,20 +308,21 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
   std::vector<uint4> up_a(2 * np);
   std::vector<uint32_t> of(n, NONE), hib((n + 31) / 32 + 1, 0);
   // panels of a level: heaviest bucket first (a level then does not end on a
-  // long item that started last), from the highest rank down in each (so
+  // long item that started last), those of at most four rows last, from the highest rank down in each (so
   // neighbours share sources)
   {
     std::vector<uint32_t> at((size_t)L * BUCKETS + 1, 0);
     size_t i = 0;
     for (uint32_t c = nc; c-- > 0;)
       for (const HostPanel& p : ch[c].pan)
-        ++at[lvl[i++] * (size_t)BUCKETS + bucket_of((uint64_t)p.nu * p.k) + 1];
+        ++at[lvl[i++] * (size_t)BUCKETS + bucket_of(p.k, (uint64_t)p.nu * p.k) + 1];
     for (size_t k = 1; k < at.size(); ++k) at[k] += at[k - 1];
+    for (uint32_t l = 0; l < L; ++l) P.lvl_small.push_back(at[l * (size_t)BUCKETS + BUCKETS - 1]);
     i = 0;
     for (uint32_t c = nc; c-- > 0;)
       for (const HostPanel& p : ch[c].pan) {
         const uint32_t l = lvl[i++], ks = stride_of(p.k);
-        const uint32_t id = at[l * (size_t)BUCKETS + bucket_of((uint64_t)p.nu * p.k)]++;
+        const uint32_t id = at[l * (size_t)BUCKETS + bucket_of(p.k, (uint64_t)p.nu * p.k)]++;
         a[id] = make_uint4(p.hi, p.k | ks << 8, p.nu, 0);
         b[id] = make_uint2((uint32_t)(sbase[c] + p.u0), (uint32_t)(wbase[c] + p.w0));
         up_a[2 * (size_t)id] = make_uint4(depth[p.hi], p.k | ks << 8, p.up_n, NONE);
@@ -312,7 +343,8 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
   // where no label of a sweep from the graph's own nodes reaches FAR, absent
   // edges weigh FAR, which the one-instruction relaxation needs
   P.absent = P.max_label < FAR ? FAR : INF;
-  std::vector<uint32_t> s(ns), t(nw), us(up_ns), ut(up_nw);
+  nw += PANEL_ROWS * PANEL_ROWS;  // (a tile of 12 rows may be read as one of 16)
+  std::vector<uint32_t> s(ns), t(nw, P.absent), us(up_ns), ut(up_nw);
   std::vector<uint16_t> em(ns);
   parallel_for(nc, [&](uint64_t c) {
     std::copy(ch[c].src.begin(), ch[c].src.end(), s.begin() + sbase[c]);
@@ -329,7 +361,7 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
       (rc = upload(&P.d_w, t, P)) || (rc = upload(&P.d_em, em, P)) ||
       (rc = upload(&P.d_tm, tm, P)) ||
       (rc = upload(&P.d_up, up_a, P)) || (rc = upload(&P.d_up_end, us, P)) ||
-      (rc = upload(&P.d_up_w, ut, P))) {
+      (rc = upload(&P.d_up_w, ut, P)) || (rc = pack_weights(P, nw))) {
     free_panels(P);
     return rc == BF_ERR_OOM ? BF_OK : rc;
   }
@@ -597,6 +629,7 @@ struct PanelScratch {
   uint32_t* tgt = nullptr;    // uploaded targets
   unsigned long long* h_counts = nullptr;  // page-locked: rows, edges
   bool counting = false;      // start_counts has work on the side stream
+  uint64_t bytes = 0;         // device memory of the graph-sized arrays and the targets
   uint32_t* h_back = nullptr;  // page-locked: sources, cursor, rows, level table
   size_t cap_tgt = 0;
 };
@@ -635,6 +668,24 @@ bf_status grow(T** p, size_t& cap, size_t need, Graph* g, bool slack) {
 }
 
 }  // namespace
+
+// Give a context's panel scratch and a schedule's panel items back (the budget
+// holds no panel rows: what the item form had before is its again).
+void drop_panel_schedule(Graph* g, Ctx& c, Sched& sc) {
+  if (c.ps) {
+    if (c.ps->counting) cudaStreamSynchronize(c.cnt);
+    g->device_bytes -= c.ps->bytes + c.ps->cap_tgt * 4;
+    free_panel_scratch(c.ps);
+    c.ps = nullptr;
+  }
+  g->device_bytes -= sc.cap_pitem * sizeof(uint4) + sc.cap_prow * 4;
+  if (sc.d_pitem) cudaFree(sc.d_pitem);
+  if (sc.d_prow) cudaFree(sc.d_prow);
+  sc.d_pitem = nullptr;
+  sc.d_prow = nullptr;
+  sc.cap_pitem = sc.cap_prow = 0;
+  sc.lvl_pan.clear();
+}
 
 // Words of the live bitmap, even: two 64-bit counters lie behind it.
 static size_t live_words(uint32_t n) { return (((size_t)n + 31) / 32 + 2) & ~(size_t)1; }
@@ -709,12 +760,14 @@ bf_status build_schedule_panels(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_t
   }
   size_t none = 0;
   if (!s.h_back) {
+    const uint64_t before = g->device_bytes;
     if ((rc = grow(&s.bits, none = 0, meta + 3 + L + 1, g, false)) ||
         (rc = grow(&s.pre, none = 0, meta, g, false)) ||
         (rc = grow(&s.bsum, none = 0, 2 * (size_t)nb, g, false)) ||
         (rc = grow(&s.live, none = 0, live_words(n) + 6, g, false)) ||
         (rc = grow(&s.list, none = 0, P.n, g, false)))
       return rc;
+    s.bytes = g->device_bytes - before;
     if (!s.h_counts && cudaHostAlloc((void**)&s.h_counts, 16, cudaHostAllocDefault) != cudaSuccess) {
       cudaGetLastError();
       s.h_counts = nullptr;

@@ -140,6 +140,12 @@ __global__ void __launch_bounds__(UPWARD_WARPS * 32, 6)
         // different sources at one index mostly name the same top-of-tree row
         const uint32_t p = !in ? NONE : pos_of ? pos_of[x] : x;
         reinterpret_cast<uint2*>(seed)[(size_t)(a.x + lane) * seed_stride + w] = make_uint2(p, d);
+      } else if (mode == UPWARD_OUT_TILES16) {
+        if (in) {  // (within its lane threshold, < 0xFFFF)
+          reinterpret_cast<uint16_t*>(seed)[((size_t)(w >> 6) * seed_stride + x) * 64 + (w & 63)] =
+              (uint16_t)d;
+          atomicOr(&flag[x], 1u << (w >> 6));
+        }
       } else if (in) {
         const uint32_t p = pos_of[x];
         if (p != NONE) {

@@ -154,7 +154,8 @@ typedef struct bf_stats {
   uint64_t sweep_bytes;       /* isochrone calls: algorithmic bytes of the gated
                                  sweeps (schedule records scanned, active source
                                  rows gathered, rows written), summed over waves */
-  uint64_t active_rows;       /* isochrone calls: rows written by the sweeps      */
+  uint64_t active_rows;       /* isochrone calls: rows written by the sweeps (rows of
+                                 64 lanes each where a wave runs over panels)     */
 } bf_stats;
 
 bf_status bf_graph_create(const bf_cch_csr* csr, const bf_config* cfg, bf_graph** out);

@@ -145,3 +145,49 @@ def test_panels_budget_falls_back_to_items(built, country_small):
             assert e.status == bfphast.BF_ERR_OOM and not served, mb
         g.close()
     assert served
+
+
+@pytest.mark.parametrize("count", [1, 63, 64, 65, 129, 2100])
+@pytest.mark.parametrize("top", [300, 0x7FFE, 0x7FFF, 0xFFFE])
+def test_isochrones_by_panels(built, count, top):
+    """Lanes at the edges of tiles and waves, thresholds at the edges of the
+    two 16-bit forms: bitsets, counts and settled lists."""
+    import bfphast
+    up, lo, hi = _band(180, 60), 1, max(2, top // 40)
+    n = len(up)
+    cch = _cch(n, up, 3, lo, hi, 0.2)
+    c = orc.Cch.from_dict(cch)
+    g = bfphast.Graph.from_cch(cch)
+    g.set_tune(isochrone_lanes=0)
+    rng = np.random.default_rng(count)
+    org = rng.integers(0, n, count).astype(np.uint32)
+    thr = rng.integers(0, top + 1, count).astype(np.uint32)
+    thr[0] = top
+    bits, counts = g.isochrone_bitsets(org, thr)
+    want_bits, want_counts = c.isochrone_bitsets(org, thr)
+    assert np.array_equal(bits, want_bits) and np.array_equal(counts, want_counts)
+    sets = g.isochrone_settled(org, thr)
+    for i in range(0, count, max(1, count // 9)):
+        rk, ds = c.bounded_seeded([(int(org[i]), 0)], int(thr[i]))
+        assert np.array_equal(sets[i][0], rk) and np.array_equal(sets[i][1], ds), i
+
+
+def test_isochrones_panels_budget_falls_back(built, country_small):
+    """A budget below one tile of 64 lanes is still served (by the item waves)."""
+    import bfphast
+    _, cch = country_small
+    c = orc.Cch.from_dict(cch)
+    org = np.array([5, 700, 33000], np.uint32)
+    thr = np.array([3000, 36000, 6000], np.uint32)
+    want_bits, want_counts = c.isochrone_bitsets(org, thr)
+    served = 0
+    for mb in range(20, 60, 2):
+        g = bfphast.Graph.from_cch(cch, hbm_budget=mb << 20)
+        try:
+            bits, counts = g.isochrone_bitsets(org, thr)
+            assert np.array_equal(bits, want_bits) and np.array_equal(counts, want_counts), mb
+            served += 1
+        except bfphast.BfError as e:
+            assert e.status == bfphast.BF_ERR_OOM and not served, mb
+        g.close()
+    assert served
