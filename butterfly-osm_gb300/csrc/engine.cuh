@@ -169,6 +169,8 @@ struct Panels {
   uint4* d_up = nullptr;
   uint32_t* d_up_end = nullptr;     // target depths
   uint32_t* d_up_w = nullptr;       // tiles [target][row], each with its triangle [from][to]
+  uint32_t* d_len = nullptr;        // length weights like d_w and d_up_w (INF where there is
+  uint32_t* d_up_len = nullptr;     // no edge), on two-channel graphs
   uint64_t bytes = 0;
 };
 
@@ -178,6 +180,7 @@ struct Sched {
   // items and edge records below are then not built
   bool panel = false;
   bool fell_back = false;           // built as items: the budget holds no panel rows
+  uint32_t words = 1;               // of the callers it was built for
   std::vector<uint32_t> lvl_pan;    // level -> first panel item
   uint4* d_pitem = nullptr;
   uint32_t* d_prow = nullptr;       // slab rows of the items' sources
@@ -271,6 +274,8 @@ struct Ctx {
   size_t cap_cseed = 0;
   uint32_t* d_one = nullptr;       // bounded-query state: active bitmap, then the threshold
   size_t cap_one = 0;
+  void* d_call = nullptr;          // seeds, units and cells of a seeded matrix call (call_buffer)
+  size_t call_bytes = 0;
   void* h_stage = nullptr;         // page-locked staging arena for schedule uploads
   size_t stage_bytes = 0;
   SchedScratch* sd = nullptr;      // device schedule builder scratch
@@ -514,16 +519,17 @@ __global__ void k_extract(const uint32_t* __restrict__ slab, uint32_t slab_strid
 
 // engine_batched.cu
 bf_status batched_prepare(Graph* g, uint32_t split_edges);
-// items: the caller reads work items and edge records (else a restricted
-// schedule may come in the panel form, which only sweep_levels reads).
+// A restricted schedule may come in the panel form (sc.panel). words: 32-bit
+// words per lane of the caller's slab (1, or 2 with lengths).
 bf_status build_schedule(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt, uint64_t T, bool all,
-                         cudaStream_t st, const uint32_t* d_tgt = nullptr, bool items = false);
+                         cudaStream_t st, const uint32_t* d_tgt = nullptr, uint32_t words = 1);
 // panel.cu
 bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
                        const std::vector<uint32_t>& parent, const std::vector<uint32_t>& depth,
                        const std::vector<uint64_t>& off, const std::vector<uint32_t>& src,
                        const std::vector<uint32_t>& w, const std::vector<uint64_t>& up_off,
-                       const std::vector<uint2>& up_rec, uint64_t max_up);
+                       const std::vector<uint2>& up_rec, uint64_t max_up, const uint32_t* len,
+                       const uint32_t* up_len);
 void free_panels(Panels& P);
 bf_status build_schedule_panels(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt,
                                 const uint32_t* d_tgt, uint64_t T, uint64_t key, cudaStream_t st);
@@ -562,6 +568,11 @@ bf_status sweep_levels_gated(Graph* g, Sched& sc, uint32_t* slab, uint32_t Kp, u
                              const uint32_t* seeded = nullptr);
 bf_status ensure_slab(Graph* g, Ctx& c, size_t bytes);
 bf_status hub_rows(Graph* g, Sched& sc, uint64_t row_bytes, cudaStream_t st, const uint32_t** hub);
+// Device memory for one call's seeds, units and cells, kept by the context up to
+// 256 MB (a cudaMalloc and a cudaFree each cost a call more than its copies;
+// outside the budget, like the call's own allocations were).
+bf_status call_buffer(Ctx& c, size_t bytes, void** out);
+void trim_call_buffer(Ctx& c);
 uint64_t ctx_budget(Graph* g, Ctx& c);
 void free_ctx(Ctx& c);
 bf_status init_ctx(Ctx& c);
@@ -615,6 +626,16 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
                         uint64_t conflict_cap, uint64_t* n_conflicts, bf_stats* st);
 bf_status bounded_seeded(Graph* g, Ctx& c, const bf_seed* seeds, uint32_t n_seeds, uint32_t threshold,
                          uint32_t* out_rank, uint32_t* out_dist, uint64_t cap, uint64_t* n_out);
+
+// twopanel.cu: the two-channel sweep and upward pass over panels (u64 labels;
+// rows of the slab are Kp2 lanes wide)
+cudaError_t sweep_panels_2ch(Graph* g, Sched& sc, uint64_t* slab, uint32_t Kp2, cudaStream_t st,
+                             uint64_t* launches, const uint32_t* seeded);
+bool upward_2ch_by_panels(const Graph* g);
+bf_status upward_2ch_kernel_init();
+bf_status launch_upward_2ch_panels(Graph* g, const uint32_t* d_units, uint64_t nu,
+                                   uint32_t threshold, const uint32_t* cidx, uint64_t* slab,
+                                   uint32_t stride, uint32_t* flag, cudaStream_t st);
 
 // twochannel.cu
 bf_status matrix_seeded_2ch(Graph* g, Ctx& c, const bf_seed2* src_seeds, const uint64_t* src_off,

@@ -120,10 +120,10 @@ __global__ void k_scatter_pairs(const uint2* __restrict__ pr, uint64_t m,
 // map is patched in place: entries of the previous schedule are reset to
 // NONE and the new ones set.
 bf_status build_schedule(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt, uint64_t T, bool all,
-                         cudaStream_t st, const uint32_t* d_tgt, bool want_items) {
+                         cudaStream_t st, const uint32_t* d_tgt, uint32_t words) {
   // restricted schedules are built on the device unless turned off: as panels
-  // (panel.cu) where the caller only sweeps, else as items (schedule.cu)
-  const bool panels = !all && T && g->tune.dev_sched && g->panels.n && !want_items;
+  // (panel.cu) where the graph has them, else as items (schedule.cu)
+  const bool panels = !all && T && g->tune.dev_sched && g->panels.n;
   const uint32_t SPLIT = std::max<uint32_t>(1, g->tune.split);
   const uint32_t SMALL_ROWS = g->tune.small_rows;
   const uint32_t SMALL_SPLIT = std::max<uint32_t>(1, std::min(SPLIT, g->tune.small_split));
@@ -132,6 +132,7 @@ bf_status build_schedule(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt, uin
                        ((uint64_t)SMALL_ROWS << 20);
   // reuse only for the same split settings and exactly the same targets
   if (sc.valid && sc.key == key && sc.T == T && (sc.panel || sc.fell_back) == panels &&
+      (!panels || sc.words == words) &&
       (all || (sc.tgt.size() == T && (T == 0 || std::memcmp(sc.tgt.data(), h_tgt, T * 4) == 0)))) {
     ++sc.uses;
     return BF_OK;
@@ -147,12 +148,13 @@ bf_status build_schedule(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt, uin
     sc.one_exec = nullptr;
   }
   sc.fell_back = false;
+  sc.words = words;
   if (panels) {
     bf_status s = build_schedule_panels(g, c, sc, h_tgt, d_tgt, T, key, st);
     if (s) return s;
     // a budget that holds 32 lanes of the rows that reach a target, but not
     // of the somewhat more rows of the panels: sweep the former
-    if (ctx_budget(g, c) / ((uint64_t)std::max<uint32_t>(sc.n_r, 1) * 4 + T * 8) >= 32)
+    if (ctx_budget(g, c) / (((uint64_t)std::max<uint32_t>(sc.n_r, 1) * 4 + T * 8) * words) >= 32)
       return BF_OK;
     BF_CUDA(cudaStreamSynchronize(st));
     drop_panel_schedule(g, c, sc);
@@ -711,6 +713,30 @@ uint64_t ctx_budget(Graph* g, Ctx& c) {
   return (g->hbm_budget > used ? g->hbm_budget - used : 0) + c.slab_bytes;
 }
 
+bf_status call_buffer(Ctx& c, size_t bytes, void** out) {
+  if (bytes > c.call_bytes) {
+    if (c.d_call) cudaFree(c.d_call);
+    c.d_call = nullptr;
+    c.call_bytes = 0;
+    if (cudaMalloc(&c.d_call, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      c.d_call = nullptr;
+      set_error("cudaMalloc of " + std::to_string(bytes) + " bytes failed");
+      return BF_ERR_OOM;
+    }
+    c.call_bytes = bytes;
+  }
+  *out = c.d_call;
+  return BF_OK;
+}
+
+void trim_call_buffer(Ctx& c) {
+  if (c.call_bytes <= (256u << 20)) return;
+  cudaFree(c.d_call);
+  c.d_call = nullptr;
+  c.call_bytes = 0;
+}
+
 static void free_sched(Sched& sc) {
   void* p[] = {sc.d_cidx, sc.d_item, sc.d_erec, sc.d_elen, sc.d_trow, sc.d_split, sc.d_hub,
                sc.d_lvl, sc.d_uses, sc.d_hub_h, sc.d_lvl_erec, sc.d_pitem, sc.d_prow};
@@ -730,6 +756,7 @@ void free_ctx(Ctx& c) {
   if (c.d_iso_tmp) cudaFree(c.d_iso_tmp);
   if (c.d_cseed) cudaFree(c.d_cseed);
   if (c.d_one) cudaFree(c.d_one);
+  if (c.d_call) cudaFree(c.d_call);
   if (c.d_iso_prog) cudaFree(c.d_iso_prog);
   if (c.d_count) cudaFree(c.d_count);
   if (c.h_stage) cudaFreeHost(c.h_stage);

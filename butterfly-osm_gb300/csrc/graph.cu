@@ -353,8 +353,11 @@ static bf_status build_graph_impl(const bf_cch_csr* csr, const bf_config* cfg, G
   if ((s = dev_upload(&g->d_lvl_start, g->lvl_start.data(), g->lvl_start.size(), g))) return s;
   uint32_t zero = 0;
   if ((s = dev_upload(&g->d_err, &zero, 1, g))) return s;
+  // (an edgeless direction of a two-channel graph still has lengths: none)
+  if (two && in_l_r.empty()) in_l_r.reserve(1);
+  if (two && up_l.empty()) up_l.reserve(1);
   if ((s = build_panels(g, run_end, parent, depth, in_off_r, in_src_r, in_w_r, up_off, up_rec,
-                        max_up))) return s;
+                        max_up, two ? in_l_r.data() : nullptr, two ? up_l.data() : nullptr))) return s;
   g->rank_at = std::move(rank_at);
   g->h_in_off = std::move(in_off);
   g->h_in_rec = std::move(in_rec);

@@ -73,7 +73,7 @@ struct HostPanel {
 // v's root path, so the depth names them) or by their rank.
 struct Edges {
   const uint64_t* off;
-  const uint32_t *end, *w;
+  const uint32_t *end, *w, *len;  // len: null on one-channel graphs
 };
 
 struct Chunk {
@@ -81,6 +81,7 @@ struct Chunk {
   std::vector<uint32_t> src, w;
   std::vector<uint16_t> em;  // per source: the rows it has an edge into
   std::vector<uint32_t> up_end, up_w;
+  std::vector<uint32_t> len, up_len;  // like w and up_w, on two-channel graphs
 };
 
 // The other ends outside the panel (`outside`), each once, ascending. False: a
@@ -130,6 +131,23 @@ void emit_panels(uint32_t lo, uint32_t hi, uint32_t ci, const Edges& dn, const E
   uint32_t* utri = ut + (size_t)p.up_n * ks;
   out.em.resize(out.em.size() + p.nu, 0);
   uint16_t* em = out.em.data() + p.u0;
+  if (dn.len) {
+    out.len.resize(out.w.size(), INF);
+    out.up_len.resize(out.up_w.size(), INF);
+  }
+  // parallel edges: the smaller (time, length)
+  auto put = [](uint32_t* at, std::vector<uint32_t>& w, std::vector<uint32_t>& len, const Edges& g,
+                uint64_t e) {
+    if (!g.len) {
+      *at = std::min(*at, g.w[e]);
+      return;
+    }
+    uint32_t& l = len[at - w.data()];
+    if (g.w[e] < *at || (g.w[e] == *at && g.len[e] < l)) {
+      *at = g.w[e];
+      l = g.len[e];
+    }
+  };
   auto find = [](const std::vector<uint32_t>& u, uint32_t x) {
     return (size_t)(std::lower_bound(u.begin(), u.end(), x) - u.begin());
   };
@@ -146,12 +164,12 @@ void emit_panels(uint32_t lo, uint32_t hi, uint32_t ci, const Edges& dn, const E
         at = tri + (size_t)(hi - s) * ks + j;
         tm[s] |= (uint16_t)(1u << j);
       }
-      *at = std::min(*at, dn.w[e]);
+      put(at, out.w, out.len, dn, e);
     }
     for (uint64_t e = up.off[v]; e < up.off[v + 1]; ++e) {
       const uint32_t d = up.end[e];
       uint32_t* at = d < top ? ut + find(uni[1], d) * ks + j : utri + (size_t)j * ks + (d - top);
-      *at = std::min(*at, up.w[e]);
+      put(at, out.up_w, out.up_len, up, e);
     }
   }
   out.pan.push_back(p);
@@ -200,7 +218,8 @@ bf_status pack_weights(Panels& P, uint64_t m) {
 
 void free_panels(Panels& P) {
   void* q[] = {P.d_a, P.d_b, P.d_of, P.d_hibits, P.d_lvl, P.d_src, P.d_w, P.d_em,
-               P.d_tm, P.d_up, P.d_up_end, P.d_up_w, P.d_w16, P.d_w16s};
+               P.d_tm, P.d_up, P.d_up_end, P.d_up_w, P.d_w16,
+               P.d_w16s, P.d_len, P.d_up_len};
   for (void* x : q)
     if (x) cudaFree(x);
   P = Panels();
@@ -214,11 +233,14 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
                        const std::vector<uint32_t>& parent, const std::vector<uint32_t>& depth,
                        const std::vector<uint64_t>& off, const std::vector<uint32_t>& src,
                        const std::vector<uint32_t>& w, const std::vector<uint64_t>& up_off,
-                       const std::vector<uint2>& up_rec, uint64_t max_up) {
+                       const std::vector<uint2>& up_rec, uint64_t max_up, const uint32_t* len,
+                       const uint32_t* up_len) {
   Panels& P = g->panels;
   const uint32_t n = g->n;
   bf_status rc;
-  if ((rc = panel_kernels_init()) || (rc = upward_kernel_init())) return rc;
+  if ((rc = panel_kernels_init()) || (rc = upward_kernel_init()) ||
+      (rc = upward_2ch_kernel_init()))
+    return rc;
   if (!n || off[n] >= 0x20000000ull || up_off[n] >= 0x20000000ull) return BF_OK;
   std::vector<uint32_t> up_end(up_off[n]), up_w(up_off[n]);
   parallel_for((n + 65535) / 65536, [&](uint64_t c) {
@@ -228,7 +250,8 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
         up_w[e] = up_rec[e].y;
       }
   });
-  const Edges dn{off.data(), src.data(), w.data()}, up{up_off.data(), up_end.data(), up_w.data()};
+  const Edges dn{off.data(), src.data(), w.data(), len};
+  const Edges up{up_off.data(), up_end.data(), up_w.data(), up_len};
   // chunks of whole runs
   std::vector<uint32_t> cut{0};
   const uint32_t step = std::max<uint32_t>(4096, n / 512);
@@ -346,6 +369,7 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
   nw += PANEL_ROWS * PANEL_ROWS;  // (a tile of 12 rows may be read as one of 16)
   std::vector<uint32_t> s(ns), t(nw, P.absent), us(up_ns), ut(up_nw);
   std::vector<uint16_t> em(ns);
+  std::vector<uint32_t> tl(len ? nw : 0, INF), utl(len ? up_nw : 0);
   parallel_for(nc, [&](uint64_t c) {
     std::copy(ch[c].src.begin(), ch[c].src.end(), s.begin() + sbase[c]);
     std::copy(ch[c].em.begin(), ch[c].em.end(), em.begin() + sbase[c]);
@@ -353,6 +377,8 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
                    [&](uint32_t x) { return x == INF ? P.absent : x; });
     std::copy(ch[c].up_end.begin(), ch[c].up_end.end(), us.begin() + up_sbase[c]);
     std::copy(ch[c].up_w.begin(), ch[c].up_w.end(), ut.begin() + up_wbase[c]);
+    std::copy(ch[c].len.begin(), ch[c].len.end(), tl.begin() + (len ? wbase[c] : 0));
+    std::copy(ch[c].up_len.begin(), ch[c].up_len.end(), utl.begin() + (len ? up_wbase[c] : 0));
     ch[c] = Chunk();
   });
   if ((rc = upload(&P.d_a, a, P)) || (rc = upload(&P.d_b, b, P)) ||
@@ -361,7 +387,8 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
       (rc = upload(&P.d_w, t, P)) || (rc = upload(&P.d_em, em, P)) ||
       (rc = upload(&P.d_tm, tm, P)) ||
       (rc = upload(&P.d_up, up_a, P)) || (rc = upload(&P.d_up_end, us, P)) ||
-      (rc = upload(&P.d_up_w, ut, P)) || (rc = pack_weights(P, nw))) {
+      (rc = upload(&P.d_up_w, ut, P)) || (len && (rc = upload(&P.d_len, tl, P))) ||
+      (len && (rc = upload(&P.d_up_len, utl, P))) || (rc = pack_weights(P, nw))) {
     free_panels(P);
     return rc == BF_ERR_OOM ? BF_OK : rc;
   }

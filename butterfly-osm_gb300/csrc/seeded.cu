@@ -184,14 +184,18 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
   const uint64_t wave = std::min<uint64_t>(max_lanes, (S + 3) & ~3ull);
   const uint32_t Kp = (uint32_t)((wave + 3) & ~3ull);
   if ((rc = ensure_slab(g, c, (size_t)rows * Kp * 4))) return rc;
-  // device copies: target seeds {rank, part}, target offsets, units, output
-  Dev d_ts, d_to, d_units, d_out;
-  if (!d_ts.alloc(nt * 8) || !d_to.alloc((T + 1) * 8) || !d_units.alloc(ns * 12) ||
-      !d_out.alloc(std::min<uint64_t>(wave, S) * T * 4))
-    return BF_ERR_OOM;
+  // device copies: [target offsets | target seeds {rank, part} | units | cells]
   static_assert(sizeof(bf_seed) == 8, "bf_seed is two u32");
-  BF_CUDA(cudaMemcpyAsync(d_ts.p, tgt_seeds, nt * 8, cudaMemcpyHostToDevice, s));
-  BF_CUDA(cudaMemcpyAsync(d_to.p, tgt_off, (T + 1) * 8, cudaMemcpyHostToDevice, s));
+  void* buf = nullptr;
+  if ((rc = call_buffer(c, (T + 1) * 8 + nt * 8 + ns * 12 + std::min<uint64_t>(wave, S) * T * 4,
+                        &buf)))
+    return rc;
+  uint64_t* d_to = static_cast<uint64_t*>(buf);
+  uint2* d_ts = reinterpret_cast<uint2*>(d_to + T + 1);
+  uint32_t* du = reinterpret_cast<uint32_t*>(d_ts + nt);
+  uint32_t* d_out = du + ns * 3;
+  BF_CUDA(cudaMemcpyAsync(d_ts, tgt_seeds, nt * 8, cudaMemcpyHostToDevice, s));
+  BF_CUDA(cudaMemcpyAsync(d_to, tgt_off, (T + 1) * 8, cudaMemcpyHostToDevice, s));
   const unsigned tpb = std::min<uint32_t>(128, ((Kp / 4 + 31) / 32) * 32);
   const unsigned lane_blocks = (Kp / 4 + tpb - 1) / tpb;
   uint64_t launches = 0;
@@ -206,7 +210,6 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
         units[nu + k - u0] = src_seeds[k].cost;
         units[2 * nu + k - u0] = (uint32_t)(si - s0);
       }
-    uint32_t* du = d_units.as<uint32_t>();
     if (nu) BF_CUDA(cudaMemcpyAsync(du, units.data(), units.size() * 4, cudaMemcpyHostToDevice, s));
     if ((rc = prepare_rows(g, c, sc, du, nu, Kp, s, &launches, max_seed))) return rc;
     if (nu) {
@@ -219,14 +222,14 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
                            max_seed)))
       return rc;
     dim3 eg((unsigned)((T + 31) / 32), (unsigned)((kw + 31) / 32)), eb(32, 8);
-    k_seeded_extract<<<eg, eb, 0, s>>>(c.d_slab, Kp, sc.d_cidx, d_to.as<uint64_t>(),
-                                       d_ts.as<uint2>(), T, (uint32_t)kw, threshold,
-                                       unreachable_from(g, sc, max_seed), d_out.as<uint32_t>());
+    k_seeded_extract<<<eg, eb, 0, s>>>(c.d_slab, Kp, sc.d_cidx, d_to, d_ts, T, (uint32_t)kw,
+                                       threshold, unreachable_from(g, sc, max_seed), d_out);
     BF_CUDA(cudaGetLastError());
     ++launches;
-    BF_CUDA(cudaMemcpyAsync(out + s0 * T, d_out.p, kw * T * 4, cudaMemcpyDeviceToHost, s));
+    BF_CUDA(cudaMemcpyAsync(out + s0 * T, d_out, kw * T * 4, cudaMemcpyDeviceToHost, s));
     BF_CUDA(cudaStreamSynchronize(s));  // units is rebuilt for the next wave
   }
+  trim_call_buffer(c);
   if ((rc = check_device_error(g, s))) return rc;
   // same-rank pairs belong to the caller's bucket engine (bucket_ch.rs:6786-6845)
   std::unordered_map<uint32_t, std::vector<uint32_t>> src_at;

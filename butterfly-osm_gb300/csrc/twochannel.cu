@@ -354,6 +354,8 @@ static bf_status launch_upward_2ch(Graph* g, const uint32_t* d_units, uint64_t n
                                    uint32_t threshold, const uint32_t* cidx, uint64_t* slab,
                                    uint32_t stride, uint32_t* flag, cudaStream_t st) {
   if (!nu) return BF_OK;
+  if (upward_2ch_by_panels(g))
+    return launch_upward_2ch_panels(g, d_units, nu, threshold, cidx, slab, stride, flag, st);
   const uint32_t dcap = ((g->max_depth + 1) + 31) & ~31u;
   const uint32_t *ur = d_units, *uc = d_units + nu, *ul = d_units + 2 * nu,
                  *ua = d_units + 3 * nu;
@@ -401,8 +403,9 @@ bf_status matrix_seeded_2ch(Graph* g, Ctx& c, const bf_seed2* src_seeds, const u
   for (uint64_t k = 0; k < nt; ++k) tr[k] = tgt_seeds[k].rank;
   std::sort(tr.begin(), tr.end());
   tr.erase(std::unique(tr.begin(), tr.end()), tr.end());
-  if ((rc = build_schedule(g, c, c.sc, tr.data(), tr.size(), false, s, nullptr, true))) return rc;
+  if ((rc = build_schedule(g, c, c.sc, tr.data(), tr.size(), false, s, nullptr, 2))) return rc;
   Sched& sc = c.sc;
+  if (st && (rc = start_counts(g, c, sc, s))) return rc;
   const uint64_t rows = std::max<uint32_t>(sc.n_r, 1);
   uint64_t max_lanes = ctx_budget(g, c) / (rows * 8 + (uint64_t)T * 4 * 2 * 2);
   max_lanes = max_lanes >= 32 ? max_lanes & ~31ull : 0;
@@ -416,15 +419,18 @@ bf_status matrix_seeded_2ch(Graph* g, Ctx& c, const bf_seed2* src_seeds, const u
   if ((rc = ensure_slab(g, c, (size_t)rows * Kp2 * 8))) return rc;
   uint64_t* slab = reinterpret_cast<uint64_t*>(c.d_slab);
   static_assert(sizeof(bf_seed2) == 12, "bf_seed2 is three u32");
-  Dev d_ts, d_to, d_units, d_out;
+  // [target offsets | target seeds | units | times | lengths]
   const uint64_t out_cells = std::min<uint64_t>(wave, S) * T;
-  if (!d_ts.alloc(nt * 12) || !d_to.alloc((T + 1) * 8) || !d_units.alloc(src_off[S] * 16) ||
-      !d_out.alloc(out_cells * 8))
-    return BF_ERR_OOM;
-  BF_CUDA(cudaMemcpyAsync(d_ts.p, tgt_seeds, nt * 12, cudaMemcpyHostToDevice, s));
-  BF_CUDA(cudaMemcpyAsync(d_to.p, tgt_off, (T + 1) * 8, cudaMemcpyHostToDevice, s));
-  uint32_t* d_ot = d_out.as<uint32_t>();
+  void* buf = nullptr;
+  if ((rc = call_buffer(c, (T + 1) * 8 + nt * 12 + src_off[S] * 16 + out_cells * 8, &buf)))
+    return rc;
+  uint64_t* d_to = static_cast<uint64_t*>(buf);
+  uint32_t* d_ts = reinterpret_cast<uint32_t*>(d_to + T + 1);
+  uint32_t* du = d_ts + nt * 3;
+  uint32_t* d_ot = du + src_off[S] * 4;
   uint32_t* d_ol = d_ot + out_cells;
+  BF_CUDA(cudaMemcpyAsync(d_ts, tgt_seeds, nt * 12, cudaMemcpyHostToDevice, s));
+  BF_CUDA(cudaMemcpyAsync(d_to, tgt_off, (T + 1) * 8, cudaMemcpyHostToDevice, s));
   const unsigned tpb = std::min<uint32_t>(128, ((Kp2 / 2 + 31) / 32) * 32);
   const unsigned lane_blocks = (Kp2 / 2 + tpb - 1) / tpb;
   uint64_t launches = 0;
@@ -446,13 +452,13 @@ bf_status matrix_seeded_2ch(Graph* g, Ctx& c, const bf_seed2* src_seeds, const u
       units[2 * nu + i] = kept[i].len;
       units[3 * nu + i] = lane_of[i];
     }
-    uint32_t* du = d_units.as<uint32_t>();
     if (nu) BF_CUDA(cudaMemcpyAsync(du, units.data(), units.size() * 4, cudaMemcpyHostToDevice, s));
-    // rows hold Kp2 u64 lanes = 2 * Kp2 u32 words
-    if ((rc = prepare_rows(g, c, sc, du, nu, 2 * Kp2, s, &launches))) return rc;
+    // rows hold Kp2 u64 lanes = 2 * Kp2 u32 words, reset to INF in both forms
+    if ((rc = prepare_rows(g, c, sc, du, nu, 2 * Kp2, s, &launches, INF))) return rc;
     if ((rc = launch_upward_2ch(g, du, nu, INF, sc.d_cidx, slab, Kp2, nullptr, s))) return rc;
     if (nu) ++launches;
-    for (uint32_t l = 0; l < g->n_levels; ++l) {
+    if (sc.panel) BF_CUDA(sweep_panels_2ch(g, sc, slab, Kp2, s, &launches, c.d_seeded));
+    for (uint32_t l = 0; !sc.panel && l < g->n_levels; ++l) {
       const uint32_t i0 = sc.lvl_item[l], i1 = sc.lvl_item[l + 1];
       if (i1 == i0) continue;
       dim3 grid(i1 - i0, lane_blocks);
@@ -462,14 +468,15 @@ bf_status matrix_seeded_2ch(Graph* g, Ctx& c, const bf_seed2* src_seeds, const u
     }
     BF_CUDA(cudaGetLastError());
     dim3 eg((unsigned)((T + 31) / 32), (unsigned)((kw + 31) / 32)), eb(32, 8);
-    k_extract_2ch<<<eg, eb, 0, s>>>(slab, Kp2, sc.d_cidx, d_to.as<uint64_t>(),
-                                    d_ts.as<uint32_t>(), T, (uint32_t)kw, threshold, d_ot, d_ol);
+    k_extract_2ch<<<eg, eb, 0, s>>>(slab, Kp2, sc.d_cidx, d_to, d_ts, T, (uint32_t)kw, threshold,
+                                    d_ot, d_ol);
     BF_CUDA(cudaGetLastError());
     ++launches;
     BF_CUDA(cudaMemcpyAsync(out_time + s0 * T, d_ot, kw * T * 4, cudaMemcpyDeviceToHost, s));
     BF_CUDA(cudaMemcpyAsync(out_len + s0 * T, d_ol, kw * T * 4, cudaMemcpyDeviceToHost, s));
     BF_CUDA(cudaStreamSynchronize(s));  // units is rebuilt for the next wave
   }
+  trim_call_buffer(c);
   if ((rc = check_device_error(g, s))) return rc;
   // same-rank pairs belong to the caller's two-channel bucket engine
   // (bucket_ch.rs:6460-6463, :6497-6516)
@@ -492,10 +499,11 @@ bf_status matrix_seeded_2ch(Graph* g, Ctx& c, const bf_seed2* src_seeds, const u
   if (n_conflicts) *n_conflicts = cells.size();
   for (uint64_t i = 0; i < cells.size() && i < conflict_cap; ++i) conflicts[i] = cells[i];
   if (st) {
+    if ((rc = finish_counts(c, sc))) return rc;
     st->n_batches += (S + wave - 1) / wave;
     st->waves += (S + wave - 1) / wave;
     st->kernel_launches += launches;
-    st->swept_nodes = sc.n_r;
+    st->swept_nodes = sc.n_live;
     st->swept_edges = sc.n_edges;
     st->lanes = Kp2;
   }

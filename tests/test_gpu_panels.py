@@ -191,3 +191,57 @@ def test_isochrones_panels_budget_falls_back(built, country_small):
             assert e.status == bfphast.BF_ERR_OOM and not served, mb
         g.close()
     assert served
+
+
+def _with_lengths(cch, seed):
+    """Few distinct times, so that ties occur everywhere, and lengths; INF kept."""
+    rng = np.random.default_rng(seed)
+    d, ln = dict(cch), []
+    for key in ("up_w", "down_w"):
+        w = np.asarray(cch[key], np.uint32)
+        d[key] = np.where(w == INF, w, rng.integers(0, 4, len(w)).astype(np.uint32))
+        ln.append(np.where(w == INF, w, rng.integers(0, 5000, len(w)).astype(np.uint32)))
+    return d, ln[0], ln[1]
+
+
+@pytest.mark.parametrize("name", ["band2", "band16", "band17", "band33", "sources300", "fan"])
+def test_panels_two_channel(built, name):
+    import bfphast
+    up, _, _ = GRAPHS[name]
+    n = len(up)
+    d, ul, dl = _with_lengths(_cch(n, up, 5, 1, 60, 0.2), 6)
+    c = orc.Cch.from_dict(d)
+    g = bfphast.Graph.from_cch(d, up_len=ul, down_len=dl)
+    rng = np.random.default_rng(n)
+
+    def sets(m):
+        return [[(int(rng.integers(0, n)), int(rng.integers(0, 8)), int(rng.integers(0, 500)))
+                 for _ in range(int(rng.integers(1, 4)))] for _ in range(m)]
+
+    for S, T in ((1, 1), (33, 40), (70, 9)):
+        src, tgt = sets(S), sets(T)
+        got = g.matrix_seeded_2ch(src, tgt, with_conflicts=True)
+        want = orc.table_phast_lopsided_2ch(c, src, tgt, INF, ul, dl)
+        assert all(np.array_equal(a, b) for a, b in zip(got, want)), (S, T)
+    for thr in (0, 3, 25, INF):
+        seeds = sets(1)[0]
+        got, want = g.phast_bounded_seeded_2ch(seeds, thr), c.bounded_seeded_2ch(seeds, thr, ul, dl)
+        assert all(np.array_equal(a, b) for a, b in zip(got, want)), thr
+
+
+def test_panels_two_channel_wide_levels(built, grid100):
+    """Levels of more units than blocks (a warp per unit) against the item sweep."""
+    import bfphast
+    d, ul, dl = _with_lengths(grid100[1], 2)
+    n = d["n"]
+    rng = np.random.default_rng(8)
+    src = [[(int(r), 0, 0)] for r in rng.choice(n, 70, replace=False)]
+    tgt = [[(int(r), 1, 1)] for r in rng.choice(n, 3000, replace=False)]
+    g = bfphast.Graph.from_cch(d, up_len=ul, down_len=dl)
+    got = g.matrix_seeded_2ch(src, tgt)
+    g.set_tune(device_schedule=0)
+    want = g.matrix_seeded_2ch(src, tgt)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    c = orc.Cch.from_dict(d)
+    ref = orc.table_phast_lopsided_2ch(c, src[:4], tgt, INF, ul, dl)
+    assert np.array_equal(got[0][:4], ref[0]) and np.array_equal(got[1][:4], ref[1])
