@@ -684,16 +684,19 @@ bf_status bf_query_batch(bf_graph* h, const uint32_t* src, uint32_t k, uint32_t 
   std::lock_guard<std::mutex> lk(g->mu);
   if (cudaSetDevice(g->device) != cudaSuccess) return cuda_status(cudaGetLastError(), "cudaSetDevice");
   cudaStream_t s = g->stream;
-  DevBuf ds, dout;
-  if ((rc = ds.alloc(k * 4)) || (rc = dout.alloc((size_t)k * g->n * 4))) return rc;
-  BF_CUDA(cudaMemcpyAsync(ds.p, src, k * 4, cudaMemcpyHostToDevice, s));
-  // every rank is a target: positions are the rank -> position table itself
-  if ((rc = plain_matrix(g, ds.as<uint32_t>(), k, g->d_pos_of, g->n, threshold,
-                         dout.as<uint32_t>(), s, nullptr)))
+  void* buf = nullptr;
+  const size_t out_bytes = (size_t)k * g->n * 4;
+  if ((rc = call_buffer(g->ctx, out_bytes + k * 4, &buf))) return rc;
+  uint32_t* d_out = static_cast<uint32_t*>(buf);
+  uint32_t* d_src = d_out + (size_t)k * g->n;
+  BF_CUDA(cudaMemcpyAsync(d_src, src, k * 4, cudaMemcpyHostToDevice, s));
+  // every rank is a target: positions are the rank -> row table itself
+  if ((rc = plain_matrix(g, d_src, k, plain_rows(g), g->n, threshold, d_out, s, nullptr)))
     return rc;
   if ((rc = check_device_error(g, s))) return rc;
-  BF_CUDA(cudaMemcpyAsync(dist_out, dout.p, (size_t)k * g->n * 4, cudaMemcpyDeviceToHost, s));
+  BF_CUDA(cudaMemcpyAsync(dist_out, d_out, out_bytes, cudaMemcpyDeviceToHost, s));
   BF_CUDA(cudaStreamSynchronize(s));
+  trim_call_buffer(g->ctx);
   return BF_OK;
 }
 

@@ -10,6 +10,9 @@
 //      lane = source. dist[v][lane] = min(seed, min over DOWN in-edges
 //      (u -> v, w) of dist[u][lane] + w) — the pull form of the rank-
 //      descending push scan of batched_phast.rs:205-250.
+//      By default all levels are walked by one cooperative launch: over panels
+//      (plainpanel.cu) where the graph has them and their upward pass fits,
+//      else k_plain_persist.
 //   3. k_extract: gathers the target rows and writes the S x T row-major
 //      matrix through a shared-memory transpose (batched_phast.rs:693-701).
 
@@ -336,7 +339,8 @@ __global__ void __launch_bounds__(512)
   }
 }
 
-// out[(row0 + l) * T + t] = slab[tpos[t]][l] for l < k; tiles of 32 targets.
+// out[(row0 + l) * T + t] = slab[tpos[t]][l] for l < k (tpos null: row t); tiles of
+// 32 targets.
 __global__ void __launch_bounds__(256)
     k_extract(const uint32_t* __restrict__ slab, uint32_t slab_stride,
               const uint32_t* __restrict__ tpos, uint64_t T, uint32_t k,
@@ -345,7 +349,7 @@ __global__ void __launch_bounds__(256)
   const uint64_t t0 = (uint64_t)blockIdx.x * 32;
   for (uint32_t r = threadIdx.y; r < 32; r += 8) {
     uint64_t t = t0 + r;
-    tile[r][threadIdx.x] = (t < T) ? slab[(size_t)tpos[t] * slab_stride + threadIdx.x] : INF;
+    tile[r][threadIdx.x] = (t < T) ? slab[(size_t)(tpos ? tpos[t] : t) * slab_stride + threadIdx.x] : INF;
   }
   __syncthreads();
   for (uint32_t l = threadIdx.y; l < k; l += 8) {
@@ -364,14 +368,22 @@ __global__ void k_to_positions(const uint32_t* __restrict__ ranks, uint64_t m,
     atomicOr(err, DEVERR_PATH);
     pos[i] = 0;
   } else {
-    pos[i] = pos_of[r];
+    pos[i] = pos_of ? pos_of[r] : r;
   }
 }
+
+// Whether the persistent plain sweep walks panels: their upward pass writes its
+// seeds by rank, where the panels are swept in place.
+static bool plain_by_panels(const Graph* g) {
+  return (g->tune.persist & 1u) && upward_by_panels(g);
+}
+
+const uint32_t* plain_rows(const Graph* g) { return plain_by_panels(g) ? nullptr : g->d_pos_of; }
 
 bf_status to_positions(Graph* g, const uint32_t* d_rank, uint64_t m, uint32_t* d_pos,
                        cudaStream_t st) {
   if (!m) return BF_OK;
-  k_to_positions<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(d_rank, m, g->d_pos_of, g->n, d_pos,
+  k_to_positions<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(d_rank, m, plain_rows(g), g->n, d_pos,
                                                               g->d_err);
   BF_CUDA(cudaGetLastError());
   return BF_OK;
@@ -490,7 +502,7 @@ bf_status launch_upward(Graph* g, const uint32_t* d_src, uint64_t k, uint32_t th
 
 static bf_status plain_upward(Graph* g, const uint32_t* d_src, uint32_t k, uint32_t threshold,
                               cudaStream_t st) {
-  return launch_upward(g, d_src, k, threshold, g->d_pos_of, g->d_seed, PLAIN_K, g->d_flag, st);
+  return launch_upward(g, d_src, k, threshold, plain_rows(g), g->d_seed, PLAIN_K, g->d_flag, st);
 }
 
 // Blocks of a persistent launch: as many as are co-resident (the cooperative
@@ -550,6 +562,7 @@ static bf_status plain_sweep_persistent(Graph* g, uint32_t threshold, cudaStream
 }
 
 static bf_status plain_sweep(Graph* g, uint32_t threshold, cudaStream_t st, uint64_t* launches) {
+  if (plain_by_panels(g)) return plain_sweep_panels(g, threshold, st, launches);
   if (g->tune.persist & 1u) return plain_sweep_persistent(g, threshold, st, launches);
   for (uint32_t l = 0; l < g->n_levels; ++l) {
     uint32_t p0 = g->lvl_start[l], p1 = g->lvl_start[l + 1];

@@ -1,0 +1,291 @@
+// plainpanel.cu — the plain engine's sweep over panels: every node of the graph,
+// K = 32 sources, in one cooperative launch.
+//
+// Slab rows are ranks (row j of a panel is rank hi - j), a lane a source. The
+// blocks walk the levels of the panel DAG with a grid barrier between them; each
+// row is written once, by its panel, so the slab needs no initial values: seeds
+// lie in a second slab, with a bit per seeded row.
+
+#include <algorithm>
+
+#include "engine.cuh"
+
+namespace bf {
+
+namespace {
+
+constexpr uint32_t PP_WARPS = 8;
+constexpr uint32_t PP_CH = 16;  // sources of a chunk: their rows are in flight together
+
+struct PlainArgs {
+  const uint4* a;       // Panels::d_a, d_b, d_lvl
+  const uint2* b;
+  const uint32_t* lvl;
+  uint32_t n_levels;
+  const uint32_t *src, *w;
+  uint32_t absent;
+  uint32_t *dist, *seed, *flag;
+  uint32_t threshold;
+};
+
+struct PlainSmem {
+  uint32_t w[PP_WARPS][PP_CH * PANEL_ROWS];         // a chunk's tile per warp
+  uint32_t tri[PP_WARPS][PANEL_ROWS * PANEL_ROWS];  // a panel's triangle per warp
+  uint32_t red[PP_WARPS][PANEL_ROWS][32];           // minima of a shared panel's warps
+  uint32_t seed[PANEL_ROWS][32];                    // and its seeds
+};
+
+__device__ __forceinline__ uint32_t min_plus(uint32_t d, uint32_t w, uint32_t acc) {
+  return __viaddmin_u32(min(d, ~w), w, acc);  // min(acc, d + w), the sum saturating at INF
+}
+
+__device__ __forceinline__ uint32_t stride_of(const uint4& a) { return (a.y >> 8) & 0xFF; }
+
+// Sources per warp of a chunk.
+template <bool SHARED>
+__device__ __forceinline__ uint32_t chunk_of(uint32_t nu) {
+  return SHARED ? min(PP_CH, (nu + PP_WARPS - 1) / PP_WARPS) : PP_CH;
+}
+
+// A chunk's source ids (a lane each) and tile, into registers.
+template <uint32_t K>
+__device__ __forceinline__ void load_chunk(const PlainArgs& g, const uint2 b, uint32_t c0,
+                                           uint32_t m, uint32_t lane, uint32_t* id,
+                                           uint32_t (&wv)[K / 2]) {
+  *id = lane < m ? __ldg(g.src + b.x + c0 + lane) : 0u;
+  const uint32_t* tile = g.w + b.y + (size_t)c0 * K;
+#pragma unroll
+  for (uint32_t i = 0; i < K / 2; ++i)
+    wv[i] = i * 32 + lane < m * K ? __ldg(tile + i * 32 + lane) : INF;
+}
+
+template <uint32_t K>
+__device__ __forceinline__ void store_chunk(const PlainArgs& g, uint32_t* ws, uint32_t lane,
+                                            const uint32_t (&wv)[K / 2]) {
+#pragma unroll
+  for (uint32_t i = 0; i < K / 2; ++i) ws[i * 32 + lane] = wv[i] == g.absent ? INF : wv[i];
+}
+
+template <uint32_t K>
+__device__ __forceinline__ void load_triangle(const PlainArgs& g, const uint4 a, const uint2 b,
+                                              uint32_t lane, uint32_t* tri) {
+  const uint32_t* t = g.w + b.y + (size_t)a.z * K;
+#pragma unroll
+  for (uint32_t i = 0; i < K * K; i += 32)
+    if (i + lane < K * K) {
+      const uint32_t v = __ldg(t + i + lane);
+      tri[i + lane] = v == g.absent ? INF : v;
+    }
+}
+
+// Row r's seeds, read and given back (its bit f is set).
+__device__ __forceinline__ uint32_t take_seed(const PlainArgs& g, uint32_t r, uint32_t lane) {
+  uint32_t* at = g.seed + (size_t)r * PLAIN_K + lane;
+  const uint32_t v = *at;
+  *at = INF;
+  __syncwarp();
+  if (lane == 0) atomicAnd(g.flag + (r >> 5), ~(1u << (r & 31)));
+  return v;
+}
+
+// What a shared panel needs that no earlier level writes: each warp's first
+// chunk, the triangle and the seeds. Returns the warp's source ids.
+template <uint32_t K>
+__device__ __forceinline__ uint32_t stage_shared(const PlainArgs& g, const uint4 a, const uint2 b,
+                                                 PlainSmem& sm) {
+  const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const uint32_t ch = chunk_of<true>(a.z), c0 = wib * ch;
+  uint32_t id = 0, wv[K / 2];
+  if (c0 < a.z) load_chunk<K>(g, b, c0, min(ch, a.z - c0), lane, &id, wv);
+  if (wib == PP_WARPS - 1) load_triangle<K>(g, a, b, lane, sm.tri[0]);
+  for (uint32_t j = wib; j < (a.y & 0xFF); j += PP_WARPS) {
+    const uint32_t r = a.x - j;
+    sm.seed[j][lane] =
+        (__ldcg(g.flag + (r >> 5)) >> (r & 31)) & 1u ? take_seed(g, r, lane) : INF;
+  }
+  if (c0 < a.z) store_chunk<K>(g, sm.w[wib], lane, wv);
+  return id;
+}
+
+// A panel (stride K) by one warp, or with SHARED by all warps of the block, a
+// chunk of the sources each, staged before (id: its first chunk's ids).
+template <uint32_t K, bool SHARED>
+__device__ __forceinline__ void plain_panel(const PlainArgs& g, const uint4 a, const uint2 b,
+                                            uint32_t id, PlainSmem& sm) {
+  const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const uint32_t rows = a.y & 0xFF, nu = a.z;
+  uint32_t* ws = sm.w[wib];
+  uint32_t* tri = sm.tri[SHARED ? 0 : wib];
+  const uint32_t ch = chunk_of<SHARED>(nu), step = SHARED ? PP_WARPS * ch : ch;
+  uint32_t c0 = SHARED ? wib * ch : 0;
+  uint32_t wv[K / 2];
+  if (!SHARED) {
+    if (nu) load_chunk<K>(g, b, 0, min(ch, nu), lane, &id, wv);
+    load_triangle<K>(g, a, b, lane, tri);
+    if (nu) store_chunk<K>(g, ws, lane, wv);
+  }
+  __syncwarp();
+  uint32_t acc[K];
+#pragma unroll
+  for (uint32_t j = 0; j < K; ++j) acc[j] = INF;
+  while (c0 < nu) {
+    const uint32_t m = min(ch, nu - c0), next = c0 + step;
+    uint32_t d[PP_CH];
+#pragma unroll
+    for (uint32_t s = 0; s < PP_CH; ++s) {
+      const uint32_t r = __shfl_sync(0xFFFFFFFFu, id, s);
+      d[s] = s < m ? __ldcg(g.dist + (size_t)r * PLAIN_K + lane) : INF;
+    }
+    if (next < nu) load_chunk<K>(g, b, next, min(ch, nu - next), lane, &id, wv);
+#pragma unroll
+    for (uint32_t s = 0; s < PP_CH; ++s) {
+      if (s >= m) break;
+#pragma unroll
+      for (uint32_t j = 0; j < K; j += 4) {
+        const uint4 x = *reinterpret_cast<const uint4*>(ws + s * K + j);
+        acc[j] = min_plus(d[s], x.x, acc[j]);
+        acc[j + 1] = min_plus(d[s], x.y, acc[j + 1]);
+        acc[j + 2] = min_plus(d[s], x.z, acc[j + 2]);
+        acc[j + 3] = min_plus(d[s], x.w, acc[j + 3]);
+      }
+    }
+    __syncwarp();
+    if (next < nu) store_chunk<K>(g, ws, lane, wv);
+    __syncwarp();
+    c0 = next;
+  }
+  if (SHARED) {
+#pragma unroll
+    for (uint32_t j = 0; j < K; ++j) sm.red[wib][j][lane] = acc[j];
+    __syncthreads();
+    for (uint32_t j = wib; j < rows; j += PP_WARPS) {
+      uint32_t v = sm.seed[j][lane];
+#pragma unroll
+      for (uint32_t q = 0; q < PP_WARPS; ++q) v = min(v, sm.red[q][j][lane]);
+      sm.red[0][j][lane] = v;
+    }
+    __syncthreads();
+  }
+  if (!SHARED || wib == 0) {
+    if (SHARED) {
+#pragma unroll
+      for (uint32_t j = 0; j < K; ++j) acc[j] = sm.red[0][j][lane];
+    } else {
+      const uint32_t w0 = (a.x + 1 - rows) >> 5, w1 = a.x >> 5;
+      const uint32_t f0 = __ldcg(g.flag + w0), f1 = w1 == w0 ? f0 : __ldcg(g.flag + w1);
+#pragma unroll
+      for (uint32_t j = 0; j < K; ++j) {
+        const uint32_t r = a.x - j;
+        if (j < rows && (((r >> 5) == w0 ? f0 : f1) >> (r & 31)) & 1u)
+          acc[j] = min(acc[j], take_seed(g, r, lane));
+      }
+    }
+#pragma unroll
+    for (uint32_t i = 0; i + 1 < K; ++i)
+#pragma unroll
+      for (uint32_t v = (i + 1) / 4; v < K / 4; ++v) {
+        const uint4 x = *reinterpret_cast<const uint4*>(tri + i * K + 4 * v);
+        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q)
+          if (4 * v + q > i) acc[4 * v + q] = min_plus(acc[i], w[q], acc[4 * v + q]);
+      }
+#pragma unroll
+    for (uint32_t j = 0; j < K; ++j)
+      if (j < rows)
+        g.dist[(size_t)(a.x - j) * PLAIN_K + lane] = acc[j] > g.threshold ? INF : acc[j];
+    __syncwarp();  // (the warp's next panel writes the shared tile and triangle)
+  }
+  if (SHARED) __syncthreads();
+}
+
+#define BF_BY_STRIDE(a, CALL)      \
+  switch (stride_of(a)) {          \
+    case 4: CALL(4); break;        \
+    case 8: CALL(8); break;        \
+    case 12: CALL(12); break;      \
+    default: CALL(16);             \
+  }
+
+// Bound by the chain of levels: a grid barrier and the dependent reads of
+// each. A level with few panels has a block share each one, what no earlier
+// level writes staged before the barrier; else every warp takes panels of its
+// own: once a block's turn comes round more than four times, its warps do
+// better apart (twice or once: within 3 %). `withhold` (a test hook, NONE otherwise) names a block that leaves
+// before its first barrier arrival.
+//
+// Two blocks an SM: three and four spill. Eight sources to all of the town's
+// 119,260 nodes: sweep 615 -> 230 us, whole call 862 -> 341; one source on
+// grid100 2250 -> 530 us; 8 sources on the 1000 x 1250 region 8.0 -> 6.9 ms, of
+// which most is the copy back.
+__global__ void __launch_bounds__(32 * PP_WARPS, 2)
+    k_plain_panels(const PlainArgs g, uint32_t* __restrict__ bar, long long timeout,
+                   uint32_t withhold, uint32_t* __restrict__ err) {
+  __shared__ __align__(16) PlainSmem sm;
+  if (blockIdx.x == withhold) return;
+  const uint32_t share = 4 * gridDim.x;
+  uint4 a = make_uint4(0, 0, 0, 0);
+  uint2 b = make_uint2(0, 0);
+  uint32_t id = 0;
+  auto stage = [&](uint32_t p) {
+    a = g.a[p];
+    b = g.b[p];
+#define BF_STAGE(K) id = stage_shared<K>(g, a, b, sm)
+    BF_BY_STRIDE(a, BF_STAGE)
+#undef BF_STAGE
+  };
+  uint32_t p0 = g.lvl[0], p1 = g.lvl[1];
+  bool staged = false;
+  for (uint32_t l = 0; l < g.n_levels; ++l) {
+    const uint32_t p2 = l + 1 < g.n_levels ? g.lvl[l + 2] : p1;
+    if (p1 - p0 <= share) {
+      for (uint32_t p = p0 + blockIdx.x; p < p1; p += gridDim.x) {
+        if (!staged) stage(p);
+        staged = false;
+#define BF_SOLVE(K) plain_panel<K, true>(g, a, b, id, sm)
+        BF_BY_STRIDE(a, BF_SOLVE)
+#undef BF_SOLVE
+      }
+    } else {
+      for (uint32_t p = p0 + blockIdx.x * PP_WARPS + (threadIdx.x >> 5); p < p1;
+           p += gridDim.x * PP_WARPS) {
+        const uint4 wa = g.a[p];
+        const uint2 wb = g.b[p];
+#define BF_SOLVE(K) plain_panel<K, false>(g, wa, wb, 0, sm)
+        BF_BY_STRIDE(wa, BF_SOLVE)
+#undef BF_SOLVE
+      }
+      __syncthreads();
+    }
+    if (l + 1 == g.n_levels) break;
+    if (p2 - p1 <= share && p1 + blockIdx.x < p2) {
+      stage(p1 + blockIdx.x);
+      staged = true;
+    }
+    if (!grid_barrier(bar, l, timeout, err)) return;
+    p0 = p1;
+    p1 = p2;
+  }
+}
+#undef BF_BY_STRIDE
+
+}  // namespace
+
+bf_status plain_sweep_panels(Graph* g, uint32_t threshold, cudaStream_t st, uint64_t* launches) {
+  bf_status s;
+  if ((s = ensure_barrier(g))) return s;
+  const Panels& P = g->panels;
+  const PlainArgs a{P.d_a,    P.d_b,     P.d_lvl,   P.n_levels, P.d_src, P.d_w,
+                    P.absent, g->d_dist, g->d_seed, g->d_flag,  threshold};
+  const bool hook = test_withhold_arrival();
+  const unsigned blocks =
+      persistent_blocks(g, (const void*)k_plain_panels, 32 * PP_WARPS, 2 * g->sm_count);
+  BF_CUDA(cudaMemsetAsync(g->d_bar, 0, 8, st));
+  BF_CUDA(launch_persistent(k_plain_panels, blocks, 32 * PP_WARPS, st, a, g->d_bar,
+                            hook ? 2000000ll : BARRIER_TIMEOUT_CYCLES, hook ? 1u : NONE,
+                            g->d_err));
+  ++*launches;
+  return BF_OK;
+}
+
+}  // namespace bf

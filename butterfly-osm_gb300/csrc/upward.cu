@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(UPWARD_WARPS * 32, 6)
           atomicOr(&flag[x], 1u << (w >> 6));
         }
       } else if (in) {
-        const uint32_t p = pos_of[x];
+        const uint32_t p = pos_of ? pos_of[x] : x;
         if (p != NONE) {
           if (unit_lane) atomicMin(&seed[(size_t)p * seed_stride + out_lane], d);
           else if (mode == UPWARD_OUT_SLAB16)  // (d is within its lane threshold, < 0xFFFF)

@@ -245,3 +245,30 @@ def test_panels_two_channel_wide_levels(built, grid100):
     c = orc.Cch.from_dict(d)
     ref = orc.table_phast_lopsided_2ch(c, src[:4], tgt, INF, ul, dl)
     assert np.array_equal(got[0][:4], ref[0]) and np.array_equal(got[1][:4], ref[1])
+
+
+@pytest.mark.parametrize("name", sorted(GRAPHS))
+def test_plain_sweep_by_panels(built, name):
+    """The plain engine's one-launch sweep (panels) and its launch per level
+    (rows) against the oracle: partial and whole batches, seeds taken back
+    between them, a threshold within the sweep, saturating sums."""
+    import bfphast
+    up, lo, hi = GRAPHS[name]
+    n = len(up)
+    cch = _cch(n, up, 7, lo, hi, 0.2)
+    c = orc.Cch.from_dict(cch)
+    g = bfphast.Graph.from_cch(cch)
+    g.set_engine(bfphast.ENGINE_PLAIN)
+    rng = np.random.default_rng(n)
+    every = np.arange(n, dtype=np.uint32)
+    for k in (1, 31, 32, 33, 100):
+        src = rng.integers(0, n, k).astype(np.uint32)
+        tgt = rng.integers(0, n, 7).astype(np.uint32)
+        want, _ = c.matrix(src, every)
+        for persist in (1, 0, 1):
+            g.set_tune(persistent_sweep=persist)
+            assert np.array_equal(g.query_batch(src), want), (k, persist)
+            assert np.array_equal(g.matrix(src, tgt), want[:, tgt]), (k, persist)
+            for thr in (0, lo, min(INF - 1, 5 * (hi // 2))):
+                got = g.matrix(src, tgt, threshold=thr)
+                assert np.array_equal(got, np.where(want[:, tgt] <= thr, want[:, tgt], INF)), thr
