@@ -84,16 +84,16 @@ __device__ __forceinline__ void relax_source(uint32_t v, const uint32_t* w, uint
   }
 }
 
-// The sources base + (set bits of bm) of a unit, four rows in flight. s: the
+// The sources base + (set bits of bm) of a unit, F rows in flight. s: the
 // source rank of base + lane.
-template <uint32_t K, bool SAT>
+template <uint32_t K, bool SAT, uint32_t F = 4>
 __device__ __forceinline__ void relax_active(uint32_t bm, uint32_t s, const uint32_t* w,
                                              uint32_t stride, const uint32_t* slab, uint32_t lane,
                                              uint32_t (&acc)[K]) {
   while (bm) {
-    uint32_t i[4], v[4];
+    uint32_t i[F], v[F];
 #pragma unroll
-    for (uint32_t q = 0; q < 4; ++q) {
+    for (uint32_t q = 0; q < F; ++q) {
       i[q] = bm ? __ffs(bm) - 1 : 32u;
       bm &= bm - 1;
       if (i[q] < 32) {
@@ -102,7 +102,7 @@ __device__ __forceinline__ void relax_active(uint32_t bm, uint32_t s, const uint
       }
     }
 #pragma unroll
-    for (uint32_t q = 0; q < 4; ++q)
+    for (uint32_t q = 0; q < F; ++q)
       if (i[q] < 32) relax_source<K, SAT>(v[q], w + (size_t)i[q] * stride, acc);
   }
 }
@@ -340,14 +340,17 @@ __global__ void __launch_bounds__(256, 4)
 }
 
 // A level of few panels: a block per unit (panel p0 + blockIdx.x, tile
-// blockIdx.y), each warp every eighth group of 32 sources. The weights of up to
-// 256 sources are staged while the level before drains.
+// blockIdx.y), each warp an eighth of up to 256 sources, whose weights are staged
+// while the level before drains, as are the seeds. Five origins on the 1000 x 1250
+// region, whole call: 1.31 ms against 1.44 with four rows in flight, groups of 32
+// sources a warp and the seeds read at the end.
 constexpr uint32_t ISO_WARPS = 8, ISO_CH = 256;
 struct IsoSplitSmem {
   uint32_t w[ISO_CH * PANEL_ROWS];
   uint32_t tri[PANEL_ROWS * PANEL_ROWS];
   uint32_t src[ISO_CH];
   uint32_t red[ISO_WARPS][PANEL_ROWS][32];
+  uint32_t seed[PANEL_ROWS][32];
 };
 
 template <uint32_t K, bool SAT>
@@ -366,12 +369,16 @@ __device__ __forceinline__ void iso_block_unit(const IsoArgs& g, const IsoPanel&
   for (uint32_t i = tid; i < p.stride * p.stride; i += TPB) sm.tri[i] = w[(size_t)p.nu * p.stride + i];
   const uint32_t seeds = lane < p.live ? g.seeded[p.hi - lane] : 0u;
   const uint32_t sd = __ballot_sync(FULL, (seeds >> t) & 1u);
+  uint32_t* slab = g.slab + (size_t)t * g.n * 32;
+  // (seeds are written before the first level is launched)
+  for (uint32_t j = warp; j < K; j += ISO_WARPS)
+    sm.seed[j][lane] =
+        (sd >> j) & 1u ? __ldcg(slab + (size_t)(p.hi - j) * 32 + lane) : far2<SAT>;
   __syncthreads();
   asm volatile("griddepcontrol.wait;" ::: "memory");
   uint32_t acc[K];
 #pragma unroll
   for (uint32_t j = 0; j < K; ++j) acc[j] = far2<SAT>;
-  uint32_t* slab = g.slab + (size_t)t * g.n * 32;
   uint32_t gathered = 0;
   for (uint32_t c0 = 0; c0 < p.nu; c0 += ISO_CH) {
     const uint32_t m = min(p.nu - c0, ISO_CH);
@@ -380,12 +387,14 @@ __device__ __forceinline__ void iso_block_unit(const IsoArgs& g, const IsoPanel&
       stage(c0, m);
       __syncthreads();
     }
-    for (uint32_t base = warp * 32; base < m; base += TPB) {
-      const uint32_t s = base + lane < m ? sm.src[base + lane] : 0u;
-      const uint32_t am = base + lane < m ? __ldcg(g.act + s) : 0u;
+    const uint32_t each = (m + ISO_WARPS - 1) / ISO_WARPS, base = warp * each;  // (at most 32)
+    if (base < m) {
+      const bool in = lane < each && base + lane < m;
+      const uint32_t s = in ? sm.src[base + lane] : 0u;
+      const uint32_t am = in ? __ldcg(g.act + s) : 0u;
       const uint32_t bm = __ballot_sync(FULL, (am >> t) & 1u);
       gathered += __popc(bm);
-      relax_active<K, SAT>(bm, s, sm.w + base * p.stride, p.stride, slab, lane, acc);
+      relax_active<K, SAT, 8>(bm, s, sm.w + base * p.stride, p.stride, slab, lane, acc);
     }
   }
   if (!__syncthreads_or(gathered | sd)) return;
@@ -393,9 +402,9 @@ __device__ __forceinline__ void iso_block_unit(const IsoArgs& g, const IsoPanel&
   for (uint32_t j = 0; j < K; ++j) sm.red[warp][j][lane] = acc[j];
   __syncthreads();
   for (uint32_t j = warp; j < K; j += ISO_WARPS) {
-    uint32_t v = sm.red[0][j][lane];
+    uint32_t v = sm.seed[j][lane];
 #pragma unroll
-    for (uint32_t q = 1; q < ISO_WARPS; ++q) v = __vminu2(v, sm.red[q][j][lane]);
+    for (uint32_t q = 0; q < ISO_WARPS; ++q) v = __vminu2(v, sm.red[q][j][lane]);
     sm.red[0][j][lane] = v;
   }
   __syncthreads();
@@ -403,7 +412,7 @@ __device__ __forceinline__ void iso_block_unit(const IsoArgs& g, const IsoPanel&
   if (warp == 0) {
 #pragma unroll
     for (uint32_t j = 0; j < K; ++j) acc[j] = sm.red[0][j][lane];
-    written = finish_unit<K, SAT>(g, p, t, sd, sm.tri, slab, lane, acc);
+    written = finish_unit<K, SAT>(g, p, t, 0, sm.tri, slab, lane, acc);  // (seeds are in)
   }
   iso_count(g, lane, gathered, written);
 }
@@ -540,7 +549,8 @@ bf_status iso_wave_panels(Graph* g, const uint32_t* d_orig, const uint32_t* d_th
                           cudaStream_t st, cudaEvent_t ev, uint64_t* launches) {
   const Panels& P = g->panels;
   const uint32_t n = g->n, tiles = (kw + 63) / 64;
-  const bool sat = tmax >= 0x7FFFu, pdl = g->tune.pdl != 0;
+  const bool sat = tmax >= 0x7FFFu;
+  bool pdl = false;  // (every level may read the seeds early, as in sweep_panels)
   uint32_t *act = words, *seeded = words + n, *thr = words + ((2 * (size_t)n + 3) & ~(size_t)3);
   BF_CUDA(cudaMemsetAsync(words, 0, 2 * (size_t)n * 4, st));
   k_iso_thr<<<(tiles * 32 + 127) / 128, 128, 0, st>>>(d_thr, kw, tiles * 64, thr);
@@ -571,6 +581,7 @@ bf_status iso_wave_panels(Graph* g, const uint32_t* d_orig, const uint32_t* d_th
       BF_CUDA(launch_level(sat ? k_iso_panels<true> : k_iso_panels<false>, dim3(big + small, y),
                            256, pdl, st, a, p0, pb, p1, big));
     }
+    pdl = g->tune.pdl != 0;
     ++*launches;
   }
   return BF_OK;

@@ -1008,7 +1008,12 @@ __device__ __forceinline__ void split_item(const uint4 a, const uint32_t* __rest
   const uint32_t* tri = pw + a.z + (size_t)nu * stride;
   for (uint32_t i = t; i < K * K; i += TPB)
     sm.tri[i] = tri[(i / K) * stride + i % K];
-  for (uint32_t i = t; i < K * LANES; i += TPB) sm.red[i] = FARV;
+  // (seeds too: they are written before the first level is launched)
+  for (uint32_t i = t; i < K * LANES; i += TPB) {
+    const uint32_t j = i / LANES, x = lane0 + i % LANES, r = a.x - j;
+    sm.red[i] = j < live && x < Kp && ((seeded[r >> 5] >> (r & 31)) & 1u)
+                    ? __ldcg(slab + (size_t)r * Kp + x) : FARV;
+  }
   __syncthreads();
   asm volatile("griddepcontrol.wait;" ::: "memory");
   uint32_t acc[K][LPT];
@@ -1024,7 +1029,7 @@ __device__ __forceinline__ void split_item(const uint4 a, const uint32_t* __rest
       __syncthreads();
     }
     if (on) {
-      constexpr uint32_t U = 4;  // source rows in flight per thread
+      constexpr uint32_t U = 16 / LPT;  // source rows in flight per thread
       for (uint32_t s0 = warp; s0 < m; s0 += U * SPLIT_WARPS) {
         uint32_t d[U][LPT];
 #pragma unroll
@@ -1060,12 +1065,7 @@ __device__ __forceinline__ void split_item(const uint4 a, const uint32_t* __rest
   if (t >= LANES || x >= Kp) return;
   uint32_t v[K][1];
 #pragma unroll
-  for (uint32_t j = 0; j < K; ++j) {
-    const uint32_t r = a.x - j;
-    v[j][0] = sm.red[j * LANES + t];
-    if (j < live && ((seeded[r >> 5] >> (r & 31)) & 1u))
-      v[j][0] = min(v[j][0], __ldcg(slab + (size_t)r * Kp + x));
-  }
+  for (uint32_t j = 0; j < K; ++j) v[j][0] = sm.red[j * LANES + t];
   solve_triangle<K, 1, SAT>(sm.tri, K, absent, v);
 #pragma unroll
   for (uint32_t j = 0; j < K; ++j)
@@ -1073,9 +1073,13 @@ __device__ __forceinline__ void split_item(const uint4 a, const uint32_t* __rest
 }
 
 // One level of panels: blockIdx.x = item, blockIdx.y = block of 32 * LPT lanes.
-// Bound by the chain of dependent levels. Against the item sweep (a level of
-// rows, a gather per edge), sweep time: 37 x 421 on the 1000 x 1250 region
-// 1.69 -> 0.40 ms, 100 x 100 on grid100 1.59 -> 0.30 ms.
+// Bound by the chain of dependent levels, 3 us each: what it must still do once
+// the level before it is done is one round of row loads, the combination and
+// the triangle; everything else, seeds too, is staged before. Against the item
+// sweep (a level of rows, a gather per edge), sweep time: 37 x 421 on the
+// 1000 x 1250 region 1.69 -> 0.16 ms, 100 x 100 on grid100 1.59 -> 0.14 ms; with
+// four rows in flight per thread, seeds read at the end and 128 lanes a block
+// for any level 0.25 and 0.28.
 template <uint32_t LPT, bool SAT>
 __global__ void __launch_bounds__(32 * SPLIT_WARPS)
     k_sweep_panels(const uint4* __restrict__ item, uint32_t i0, const uint32_t* __restrict__ prow,
@@ -1405,8 +1409,12 @@ cudaError_t launch_panels(const Graph* g, const Sched& sc, uint32_t i0, uint32_t
                         (const uint4*)sc.d_pitem, i0, (const uint32_t*)sc.d_prow,
                         (const uint32_t*)P.d_w, P.absent, slab, Kp, seeded);
   };
-  if (Kp <= 32) return go(k_sweep_panels<1, SAT>, 32);
-  if (Kp <= 64) return go(k_sweep_panels<2, SAT>, 64);
+  // lanes a block: as many as still give two blocks an SM (fewer lanes a thread
+  // keep more rows in flight), else 32. 100 lanes on grid100, whole call: 344 us
+  // against 420 with 128 lanes a block
+  const uint64_t few = 2ull * g->sm_count;
+  if (Kp <= 32 || m * (uint64_t)((Kp + 63) / 64) < few) return go(k_sweep_panels<1, SAT>, 32);
+  if (Kp <= 64 || m * (uint64_t)((Kp + 127) / 128) < few) return go(k_sweep_panels<2, SAT>, 64);
   return go(k_sweep_panels<4, SAT>, 128);
 }
 
@@ -1443,13 +1451,16 @@ uint32_t unreachable_from(const Graph* g, const Sched& sc, uint64_t max_seed) {
 // longest paths).
 cudaError_t sweep_panels(Graph* g, Sched& sc, uint32_t* slab, uint32_t Kp, bool sat,
                          cudaStream_t st, uint64_t* launches, const uint32_t* seeded) {
-  const bool pdl = g->tune.pdl != 0;
+  // the first level waits for what ran before it, so that every level may read
+  // the seeds while the level before it drains
+  bool pdl = false;
   for (uint32_t l = 0; l + 1 < sc.lvl_pan.size(); ++l) {
     const uint32_t i0 = sc.lvl_pan[l], m = sc.lvl_pan[l + 1] - i0;
     if (!m) continue;
     const cudaError_t e = sat ? launch_panels<true>(g, sc, i0, m, slab, Kp, seeded, pdl, st)
                               : launch_panels<false>(g, sc, i0, m, slab, Kp, seeded, pdl, st);
     if (e != cudaSuccess) return e;
+    pdl = g->tune.pdl != 0;
     ++*launches;
   }
   return cudaSuccess;

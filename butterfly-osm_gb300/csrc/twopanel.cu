@@ -16,6 +16,7 @@ namespace {
 constexpr unsigned FULL = 0xFFFFFFFFu;
 constexpr uint64_t LINF = ~0ull;
 constexpr uint32_t TP_WARPS = 8, TP_CH = 128;
+constexpr uint32_t TP_FLIGHT = 8;  // source rows in flight per thread of a shared panel
 
 __device__ __forceinline__ uint64_t lab_relax(uint64_t a, uint32_t wt, uint32_t wl, uint64_t acc) {
   const uint32_t t = sat_add((uint32_t)(a >> 32), wt), l = sat_add((uint32_t)a, wl);
@@ -35,18 +36,19 @@ __device__ __forceinline__ uint32_t time_of(uint32_t wt, uint32_t wl) {
   return wl == INF ? INF : wt;  // (absent edges may weigh less in the time tile)
 }
 
+// Row j's seed in lane x (LINF where it has none).
+__device__ __forceinline__ uint64_t seed_of(const TwoArgs& g, uint4 it, uint32_t j, uint32_t x) {
+  const uint32_t r = it.x - j;
+  if (j >= (it.y & 31u) || !((g.seeded[r >> 5] >> (r & 31)) & 1u)) return LINF;
+  return __ldcg((const unsigned long long*)g.slab + (size_t)r * g.Kp2 + x);
+}
+
 // Rows i < j of the panel into row j, then all live rows of one lane.
 template <uint32_t K>
 __device__ __forceinline__ void finish_rows(const TwoArgs& g, uint4 it, uint32_t x,
                                             const uint32_t* tt, const uint32_t* tl,
                                             uint64_t (&v)[K]) {
   const uint32_t live = it.y & 31u, stride = (it.y >> 5) & 31u;
-#pragma unroll
-  for (uint32_t j = 0; j < K; ++j) {
-    const uint32_t r = it.x - j;
-    if (j < live && ((g.seeded[r >> 5] >> (r & 31)) & 1u))
-      v[j] = min(v[j], (uint64_t)__ldcg((const unsigned long long*)g.slab + (size_t)r * g.Kp2 + x));
-  }
 #pragma unroll
   for (uint32_t i = 0; i + 1 < K; ++i)
 #pragma unroll
@@ -65,6 +67,7 @@ struct TwoSmem {
   uint32_t wt[TP_CH * PANEL_ROWS], wl[TP_CH * PANEL_ROWS];
   uint32_t tt[PANEL_ROWS * PANEL_ROWS], tl[PANEL_ROWS * PANEL_ROWS];
   uint32_t row[TP_CH];
+  uint64_t seed[PANEL_ROWS][32];
 };
 
 template <uint32_t K>
@@ -89,6 +92,8 @@ __device__ __forceinline__ void block_item(const TwoArgs& g, uint4 it, TwoSmem& 
     sm.tl[i] = g.wl[it.z + (size_t)nu * stride + i];
     sm.tt[i] = g.wt[it.z + (size_t)nu * stride + i];
   }
+  // (seeds are written before the first level is launched)
+  for (uint32_t j = warp; j < K; j += TP_WARPS) sm.seed[j][lane] = on ? seed_of(g, it, j, x) : LINF;
   __syncthreads();
   asm volatile("griddepcontrol.wait;" ::: "memory");
   uint64_t acc[K];
@@ -102,27 +107,31 @@ __device__ __forceinline__ void block_item(const TwoArgs& g, uint4 it, TwoSmem& 
       __syncthreads();
     }
     if (on)
-      for (uint32_t s0 = warp; s0 < m; s0 += 2 * TP_WARPS) {
-        const uint32_t s1 = s0 + TP_WARPS;
+      for (uint32_t s0 = warp; s0 < m; s0 += TP_FLIGHT * TP_WARPS) {
         const unsigned long long* slab = (const unsigned long long*)g.slab + x;
-        const uint64_t d0 = __ldcg(slab + (size_t)sm.row[s0] * g.Kp2);
-        const uint64_t d1 = s1 < m ? __ldcg(slab + (size_t)sm.row[s1] * g.Kp2) : LINF;
+        uint64_t d[TP_FLIGHT];
 #pragma unroll
-        for (uint32_t j = 0; j < K; ++j)
-          acc[j] = lab_relax(d0, sm.wt[s0 * stride + j], sm.wl[s0 * stride + j], acc[j]);
-        if (s1 < m)
+        for (uint32_t q = 0; q < TP_FLIGHT; ++q) {
+          const uint32_t s = s0 + q * TP_WARPS;
+          d[q] = s < m ? __ldcg(slab + (size_t)sm.row[s] * g.Kp2) : LINF;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < TP_FLIGHT; ++q) {
+          const uint32_t s = s0 + q * TP_WARPS;
+          if (s >= m) break;
 #pragma unroll
           for (uint32_t j = 0; j < K; ++j)
-            acc[j] = lab_relax(d1, sm.wt[s1 * stride + j], sm.wl[s1 * stride + j], acc[j]);
+            acc[j] = lab_relax(d[q], sm.wt[s * stride + j], sm.wl[s * stride + j], acc[j]);
+        }
       }
   }
 #pragma unroll
   for (uint32_t j = 0; j < K; ++j) red[warp][j][lane] = acc[j];
   __syncthreads();
   for (uint32_t j = warp; j < K; j += TP_WARPS) {
-    uint64_t v = red[0][j][lane];
+    uint64_t v = sm.seed[j][lane];
 #pragma unroll
-    for (uint32_t q = 1; q < TP_WARPS; ++q) v = min(v, red[q][j][lane]);
+    for (uint32_t q = 0; q < TP_WARPS; ++q) v = min(v, red[q][j][lane]);
     red[0][j][lane] = v;
   }
   __syncthreads();
@@ -134,7 +143,8 @@ __device__ __forceinline__ void block_item(const TwoArgs& g, uint4 it, TwoSmem& 
 
 // Bound by the chain of levels, and with u64 labels by a level's arithmetic (ten
 // instructions a weight). 60 x 90 ends of one to three seeds on the 1000 x 1250
-// region, whole call: 4.85 ms with a launch per level of rows, 1.06 ms by panels.
+// region, whole call: 4.85 ms with a launch per level of rows, 0.98 ms by panels
+// (1.08 with two rows in flight and the seeds read at the end).
 __global__ void __launch_bounds__(32 * TP_WARPS) k_two_split(const TwoArgs g, uint32_t i0) {
   extern __shared__ __align__(16) unsigned char two_smem[];
   TwoSmem& sm = *reinterpret_cast<TwoSmem*>(two_smem);
@@ -169,6 +179,8 @@ __device__ __forceinline__ void warp_item(const TwoArgs& g, uint4 it, uint32_t x
       acc[j] = lab_relax(d, time_of(wt[(size_t)s * stride + j], l), l, acc[j]);
     }
   }
+#pragma unroll
+  for (uint32_t j = 0; j < K; ++j) acc[j] = min(acc[j], seed_of(g, it, j, x));
   finish_rows<K>(g, it, x, wt + (size_t)nu * stride, wl + (size_t)nu * stride, acc);
 }
 
@@ -316,7 +328,7 @@ size_t upward_two_smem(const Graph* g) {
 cudaError_t sweep_panels_2ch(Graph* g, Sched& sc, uint64_t* slab, uint32_t Kp2, cudaStream_t st,
                              uint64_t* launches, const uint32_t* seeded) {
   const Panels& P = g->panels;
-  const bool pdl = g->tune.pdl != 0;
+  bool pdl = false;  // (every level may read the seeds early, as in sweep_panels)
   const TwoArgs a{sc.d_pitem, sc.d_prow, P.d_w, P.d_len, slab, Kp2, seeded};
   const uint32_t tiles = (Kp2 + 31) / 32;
   for (uint32_t l = 0; l + 1 < sc.lvl_pan.size(); ++l) {
@@ -332,6 +344,7 @@ cudaError_t sweep_panels_2ch(Graph* g, Sched& sc, uint64_t* slab, uint32_t Kp2, 
             : launch_level(k_two_warps, dim3((unsigned)((units + 7) / 8)), 256, pdl, st, a, i0, m,
                            tiles);
     if (e != cudaSuccess) return e;
+    pdl = g->tune.pdl != 0;
     ++*launches;
   }
   return cudaSuccess;
