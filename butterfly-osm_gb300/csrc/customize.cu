@@ -20,8 +20,10 @@
 // its lower neighbours computes it: nodes are grouped by elimination-tree
 // height (kept when heights strictly increase along every edge, which the
 // plan verifies; else longest-path levels), and a level pushes the
-// candidates of all its apexes. Middles, tie-breaks and saturating sums
-// therefore match the reference bit for bit, from any seeds.
+// candidates of all its apexes; near the top, where a level is a few apexes,
+// panels of up to 16 of them push together (cchpanel.cu). Middles, tie-breaks
+// and saturating sums therefore match the reference bit for bit, from any
+// seeds.
 //
 // State layout for the relaxation: every node j has a row R(j) of its upper
 // neighbours in either direction (ascending); the unordered pair {j, v},
@@ -43,7 +45,7 @@
 #include <string>
 #include <vector>
 
-#include "engine.cuh"
+#include "customize.cuh"
 
 using namespace bf;
 
@@ -53,13 +55,6 @@ constexpr int RT = 256;      // threads per relaxation block
 constexpr int RI = 2;        // pair candidates per thread
 constexpr int RC = RT * RI;  // pair candidates per block
 constexpr uint32_t DIR_DOWN = 0x80000000u;  // bottom-up list entry: a DOWN edge
-// Target of a pair candidate: the pair's slot index with the directions
-// present in the topology; neither bit set = nothing to relax.
-constexpr uint32_t T_UP = 1u << 31;
-constexpr uint32_t T_DOWN = 1u << 30;
-constexpr uint32_t T_PAIR = T_DOWN - 1;
-// per-pair flag byte
-constexpr uint8_t P_UP = 1, P_DOWN = 2, P_UP_SHORT = 4, P_DOWN_SHORT = 8;
 
 // Device view of a plan.
 struct PlanDev {
@@ -74,11 +69,6 @@ struct PlanDev {
   const uint32_t* apex;  // apexes (row of >= 2) in level order
   const uint64_t* cpre;  // pair-candidate prefix over `apex` [napex + 1]
 };
-
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 
 // Index of v in tgt[off[u], off[u + 1]) (ascending), or ~0 when absent
 // (find_edge_index, customization.rs:1507-1521).
@@ -96,18 +86,6 @@ __device__ __forceinline__ uint64_t find_edge(const uint64_t* __restrict__ off,
       hi = mid;
   }
   return (lo < end && __ldg(tgt + lo) == v) ? lo : ~0ull;
-}
-
-// Candidate value of a triangle from its two packed legs; false when a leg
-// has weight (time) u32::MAX, which the reference skips.
-template <bool LEX>
-__device__ __forceinline__ bool candidate(uint64_t leg1, uint64_t leg2, uint32_t m,
-                                          uint64_t* out) {
-  const uint32_t a = (uint32_t)(leg1 >> 32), b = (uint32_t)(leg2 >> 32);
-  if (a == INF || b == INF) return false;
-  const uint32_t lo = LEX ? sat_add((uint32_t)leg1, (uint32_t)leg2) : m;
-  *out = ((uint64_t)sat_add(a, b) << 32) | lo;
-  return true;
 }
 
 // One block of RC consecutive pair candidates of a level, computed when the
@@ -424,6 +402,7 @@ struct bf_cch {
   uint64_t* d_cpre = nullptr;
   Blk* d_blk = nullptr;                             // relaxation blocks, level after level
   uint32_t* d_tidx = nullptr;                       // target per pair candidate (or null)
+  CchPanels panels;                                 // the upper levels by panels
   std::vector<uint64_t> lv_blk;                     // [levels + 1] first block per level
   uint32_t napex = 0;
   uint64_t ncand = 0;                               // pair candidates
@@ -458,6 +437,7 @@ void free_plan(bf_cch* c) {
                   c->d_w[1], c->d_w[2], c->d_w[3], c->d_l[0], c->d_l[1], c->d_err};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  free_cch_panels(c->panels);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   if (c->s) cudaStreamDestroy(c->s);
@@ -669,6 +649,10 @@ bf_status build_plan(bf_cch* c, const bf_cch_topo* t) {
     k_tidx<<<(unsigned)blks.size(), RT, 0, c->s>>>(c->dev(), c->d_blk, c->d_tidx);
     BF_CUDA(cudaGetLastError());
     BF_CUDA(cudaStreamSynchronize(c->s));
+    // the panels' index likewise
+    BF_CUDA(cudaMemGetInfo(&fr, &tot));
+    return build_cch_panels(c->panels, n, qo, qt, pf, lev, L, c->d_qo, c->d_qt, c->d_pf, fr / 4,
+                            c->s);
   }
   return BF_OK;
 }
@@ -684,7 +668,8 @@ bf_status run_relax(bf_cch* c, bool lex) {
     const PlanDev p = c->dev();
     const Blk* blk = c->d_blk;
     const uint32_t* ti = c->d_tidx;
-    for (size_t l = 0; l + 1 < c->lv_blk.size() && err == cudaSuccess; ++l) {
+    for (size_t l = 0; l + 1 < c->lv_blk.size() && l < c->panels.first_level && err == cudaSuccess;
+         ++l) {
       const uint64_t b0 = c->lv_blk[l], b1 = c->lv_blk[l + 1];
       if (b1 == b0) continue;
       const dim3 grid((unsigned)(b1 - b0));
@@ -700,6 +685,7 @@ bf_status run_relax(bf_cch* c, bool lex) {
                                  c->d_sl);
       first = false;
     }
+    if (err == cudaSuccess) err = relax_cch_panels(c->panels, lex, !first, c->d_sl, c->s);
     cudaError_t e2 = cudaStreamEndCapture(c->s, &g);
     if (err == cudaSuccess) err = e2;
     if (err == cudaSuccess) err = cudaGraphInstantiate(&ge, g, 0);
