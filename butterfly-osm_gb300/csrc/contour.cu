@@ -33,6 +33,7 @@ namespace {
 
 struct IsoDev {
   double ox, oy, cell;
+  double inv;  // 1 / cell for cell_index, NaN where that is no normal number
   int32_t col0, row0;
   uint32_t wpr, height;  // words per row, rows
   uint64_t woff;         // first word
@@ -44,20 +45,51 @@ __device__ __forceinline__ void cell_of(const IsoDev& g, double x, double y, int
   *r = (int32_t)floor(__ddiv_rn(__dsub_rn(y, g.oy), g.cell));
 }
 
-__device__ __forceinline__ void set_cell(const IsoDev& g, int32_t c, int32_t r,
-                                         unsigned long long* words, uint32_t* err) {
+// floor(rn(rn(v - o) / cell)), cell_of's index of one coordinate, without the
+// division for nearly every point: doubles run at a sixty-fourth of the integer
+// rate here, a division some ten of them. One multiply-add onto 1.5 * 2^32
+// leaves q = (v - o) / cell in the sum's bits in units of 2^-20, off by less
+// than one (half for the sum's rounding, under a quarter for the rounding of
+// 1 / cell at |q| < 2^31). Where that lies at least four units from an integer,
+// q itself and the rounded quotient have the floor it shows; else, and where the
+// sum left [2^32, 2^33), the division decides.
+__device__ __forceinline__ int32_t cell_index(double v, double o, double cell, double inv) {
+  const double t = __dsub_rn(v, o);
+  const uint64_t b = (uint64_t)__double_as_longlong(__fma_rn(t, inv, 6442450944.0));
+  const uint32_t frac = (uint32_t)b & 0xFFFFFu;
+  if ((b >> 52) == 0x41Fu && frac - 4u <= 0xFFFFFu - 8u)
+    return (int32_t)((uint32_t)(b >> 20) ^ 0x80000000u);
+  return (int32_t)floor(__ddiv_rn(t, cell));
+}
+
+// Word and bit of a cell; false (an error: a bug, never a write) outside the
+// raster the layout computed.
+__device__ __forceinline__ bool cell_word(const IsoDev& g, int32_t c, int32_t r, uint64_t* word,
+                                          unsigned long long* bit, uint32_t* err) {
   const int64_t lc = (int64_t)c - g.col0, lr = (int64_t)r - g.row0;
   if (lc < 0 || lr < 0 || lc >= (int64_t)g.wpr * 64 || lr >= (int64_t)g.height) {
-    atomicOr(err, 1u);  // outside the raster the layout computed: a bug, never a write
-    return;
+    atomicOr(err, 1u);
+    return false;
   }
-  atomicOr(words + g.woff + (uint64_t)lr * g.wpr + (uint64_t)(lc >> 6), 1ull << (lc & 63));
+  *word = g.woff + (uint64_t)lr * g.wpr + (uint64_t)(lc >> 6);
+  *bit = 1ull << (lc & 63);
+  return true;
+}
+
+__device__ __forceinline__ void set_cell(const IsoDev& g, int32_t c, int32_t r,
+                                         unsigned long long* words, uint32_t* err) {
+  uint64_t w;
+  unsigned long long bit;
+  if (cell_word(g, c, r, &w, &bit, err)) atomicOr(words + w, bit);
 }
 
 // stamp_line (sparse_contour.rs:112-144) over every consecutive point pair
 // of a segment, and every point of it: one thread per segment, each point's
-// cell computed once (two IEEE double divisions), the line drawn from the
-// previous point's cell. Point ranges are clamped to the points given.
+// cell computed once, the line drawn from the previous point's cell, which is
+// set already. Cells that follow each other in one word are set together. Point
+// ranges are clamped to the points given. 5.5 M segments of two points:
+// 127 us against 443 with two divisions a point and four atomics a segment; the
+// points are 26 us of HBM.
 __global__ void k_stamp(uint64_t n_seg, uint64_t n_pts, const double2* __restrict__ xy,
                         const uint64_t* __restrict__ seg_pt, const uint32_t* __restrict__ seg_iso,
                         const IsoDev* __restrict__ iso, unsigned long long* __restrict__ words,
@@ -66,34 +98,52 @@ __global__ void k_stamp(uint64_t n_seg, uint64_t n_pts, const double2* __restric
        s += (uint64_t)gridDim.x * blockDim.x) {
     const IsoDev g = iso[seg_iso[s]];
     const uint64_t p1 = min(seg_pt[s + 1], n_pts), p0 = min(seg_pt[s], p1);
-    int32_t pc = 0, pr = 0;
-    for (uint64_t p = p0; p < p1; ++p) {
-      int32_t c1, r1;
-      const double2 q = xy[p];
-      cell_of(g, q.x, q.y, &c1, &r1);
-      set_cell(g, c1, r1, words, err);
-      if (p > p0) {
-        const int32_t c0 = pc, r0 = pr;
-        const int32_t dx = abs(c1 - c0), dy = abs(r1 - r0);
-        const int32_t sx = c0 < c1 ? 1 : -1, sy = r0 < r1 ? 1 : -1;
-        int32_t e = dx - dy, c = c0, r = r0;
-        for (int64_t guard = 0; guard <= (int64_t)dx + dy; ++guard) {  // dx + dy + 1 cells at most
-          set_cell(g, c, r, words, err);
-          if (c == c1 && r == r1) break;
-          const int32_t e2 = 2 * e;
-          if (e2 > -dy) {
-            e -= dy;
-            c += sx;
-          }
-          if (e2 < dx) {
-            e += dx;
-            r += sy;
-          }
-        }
+    int32_t c = 0, r = 0;
+    uint64_t word = 0;
+    unsigned long long bits = 0;  // of `word`, not set yet
+    auto set = [&]() {
+      uint64_t w;
+      unsigned long long bit;
+      if (!cell_word(g, c, r, &w, &bit, err)) return;
+      if (bits && w != word) {
+        atomicOr(words + word, bits);
+        bits = 0;
       }
-      pc = c1;
-      pr = r1;
+      word = w;
+      bits |= bit;
+    };
+    for (uint64_t p = p0; p < p1; ++p) {
+      const double2 q = xy[p];
+      const int32_t c1 = cell_index(q.x, g.ox, g.cell, g.inv);
+      const int32_t r1 = cell_index(q.y, g.oy, g.cell, g.inv);
+      if (p == p0) {
+        c = c1;
+        r = r1;
+        set();
+        continue;
+      }
+      const int32_t dx = abs(c1 - c), dy = abs(r1 - r);
+      const int32_t sx = c < c1 ? 1 : -1, sy = r < r1 ? 1 : -1;
+      int32_t e = dx - dy;
+      for (int64_t guard = 0; guard < (int64_t)dx + dy && (c != c1 || r != r1); ++guard) {
+        const int32_t e2 = 2 * e;
+        if (e2 > -dy) {
+          e -= dy;
+          c += sx;
+        }
+        if (e2 < dx) {
+          e += dx;
+          r += sy;
+        }
+        set();
+      }
+      if (c != c1 || r != r1) {  // (a line ends at its point; set it in any case)
+        c = c1;
+        r = r1;
+        set();
+      }
     }
+    if (bits) atomicOr(words + word, bits);
   }
 }
 
@@ -165,13 +215,20 @@ struct Extent {
   uint32_t has_points, pad;
 };
 
-__device__ __forceinline__ double warp_min(double v) {
-  for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-  return v;
+// Doubles in the order of signed integers, compared at the integer rate (a
+// sixty-fourth of it is the doubles'). NaN counts for nothing, as in fmin.
+__device__ __forceinline__ int64_t ordered(double d) {
+  const int64_t b = __double_as_longlong(d);
+  return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFll);
 }
-__device__ __forceinline__ double warp_max(double v) {
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-  return v;
+__device__ __forceinline__ double from_ordered(int64_t k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7FFFFFFFFFFFFFFFll));
+}
+__device__ __forceinline__ void widen(double d, int64_t* lo, int64_t* hi) {
+  if ((uint64_t)(__double_as_longlong(d) & 0x7FFFFFFFFFFFFFFFll) > 0x7FF0000000000000ull) return;
+  const int64_t k = ordered(d);
+  *lo = min(*lo, k);
+  *hi = max(*hi, k);
 }
 
 __global__ void __launch_bounds__(256) k_minmax(uint64_t n_pts, const double2* __restrict__ xy,
@@ -189,18 +246,21 @@ __global__ void __launch_bounds__(256) k_minmax(uint64_t n_pts, const double2* _
   }
   const uint64_t q1 = min(seg_pt[s1], n_pts), q0 = min(seg_pt[s0], q1);
   const uint64_t pa = q0 + (q1 - q0) * ch / EXT_CHUNKS, pb = q0 + (q1 - q0) * (ch + 1) / EXT_CHUNKS;
-  double mnx = INFINITY, mny = INFINITY, mxx = -INFINITY, mxy = -INFINITY;
+  int64_t x0 = ordered(INFINITY), y0 = x0, x1 = ordered(-INFINITY), y1 = x1;
+#pragma unroll 4
   for (uint64_t p = pa + threadIdx.x; p < pb; p += blockDim.x) {
     const double2 q = xy[p];
-    mnx = fmin(mnx, q.x);
-    mny = fmin(mny, q.y);
-    mxx = fmax(mxx, q.x);
-    mxy = fmax(mxy, q.y);
+    widen(q.x, &x0, &x1);
+    widen(q.y, &y0, &y1);
   }
-  mnx = warp_min(mnx);
-  mny = warp_min(mny);
-  mxx = warp_max(mxx);
-  mxy = warp_max(mxy);
+  for (int o = 16; o > 0; o >>= 1) {
+    x0 = min(x0, (int64_t)__shfl_xor_sync(0xFFFFFFFFu, (long long)x0, o));
+    y0 = min(y0, (int64_t)__shfl_xor_sync(0xFFFFFFFFu, (long long)y0, o));
+    x1 = max(x1, (int64_t)__shfl_xor_sync(0xFFFFFFFFu, (long long)x1, o));
+    y1 = max(y1, (int64_t)__shfl_xor_sync(0xFFFFFFFFu, (long long)y1, o));
+  }
+  const double mnx = from_ordered(x0), mny = from_ordered(y0);
+  const double mxx = from_ordered(x1), mxy = from_ordered(y1);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = MinMax{mnx, mny, mxx, mxy};
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -374,6 +434,7 @@ bool place(uint32_t n_iso, const Extent* ext, const double* cell_m, uint32_t dil
     g.ox = ext[k].ox;
     g.oy = ext[k].oy;
     g.cell = cell_m[k];
+    g.inv = std::isnormal(1.0 / g.cell) ? 1.0 / g.cell : NAN;
     g.col0 = (int32_t)c0;
     g.row0 = (int32_t)r0;
     g.wpr = (uint32_t)((c1 - c0 + 1 + 63) / 64);
