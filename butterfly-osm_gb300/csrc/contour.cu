@@ -1093,8 +1093,11 @@ bf_status bf_mercator(uint64_t n, const int32_t* lat_lon_e7, double* xy) {
     set_error("bf_mercator: null argument");
     return BF_ERR_INVALID;
   }
-  parallel_for((n + 65535) / 65536, [&](uint64_t b) {
-    for (uint64_t i = b * 65536; i < std::min<uint64_t>(n, (b + 1) * 65536); ++i)
+  // pieces worth the starting of a thread: 63,000 points take 1.1 ms on one
+  // thread, 0.35 in pieces of 8192, 0.9 in pieces of 2048
+  constexpr uint64_t PIECE = 8192;
+  parallel_for((n + PIECE - 1) / PIECE, [&](uint64_t b) {
+    for (uint64_t i = b * PIECE; i < std::min<uint64_t>(n, (b + 1) * PIECE); ++i)
       mercator_e7(lat_lon_e7[2 * i], lat_lon_e7[2 * i + 1], xy + 2 * i, xy + 2 * i + 1);
   });
   return BF_OK;

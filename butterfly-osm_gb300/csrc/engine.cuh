@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <exception>
 #include <functional>
 #include <mutex>
 #include <thread>
@@ -423,7 +424,11 @@ inline void parallel_for(uint64_t n, F&& f) {
     for (uint64_t i; (i = next.fetch_add(1)) < n;) f(i);
   };
   std::vector<std::thread> pool;
-  for (unsigned t = 1; t < nt; ++t) pool.emplace_back(work);
+  try {
+    pool.reserve(nt);
+    for (unsigned t = 1; t < nt; ++t) pool.emplace_back(work);
+  } catch (const std::exception&) {  // fewer threads, then
+  }
   work();
   for (auto& th : pool) th.join();
 }

@@ -42,7 +42,9 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <mutex>
+#include <thread>
 
 #include "engine.cuh"
 #include "scan.cuh"
@@ -720,19 +722,48 @@ bf_status trace_rings_device(const uint64_t* d_words, const bf_raster* ras, uint
     TW += (uint64_t)R.width_words * R.height;
   }
   std::vector<double> lon(std::max<uint64_t>(nlon, 1)), lat(std::max<uint64_t>(nlat, 1));
-  parallel_for(n_iso, [&](uint64_t k) {
-    const bf_raster& R = ras[k];
-    const double cell = cell_m[k];
-    for (uint64_t c = 0; c < (uint64_t)R.width_words * 64; ++c) {
-      const double x = R.origin_x + ((double)(R.col0 + (int64_t)c) + 0.5) * cell;
-      lon[iso[k].lon_off + c] = (x / EARTH_R_T) * (180.0 / PI_T);
+  // filled beside the device's tracing, which needs neither; a piece is worth the
+  // starting of a thread (10 ns an entry against some 50 us)
+  constexpr uint64_t PIECE = 16384;
+  auto tables = [&]() {
+    const uint64_t pc = (nlon + 8 * PIECE - 1) / (8 * PIECE), pr = (nlat + PIECE - 1) / PIECE;
+    parallel_for(pc + pr, [&](uint64_t i) {
+      const bool rows = i >= pc;
+      const uint64_t first = rows ? (i - pc) * PIECE : i * 8 * PIECE;
+      const uint64_t last = rows ? std::min(nlat, first + PIECE) : std::min(nlon, first + 8 * PIECE);
+      auto off = [&](const TIso& t) { return rows ? t.lat_off : t.lon_off; };
+      // the raster that holds entry `first`, then on
+      uint32_t k = (uint32_t)(std::upper_bound(iso.begin(), iso.end(), first,
+                                               [&](uint64_t v, const TIso& t) { return v < off(t); }) -
+                              iso.begin()) - 1;
+      for (uint64_t at = first; at < last; ++k) {
+        const bf_raster& R = ras[k];
+        const double cell = cell_m[k];
+        const uint64_t end = std::min(last, k + 1 < n_iso ? off(iso[k + 1]) : last);
+        for (; !rows && at < end; ++at) {
+          const int64_t c = (int64_t)(at - iso[k].lon_off);
+          const double x = R.origin_x + ((double)(R.col0 + c) + 0.5) * cell;
+          lon[at] = (x / EARTH_R_T) * (180.0 / PI_T);
+        }
+        for (; rows && at < end; ++at) {
+          const int64_t r = (int64_t)(at - iso[k].lat_off);
+          const double y = R.origin_y + ((double)(R.row0 + r) + 0.5) * cell;
+          lat[at] = (2.0 * std::atan(std::exp(y / EARTH_R_T)) - PI_T / 2.0) * (180.0 / PI_T);
+        }
+      }
+    });
+  };
+  struct Side {  // (joined on every way out, before the tables go)
+    std::thread t;
+    ~Side() {
+      if (t.joinable()) t.join();
     }
-    for (uint64_t r = 0; r < R.height; ++r) {
-      const double y = R.origin_y + ((double)(R.row0 + (int64_t)r) + 0.5) * cell;
-      lat[iso[k].lat_off + r] =
-          (2.0 * std::atan(std::exp(y / EARTH_R_T)) - PI_T / 2.0) * (180.0 / PI_T);
-    }
-  });
+  } side;
+  try {
+    side.t = std::thread(tables);
+  } catch (const std::exception&) {
+    tables();
+  }
   std::vector<double> tol(n_iso);
   for (uint32_t k = 0; k < n_iso; ++k) tol[k] = simplify_m[k] / 111000.0;
   if (!w.h_small) BF_CUDA(cudaHostAlloc((void**)&w.h_small, 64, cudaHostAllocDefault));
@@ -749,8 +780,6 @@ bf_status trace_rings_device(const uint64_t* d_words, const bf_raster* ras, uint
   get(T_LAT, lat.size(), &d_lat);
   if (e != cudaSuccess) return cuda_status(e, "contour tracing: device memory");
   BF_CUDA(cudaMemcpyAsync(d_iso, iso.data(), n_iso * sizeof(TIso), cudaMemcpyHostToDevice, st));
-  BF_CUDA(cudaMemcpyAsync(d_lon, lon.data(), lon.size() * 8, cudaMemcpyHostToDevice, st));
-  BF_CUDA(cudaMemcpyAsync(d_lat, lat.data(), lat.size() * 8, cudaMemcpyHostToDevice, st));
   BF_CUDA(cudaMemsetAsync(d_err, 0, 8, st));
   {  // the rasters, packed in raster order
     uint64_t *d_pack, *d_src;
@@ -921,6 +950,9 @@ bf_status trace_rings_device(const uint64_t* d_words, const bf_raster* ras, uint
   if (e != cudaSuccess) return cuda_status(e, "contour tracing: device memory");
   BF_CUDA(cudaMemcpyAsync(d_poff, poff.data(), poff.size() * 8, cudaMemcpyHostToDevice, st));
   BF_CUDA(cudaMemcpyAsync(d_tol, tol.data(), n_iso * 8, cudaMemcpyHostToDevice, st));
+  if (side.t.joinable()) side.t.join();
+  BF_CUDA(cudaMemcpyAsync(d_lon, lon.data(), lon.size() * 8, cudaMemcpyHostToDevice, st));
+  BF_CUDA(cudaMemcpyAsync(d_lat, lat.data(), lat.size() * 8, cudaMemcpyHostToDevice, st));
   k_tr_project<<<std::min<uint32_t>(n_iso, 152 * 8), TPB, 0, st>>>(
       n_iso, d_best, d_voff, d_verts, d_poff, d_iso, d_lon, d_lat, d_pts, d_pring);
   // Douglas-Peucker: levels until one splits nothing (every open range then
