@@ -157,7 +157,8 @@ struct Panels {
   uint2* d_b = nullptr;             // {first source, first weight}
   uint32_t* d_of = nullptr;         // [n] rank -> panel
   uint32_t* d_hibits = nullptr;     // [n bits] highest ranks of panels
-  uint32_t* d_lvl = nullptr;        // device copy of lvl_first
+  uint32_t* d_lvl = nullptr;        // device copies of lvl_first and lvl_small
+  uint32_t* d_lvl_small = nullptr;
   uint32_t* d_src = nullptr;        // source ranks
   uint32_t* d_w = nullptr;          // tiles [source][row], each followed by its panel's
                                     // triangle [row][row]; `absent` where there is no edge
@@ -186,6 +187,7 @@ struct Sched {
   uint4* d_pitem = nullptr;
   uint32_t* d_prow = nullptr;       // slab rows of the items' sources
   size_t cap_pitem = 0, cap_prow = 0;
+  uint64_t n_prow = 0;              // sources of all items
   bool counted = false;             // n_live / n_edges hold the rows that reach a target
   uint32_t n_live = 0;
   bool valid = false;

@@ -1089,6 +1089,10 @@ bf_status batched_matrix(Graph* g, Ctx& c, const uint32_t* d_src, uint64_t S, co
     stats->swept_nodes = sc.n_live;
     stats->swept_edges = sc.n_edges;
     stats->lanes = Kp;
+    if (sc.panel)  // rows of sources read, rows written, items and source rows' numbers
+      stats->sweep_bytes += (S + wave - 1) / wave *
+                            (4ull * Kp * (sc.n_prow + sc.n_r) + 4 * sc.n_prow +
+                             16ull * sc.lvl_pan.back());
     stats->kernel_launches += launches;
     stats->upward_ms += t_up;
     stats->downward_ms += t_dn;

@@ -217,7 +217,7 @@ bf_status pack_weights(Panels& P, uint64_t m) {
 }  // namespace
 
 void free_panels(Panels& P) {
-  void* q[] = {P.d_a, P.d_b, P.d_of, P.d_hibits, P.d_lvl, P.d_src, P.d_w, P.d_em,
+  void* q[] = {P.d_a, P.d_b, P.d_of, P.d_hibits, P.d_lvl, P.d_lvl_small, P.d_src, P.d_w, P.d_em,
                P.d_tm, P.d_up, P.d_up_end, P.d_up_w, P.d_w16,
                P.d_w16s, P.d_len, P.d_up_len};
   for (void* x : q)
@@ -383,7 +383,8 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
   });
   if ((rc = upload(&P.d_a, a, P)) || (rc = upload(&P.d_b, b, P)) ||
       (rc = upload(&P.d_of, of, P)) || (rc = upload(&P.d_hibits, hib, P)) ||
-      (rc = upload(&P.d_lvl, P.lvl_first, P)) || (rc = upload(&P.d_src, s, P)) ||
+      (rc = upload(&P.d_lvl, P.lvl_first, P)) ||
+      (rc = upload(&P.d_lvl_small, P.lvl_small, P)) || (rc = upload(&P.d_src, s, P)) ||
       (rc = upload(&P.d_w, t, P)) || (rc = upload(&P.d_em, em, P)) ||
       (rc = upload(&P.d_tm, tm, P)) ||
       (rc = upload(&P.d_up, up_a, P)) || (rc = upload(&P.d_up_end, us, P)) ||
@@ -852,6 +853,7 @@ bf_status build_schedule_panels(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_t
   sc.lvl_pan.assign(lvl, lvl + L + 1);
   sc.panel = true;
   sc.n_r = n_r;
+  sc.n_prow = n_rows;
   sc.counted = false;
   sc.lvl_item.clear();  // per-level tables of the item form are made on demand
   sc.lvl_row.clear();

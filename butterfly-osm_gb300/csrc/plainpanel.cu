@@ -20,7 +20,7 @@ constexpr uint32_t PP_CH = 16;  // sources of a chunk: their rows are in flight 
 struct PlainArgs {
   const uint4* a;       // Panels::d_a, d_b, d_lvl
   const uint2* b;
-  const uint32_t* lvl;
+  const uint32_t *lvl, *lvl_small;
   uint32_t n_levels;
   const uint32_t *src, *w;
   uint32_t absent;
@@ -199,6 +199,79 @@ __device__ __forceinline__ void plain_panel(const PlainArgs& g, const uint4 a, c
   if (SHARED) __syncthreads();
 }
 
+// A panel of up to four rows by eight threads, four lanes each (m8: their bits
+// of the warp): four panels of a warp at a time, and rows, weights and seeds move
+// 16 bytes a load.
+__device__ __forceinline__ uint4 min_plus4(const uint4 d, uint32_t w, const uint4 acc) {
+  return make_uint4(min_plus(d.x, w, acc.x), min_plus(d.y, w, acc.y), min_plus(d.z, w, acc.z),
+                    min_plus(d.w, w, acc.w));
+}
+
+__device__ __forceinline__ void plain_small(const PlainArgs& g, uint32_t p, unsigned m8) {
+  constexpr uint32_t K = 4, U = 4;  // source rows in flight
+  const uint4 a = g.a[p];
+  const uint2 b = g.b[p];
+  const uint32_t rows = a.y & 0xFF, nu = a.z, l4 = (threadIdx.x & 7) * 4;
+  const uint32_t* tile = g.w + b.y;
+  const uint32_t w0 = (a.x + 1 - rows) >> 5, w1 = a.x >> 5;
+  const uint32_t f0 = __ldcg(g.flag + w0), f1 = w1 == w0 ? f0 : __ldcg(g.flag + w1);
+  __syncwarp(m8);  // (all have read the bits before one clears them)
+  uint4 acc[K];
+#pragma unroll
+  for (uint32_t j = 0; j < K; ++j) {
+    const uint32_t r = a.x - j;
+    acc[j] = make_uint4(INF, INF, INF, INF);
+    if (j < rows && (((r >> 5) == w0 ? f0 : f1) >> (r & 31)) & 1u) {
+      uint4* at = reinterpret_cast<uint4*>(g.seed + (size_t)r * PLAIN_K + l4);
+      acc[j] = *at;
+      *at = make_uint4(INF, INF, INF, INF);
+      if (l4 == 0) atomicAnd(g.flag + (r >> 5), ~(1u << (r & 31)));
+    }
+  }
+  auto weights = [&](uint32_t at) {
+    uint4 w = __ldg(reinterpret_cast<const uint4*>(tile + (size_t)at * K));
+    w.x = w.x == g.absent ? INF : w.x;
+    w.y = w.y == g.absent ? INF : w.y;
+    w.z = w.z == g.absent ? INF : w.z;
+    w.w = w.w == g.absent ? INF : w.w;
+    return w;
+  };
+  for (uint32_t s = 0; s < nu; s += U) {
+    uint4 d[U];
+#pragma unroll
+    for (uint32_t q = 0; q < U; ++q)
+      if (s + q < nu)
+        d[q] = __ldcg(reinterpret_cast<const uint4*>(
+            g.dist + (size_t)__ldg(g.src + b.x + s + q) * PLAIN_K + l4));
+#pragma unroll
+    for (uint32_t q = 0; q < U; ++q) {
+      if (s + q >= nu) break;
+      const uint4 w = weights(s + q);
+      acc[0] = min_plus4(d[q], w.x, acc[0]);
+      acc[1] = min_plus4(d[q], w.y, acc[1]);
+      acc[2] = min_plus4(d[q], w.z, acc[2]);
+      acc[3] = min_plus4(d[q], w.w, acc[3]);
+    }
+  }
+#pragma unroll
+  for (uint32_t i = 0; i + 1 < K; ++i) {
+    const uint4 w = weights(nu + i);
+    if (i < 1) acc[1] = min_plus4(acc[i], w.y, acc[1]);
+    if (i < 2) acc[2] = min_plus4(acc[i], w.z, acc[2]);
+    acc[3] = min_plus4(acc[i], w.w, acc[3]);
+  }
+#pragma unroll
+  for (uint32_t j = 0; j < K; ++j) {
+    if (j >= rows) break;
+    uint4 v = acc[j];
+    v.x = v.x > g.threshold ? INF : v.x;
+    v.y = v.y > g.threshold ? INF : v.y;
+    v.z = v.z > g.threshold ? INF : v.z;
+    v.w = v.w > g.threshold ? INF : v.w;
+    *reinterpret_cast<uint4*>(g.dist + (size_t)(a.x - j) * PLAIN_K + l4) = v;
+  }
+}
+
 #define BF_BY_STRIDE(a, CALL)      \
   switch (stride_of(a)) {          \
     case 4: CALL(4); break;        \
@@ -214,11 +287,12 @@ __device__ __forceinline__ void plain_panel(const PlainArgs& g, const uint4 a, c
 // better apart (twice or once: within 3 %). `withhold` (a test hook, NONE otherwise) names a block that leaves
 // before its first barrier arrival.
 //
-// Two blocks an SM: three and four spill. Eight sources to all of the town's
-// 119,260 nodes: sweep 615 -> 230 us, whole call 862 -> 341; one source on
-// grid100 2250 -> 530 us; 8 sources on the 1000 x 1250 region 8.0 -> 6.9 ms, of
-// which most is the copy back.
-__global__ void __launch_bounds__(32 * PP_WARPS, 2)
+// Eight sources to all of the town's 119,249 nodes: sweep 615 -> 230 us, whole
+// call 849 -> 348; one source on grid100 2250 -> 570 us; a batch's sweep on the
+// 1000 x 1250 region 2.99 -> 1.44 ms, on the country graph 6.73 -> 4.71 (9.1 with
+// a warp for panels of up to four rows too).
+template <int PER_SM>
+__global__ void __launch_bounds__(32 * PP_WARPS, PER_SM)
     k_plain_panels(const PlainArgs g, uint32_t* __restrict__ bar, long long timeout,
                    uint32_t withhold, uint32_t* __restrict__ err) {
   __shared__ __align__(16) PlainSmem sm;
@@ -247,7 +321,8 @@ __global__ void __launch_bounds__(32 * PP_WARPS, 2)
 #undef BF_SOLVE
       }
     } else {
-      for (uint32_t p = p0 + blockIdx.x * PP_WARPS + (threadIdx.x >> 5); p < p1;
+      const uint32_t ps = g.lvl_small[l];  // panels of up to four rows, last in a level
+      for (uint32_t p = p0 + blockIdx.x * PP_WARPS + (threadIdx.x >> 5); p < ps;
            p += gridDim.x * PP_WARPS) {
         const uint4 wa = g.a[p];
         const uint2 wb = g.b[p];
@@ -255,6 +330,9 @@ __global__ void __launch_bounds__(32 * PP_WARPS, 2)
         BF_BY_STRIDE(wa, BF_SOLVE)
 #undef BF_SOLVE
       }
+      for (uint32_t p = ps + (blockIdx.x * PP_WARPS * 32 + threadIdx.x) / 8; p < p1;
+           p += gridDim.x * PP_WARPS * 4)
+        plain_small(g, p, 0xFFu << (threadIdx.x & 24));
       __syncthreads();
     }
     if (l + 1 == g.n_levels) break;
@@ -275,13 +353,18 @@ bf_status plain_sweep_panels(Graph* g, uint32_t threshold, cudaStream_t st, uint
   bf_status s;
   if ((s = ensure_barrier(g))) return s;
   const Panels& P = g->panels;
-  const PlainArgs a{P.d_a,    P.d_b,     P.d_lvl,   P.n_levels, P.d_src, P.d_w,
+  const PlainArgs a{P.d_a,    P.d_b,     P.d_lvl,   P.d_lvl_small, P.n_levels, P.d_src, P.d_w,
                     P.absent, g->d_dist, g->d_seed, g->d_flag,  threshold};
   const bool hook = test_withhold_arrival();
-  const unsigned blocks =
-      persistent_blocks(g, (const void*)k_plain_panels, 32 * PP_WARPS, 2 * g->sm_count);
+  // a slab beyond L2: rows come from HBM, and more blocks hide that although
+  // their kernel spills (country graph 4.7 ms a batch against 5.45 with two an
+  // SM, the town 400 us a call against 361)
+  const bool wide = (uint64_t)g->n * PLAIN_K * 4 > (128ull << 20);
+  const auto kern = wide ? k_plain_panels<4> : k_plain_panels<2>;
+  const unsigned blocks = persistent_blocks(g, (const void*)kern, 32 * PP_WARPS,
+                                            (wide ? 4 : 2) * g->sm_count);
   BF_CUDA(cudaMemsetAsync(g->d_bar, 0, 8, st));
-  BF_CUDA(launch_persistent(k_plain_panels, blocks, 32 * PP_WARPS, st, a, g->d_bar,
+  BF_CUDA(launch_persistent(kern, blocks, 32 * PP_WARPS, st, a, g->d_bar,
                             hook ? 2000000ll : BARRIER_TIMEOUT_CYCLES, hook ? 1u : NONE,
                             g->d_err));
   ++*launches;

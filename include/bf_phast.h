@@ -153,7 +153,9 @@ typedef struct bf_stats {
   double schedule_ms;         /* host time building sweep schedules (0 on reuse)  */
   uint64_t sweep_bytes;       /* isochrone calls: algorithmic bytes of the gated
                                  sweeps (schedule records scanned, active source
-                                 rows gathered, rows written), summed over waves */
+                                 rows gathered, rows written), summed over waves;
+                                 matrix calls swept over panels: likewise, each
+                                 panel's source rows gathered once              */
   uint64_t active_rows;       /* isochrone calls: rows written by the sweeps (rows of
                                  64 lanes each where a wave runs over panels)     */
 } bf_stats;
@@ -166,9 +168,11 @@ bf_status bf_graph_set_engine(bf_graph* g, uint32_t engine, uint32_t k_lanes);
 
 /* Tunables of the batched engine's sweep. */
 typedef struct bf_tune {
-  uint32_t threads_per_block;  /* sweep block size (each thread owns 4 lanes)    */
+  uint32_t threads_per_block;  /* sweep block size (each thread owns 4 lanes);
+                                  sweeps over panels have their own             */
   uint32_t edges_per_item;     /* max in-edges per work item (larger in-degrees
-                                  are split into slices combined by atomicMin)   */
+                                  are split into slices combined by atomicMin);
+                                  sweeps of single rows only                    */
   uint32_t graph_capture;      /* replay the level schedule from a CUDA graph   */
   uint32_t lanes_per_wave;     /* 0 = as many lanes as the HBM budget allows     */
   double step_ms;              /* device time of the sample under this choice    */
@@ -190,9 +194,11 @@ typedef struct bf_tune {
   uint32_t mapped_output;      /* 1: bf_matrix into page-locked host memory is
                                   written by the extraction kernel directly     */
   uint32_t hub_l2_mb;          /* L2 megabytes kept for the most-gathered rows
-                                  (evict-last cache hints; 0 = no hints)         */
+                                  (evict-last cache hints; 0 = no hints); sweeps
+                                  of single rows only                            */
   uint32_t device_schedule;    /* 1: target-restricted schedules are built on
-                                  the device; 0: by host threads (same rows)    */
+                                  the device, over panels; 0: by host threads,
+                                  over single rows (the same rows counted)      */
   uint32_t persistent_sweep;   /* bit 0 (default): the plain engine's sweep of a
                                   K = 32 batch, bit 1: each 16-bit isochrone
                                   wave's sweep, runs as one cooperative launch

@@ -272,3 +272,29 @@ def test_plain_sweep_by_panels(built, name):
             for thr in (0, lo, min(INF - 1, 5 * (hi // 2))):
                 got = g.matrix(src, tgt, threshold=thr)
                 assert np.array_equal(got, np.where(want[:, tgt] <= thr, want[:, tgt], INF)), thr
+
+
+def test_plain_sweep_of_a_slab_beyond_l2(built):
+    """A graph whose plain slab exceeds L2 (the sweep's other launch shape):
+    55,000 runs of 20 ranks, each rank joined to the next three of its run."""
+    import bfphast
+    n, run = 1_100_000, 20
+    u = np.arange(n, dtype=np.int64)
+    pairs = [np.stack([v := u[(u % run) < run - k], v + k], 1) for k in (1, 2, 3)]
+    up = np.concatenate(pairs)
+    up = up[np.lexsort((up[:, 1], up[:, 0]))]
+    rng = np.random.default_rng(2)
+    w = rng.integers(1, 100, (2, len(up))).astype(np.uint32)
+    o = np.lexsort((up[:, 0], up[:, 1]))
+    off = np.zeros((2, n + 1), np.uint64)
+    off[0, 1:] = np.cumsum(np.bincount(up[:, 0], minlength=n))
+    off[1, 1:] = np.cumsum(np.bincount(up[:, 1], minlength=n))
+    cch = dict(n=n, up_off=off[0], up_tgt=up[:, 1].astype(np.uint32), up_w=w[0],
+               down_off=off[1], down_tgt=up[o, 0].astype(np.uint32), down_w=w[1][o])
+    g = bfphast.Graph.from_cch(cch)
+    g.set_engine(bfphast.ENGINE_PLAIN)
+    src = rng.integers(0, n, 33).astype(np.uint32)
+    got = g.query_batch(src)
+    g.set_tune(persistent_sweep=0)
+    assert np.array_equal(got, g.query_batch(src))
+    assert ((got != INF).sum(1) == run).all() and (got[np.arange(33), src] == 0).all()
