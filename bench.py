@@ -250,7 +250,11 @@ def run_ours(args, rank, world, dist):
     # roofline of the dominant kernel (the restricted downward sweep)
     st = stats[-1]
     K, M, N = st["lanes"], st["swept_edges"], st["swept_nodes"]
-    alg_bytes = 8 * M + 4 * (N + 1) + 4 * K * M + 4 * K * N
+    # a sweep over panels reads a source row once for up to 16 rows (the library
+    # counts those); one over single rows once per edge
+    row_bytes = 8 * M + 4 * (N + 1) + 4 * K * M + 4 * K * N
+    panels = st["sweep_bytes"] > 0
+    alg_bytes = int(st["sweep_bytes"]) // max(1, int(st["waves"])) if panels else row_bytes
     sweep_s = st["downward_ms"] / 1e3
     peak, peak_kind = measured_peak()
     achieved = alg_bytes / sweep_s / 1e9
@@ -258,7 +262,7 @@ def run_ours(args, rank, world, dist):
     # large levels at 2000 lanes, scaled by this sweep's algorithmic bytes
     traffic = ratio = None
     prof = ROOT / "profiles" / "sweep_items_country2000.json"
-    if prof.exists():
+    if prof.exists() and not panels:
         ratio = json.loads(prof.read_text()).get("traffic_per_alg_byte")
         if ratio:
             traffic = int(round(ratio * alg_bytes))
@@ -266,8 +270,8 @@ def run_ours(args, rank, world, dist):
             "frac": round(achieved / peak, 4), "traffic": traffic,
             "traffic_source": ("scaled: %s DRAM bytes per algorithmic byte, 3 launches at "
                                "2000 lanes" % ratio) if traffic else None,
-            "peak_kind": peak_kind, "kernel": "k_sweep_items",
-            "alg_bytes_per_sweep": alg_bytes, "sweep_ms": round(st["downward_ms"], 3),
+            "peak_kind": peak_kind, "kernel": "k_sweep_panels_ring" if panels else "k_sweep_items",
+            "alg_bytes_per_sweep": alg_bytes, "row_gather_bytes_per_sweep": row_bytes, "sweep_ms": round(st["downward_ms"], 3),
             "swept_nodes": N, "swept_edges": M, "lanes": K}
 
     if args.level_table:
