@@ -337,6 +337,7 @@ bf_status build_cch_panels(CchPanels& P, uint32_t n, const std::vector<uint64_t>
   BF_CUDA(put(&P.d_ent, ent));
   BF_CUDA(put(&P.d_solve, solve));
   BF_CUDA(put(&P.d_push, push));
+  BF_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // (the uploads, before `s`)
   BF_CUDA(cudaMalloc(&P.d_tgt, std::max<size_t>(push.size(), 1) * CP_TILE * CP_TILE * 4));
   if (!push.empty())
     k_cp_targets<<<(unsigned)push.size(), CP_TILE * CP_TILE, 0, s>>>(P.d_pan, P.d_col, P.d_push,

@@ -641,6 +641,8 @@ bf_status build_plan(bf_cch* c, const bf_cch_topo* t) {
   for (int i = 0; i < 4; ++i) BF_CUDA(cudaMalloc(&c->d_w[i], nmax * 4));
   for (int i = 0; i < 2; ++i) BF_CUDA(cudaMalloc(&c->d_l[i], nmax * 4));
   BF_CUDA(cudaMalloc(&c->d_err, 4));
+  // the uploads, before work on the plan's own stream
+  BF_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
   // target index: 4 bytes per pair candidate while that fits a quarter of free HBM
   size_t fr = 0, tot = 0;
   BF_CUDA(cudaMemGetInfo(&fr, &tot));

@@ -416,7 +416,9 @@ bf_status check_device_error(Graph* g, cudaStream_t st) {
 
 bool test_withhold_arrival() { return std::getenv("BF_TEST_WITHHOLD_ARRIVAL") != nullptr; }
 
-static bf_status plain_buffers(Graph* g) {
+// The seed rows and bits start clear on `st`, before the call's own work there (a
+// memset on the default stream would run beside a stream that does not wait for it).
+static bf_status plain_buffers(Graph* g, cudaStream_t st) {
   if (g->d_dist) return BF_OK;
   const size_t slab = (size_t)g->n * PLAIN_K * sizeof(uint32_t);
   if (cudaMalloc(&g->d_dist, slab) != cudaSuccess || cudaMalloc(&g->d_seed, slab) != cudaSuccess ||
@@ -426,8 +428,8 @@ static bf_status plain_buffers(Graph* g) {
     return BF_ERR_OOM;
   }
   g->device_bytes += 2 * slab + ((g->n + 31) / 32) * 4;
-  BF_CUDA(cudaMemset(g->d_seed, 0xFF, slab));
-  BF_CUDA(cudaMemset(g->d_flag, 0, ((g->n + 31) / 32) * 4));
+  BF_CUDA(cudaMemsetAsync(g->d_seed, 0xFF, slab, st));
+  BF_CUDA(cudaMemsetAsync(g->d_flag, 0, ((g->n + 31) / 32) * 4, st));
   return BF_OK;
 }
 
@@ -580,7 +582,7 @@ bf_status plain_matrix(Graph* g, const uint32_t* d_src, uint64_t S, const uint32
                        uint64_t T, uint32_t threshold, uint32_t* d_out, cudaStream_t st,
                        bf_stats* stats) {
   bf_status s;
-  if ((s = plain_buffers(g))) return s;
+  if ((s = plain_buffers(g, st))) return s;
   const uint64_t nb = (S + PLAIN_K - 1) / PLAIN_K;
   uint64_t launches = 0;
   float t_up = 0, t_dn = 0, t_ex = 0;

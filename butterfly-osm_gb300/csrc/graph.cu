@@ -363,6 +363,8 @@ static bf_status build_graph_impl(const bf_cch_csr* csr, const bf_config* cfg, G
   g->h_in_rec = std::move(in_rec);
   g->h_in_len = std::move(in_len);
   g->has_len = two;
+  // the uploads, before work on streams that do not wait for the default one
+  BF_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
   (void)cfg;
   return BF_OK;
 }
