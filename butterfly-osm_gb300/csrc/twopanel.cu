@@ -23,6 +23,22 @@ __device__ __forceinline__ uint64_t lab_relax(uint64_t a, uint32_t wt, uint32_t 
   return min(acc, (uint64_t)t << 32 | l);
 }
 
+// A source's label into all K rows of a panel: its weights 16 bytes a load
+// (strides are multiples of four).
+template <uint32_t K>
+__device__ __forceinline__ void relax_source(uint64_t d, const uint32_t* wt, const uint32_t* wl,
+                                             uint64_t (&acc)[K]) {
+#pragma unroll
+  for (uint32_t j = 0; j < K; j += 4) {
+    const uint4 t = *reinterpret_cast<const uint4*>(wt + j);
+    const uint4 l = *reinterpret_cast<const uint4*>(wl + j);
+    acc[j] = lab_relax(d, t.x, l.x, acc[j]);
+    if (j + 1 < K) acc[j + 1] = lab_relax(d, t.y, l.y, acc[j + 1]);
+    if (j + 2 < K) acc[j + 2] = lab_relax(d, t.z, l.z, acc[j + 2]);
+    if (j + 3 < K) acc[j + 3] = lab_relax(d, t.w, l.w, acc[j + 3]);
+  }
+}
+
 struct TwoArgs {
   const uint4* item;       // panel items (Sched::d_pitem)
   const uint32_t* prow;    // slab rows of their sources
@@ -52,9 +68,14 @@ __device__ __forceinline__ void finish_rows(const TwoArgs& g, uint4 it, uint32_t
 #pragma unroll
   for (uint32_t i = 0; i + 1 < K; ++i)
 #pragma unroll
-    for (uint32_t j = i + 1; j < K; ++j) {
-      const uint32_t wl = tl[i * stride + j];
-      v[j] = lab_relax(v[i], time_of(tt[i * stride + j], wl), wl, v[j]);
+    for (uint32_t j4 = (i + 1) / 4 * 4; j4 < K; j4 += 4) {
+      const uint4 t = *reinterpret_cast<const uint4*>(tt + i * stride + j4);
+      const uint4 l = *reinterpret_cast<const uint4*>(tl + i * stride + j4);
+      const uint32_t wt[4] = {t.x, t.y, t.z, t.w}, wl[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q)
+        if (j4 + q > i && j4 + q < K)
+          v[j4 + q] = lab_relax(v[i], time_of(wt[q], wl[q]), wl[q], v[j4 + q]);
     }
 #pragma unroll
   for (uint32_t j = 0; j < K; ++j)
@@ -119,9 +140,7 @@ __device__ __forceinline__ void block_item(const TwoArgs& g, uint4 it, TwoSmem& 
         for (uint32_t q = 0; q < TP_FLIGHT; ++q) {
           const uint32_t s = s0 + q * TP_WARPS;
           if (s >= m) break;
-#pragma unroll
-          for (uint32_t j = 0; j < K; ++j)
-            acc[j] = lab_relax(d[q], sm.wt[s * stride + j], sm.wl[s * stride + j], acc[j]);
+          relax_source<K>(d[q], sm.wt + s * stride, sm.wl + s * stride, acc);
         }
       }
   }
@@ -143,8 +162,9 @@ __device__ __forceinline__ void block_item(const TwoArgs& g, uint4 it, TwoSmem& 
 
 // Bound by the chain of levels, and with u64 labels by a level's arithmetic (ten
 // instructions a weight). 60 x 90 ends of one to three seeds on the 1000 x 1250
-// region, whole call: 4.85 ms with a launch per level of rows, 0.98 ms by panels
-// (1.08 with two rows in flight and the seeds read at the end).
+// region, whole call: 4.85 ms with a launch per level of rows, 0.94 ms by panels
+// (1.08 with two rows in flight and the seeds read at the end, 0.96 with a load
+// per weight instead of one per four).
 __global__ void __launch_bounds__(32 * TP_WARPS) k_two_split(const TwoArgs g, uint32_t i0) {
   extern __shared__ __align__(16) unsigned char two_smem[];
   TwoSmem& sm = *reinterpret_cast<TwoSmem*>(two_smem);
