@@ -581,7 +581,7 @@ def run_isochrones(g, cch, count, seed=42):
                      "candidates": tune["tried"], "sample_ms": round(tune["step_ms"], 2)},
             "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak,
                          "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": None,
-                         "peak_kind": peak_kind, "kernel": "k_sweep_gated16 (all waves)",
+                         "peak_kind": peak_kind, "kernel": "k_iso_panels, k_iso_split (all waves)",
                          "alg_bytes": int(sweep_bytes), "sweep_ms": round(sweep_ms, 3),
                          "bytes_rule": "per wave: 16 B per work item + 8 B per edge record "
                                        "scanned, 2 B x lanes per active source row gathered "
