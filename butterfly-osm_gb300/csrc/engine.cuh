@@ -102,14 +102,20 @@ constexpr long long BARRIER_TIMEOUT_CYCLES = 4000000000ll;
 // The release/acquire pair orders each block's writes before the barrier
 // against every block's reads after it; callers read data other blocks wrote
 // through L2 (ld.cg), never through L1.
-__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t b, long long timeout,
-                                             uint32_t* err) {
-  __shared__ int s_ok;
+// In two halves: work between them that no other block waits for runs while the
+// others arrive.
+__device__ __forceinline__ void grid_arrive(uint32_t* bar) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    const uint32_t target = (b + 1) * gridDim.x;
     __threadfence();
     atomicAdd(bar, 1u);
+  }
+}
+__device__ __forceinline__ bool grid_wait(uint32_t* bar, uint32_t b, long long timeout,
+                                          uint32_t* err) {
+  __shared__ int s_ok;
+  if (threadIdx.x == 0) {
+    const uint32_t target = (b + 1) * gridDim.x;
     const long long t0 = clock64();
     int ok = 1;
     for (;;) {
@@ -133,6 +139,11 @@ __device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t b, long lon
   }
   __syncthreads();
   return s_ok != 0;
+}
+__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t b, long long timeout,
+                                             uint32_t* err) {
+  grid_arrive(bar);
+  return grid_wait(bar, b, timeout, err);
 }
 
 // Lanes per batch of the plain engine (one warp lane per source).

@@ -282,15 +282,16 @@ __device__ __forceinline__ void plain_small(const PlainArgs& g, uint32_t p, unsi
 
 // Bound by the chain of levels: a grid barrier and the dependent reads of
 // each. A level with few panels has a block share each one, what no earlier
-// level writes staged before the barrier; else every warp takes panels of its
+// level writes staged between its arrival at the barrier and its wait; else every warp takes panels of its
 // own: once a block's turn comes round more than four times, its warps do
 // better apart (twice or once: within 3 %). `withhold` (a test hook, NONE otherwise) names a block that leaves
 // before its first barrier arrival.
 //
-// Eight sources to all of the town's 119,249 nodes: sweep 615 -> 230 us, whole
-// call 849 -> 348; one source on grid100 2250 -> 570 us; a batch's sweep on the
-// 1000 x 1250 region 2.99 -> 1.44 ms, on the country graph 6.73 -> 4.71 (9.1 with
-// a warp for panels of up to four rows too).
+// Eight sources to all of the town's 119,249 nodes: sweep 615 -> 220 us, whole
+// call 849 -> 335 (348 with the staging before the arrival); one source on grid100
+// 2250 -> 550 us; a batch's sweep on the 1000 x 1250 region 2.99 -> 1.35 ms, on
+// the country graph 6.73 -> 4.55 (9.1 with a warp for panels of up to four rows
+// too).
 template <int PER_SM>
 __global__ void __launch_bounds__(32 * PP_WARPS, PER_SM)
     k_plain_panels(const PlainArgs g, uint32_t* __restrict__ bar, long long timeout,
@@ -336,11 +337,12 @@ __global__ void __launch_bounds__(32 * PP_WARPS, PER_SM)
       __syncthreads();
     }
     if (l + 1 == g.n_levels) break;
+    grid_arrive(bar);
     if (p2 - p1 <= share && p1 + blockIdx.x < p2) {
       stage(p1 + blockIdx.x);
       staged = true;
     }
-    if (!grid_barrier(bar, l, timeout, err)) return;
+    if (!grid_wait(bar, l, timeout, err)) return;
     p0 = p1;
     p1 = p2;
   }
