@@ -507,7 +507,8 @@ bf_status to_positions(Graph* g, const uint32_t* d_rank, uint64_t n, uint32_t* d
                        cudaStream_t st);
 bf_status check_device_error(Graph* g, cudaStream_t st);
 // plainpanel.cu: the sweep of one batch over panels (rows are ranks)
-bf_status plain_sweep_panels(Graph* g, uint32_t threshold, cudaStream_t st, uint64_t* launches);
+bf_status plain_sweep_panels(Graph* g, uint32_t k, uint32_t threshold, cudaStream_t st,
+                             uint64_t* launches);
 bf_status launch_upward(Graph* g, const uint32_t* d_src, uint64_t k, uint32_t threshold,
                         const uint32_t* pos_map, uint32_t* seed, uint32_t stride, uint32_t* flag,
                         cudaStream_t st, const uint32_t* lane_thr = nullptr,

@@ -563,8 +563,9 @@ static bf_status plain_sweep_persistent(Graph* g, uint32_t threshold, cudaStream
   return BF_OK;
 }
 
-static bf_status plain_sweep(Graph* g, uint32_t threshold, cudaStream_t st, uint64_t* launches) {
-  if (plain_by_panels(g)) return plain_sweep_panels(g, threshold, st, launches);
+static bf_status plain_sweep(Graph* g, uint32_t k, uint32_t threshold, cudaStream_t st,
+                             uint64_t* launches) {
+  if (plain_by_panels(g)) return plain_sweep_panels(g, k, threshold, st, launches);
   if (g->tune.persist & 1u) return plain_sweep_persistent(g, threshold, st, launches);
   for (uint32_t l = 0; l < g->n_levels; ++l) {
     uint32_t p0 = g->lvl_start[l], p1 = g->lvl_start[l + 1];
@@ -593,7 +594,7 @@ bf_status plain_matrix(Graph* g, const uint32_t* d_src, uint64_t S, const uint32
     if ((s = plain_upward(g, d_src + s0, k, threshold, st))) return s;
     ++launches;
     if (stats) BF_CUDA(cudaEventRecord(g->ev[1], st));
-    if ((s = plain_sweep(g, threshold, st, &launches))) return s;
+    if ((s = plain_sweep(g, k, threshold, st, &launches))) return s;
     if (stats) BF_CUDA(cudaEventRecord(g->ev[2], st));
     if (T) {
       dim3 blk(32, 8);

@@ -88,6 +88,12 @@ __device__ __forceinline__ uint32_t take_seed(const PlainArgs& g, uint32_t r, ui
   return v;
 }
 
+// The minimum over the four groups of eight lanes.
+__device__ __forceinline__ uint32_t across(uint32_t v) {
+  v = min(v, __shfl_xor_sync(0xFFFFFFFFu, v, 8));
+  return min(v, __shfl_xor_sync(0xFFFFFFFFu, v, 16));
+}
+
 // What a shared panel needs that no earlier level writes: each warp's first
 // chunk, the triangle and the seeds. Returns the warp's source ids.
 template <uint32_t K>
@@ -108,11 +114,15 @@ __device__ __forceinline__ uint32_t stage_shared(const PlainArgs& g, const uint4
 }
 
 // A panel (stride K) by one warp, or with SHARED by all warps of the block, a
-// chunk of the sources each, staged before (id: its first chunk's ids).
-template <uint32_t K, bool SHARED>
+// chunk of the sources each, staged before (id: its first chunk's ids). NARROW
+// (at most 8 lanes hold sources): four of the panel's sources side by side, eight
+// lanes each, their minima combined at the end.
+template <uint32_t K, bool SHARED, bool NARROW>
 __device__ __forceinline__ void plain_panel(const PlainArgs& g, const uint4 a, const uint2 b,
                                             uint32_t id, PlainSmem& sm) {
   const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  constexpr uint32_t SIDE = NARROW ? 4 : 1;  // sources side by side
+  const uint32_t at = NARROW ? lane & 7 : lane, side = NARROW ? lane >> 3 : 0;
   const uint32_t rows = a.y & 0xFF, nu = a.z;
   uint32_t* ws = sm.w[wib];
   uint32_t* tri = sm.tri[SHARED ? 0 : wib];
@@ -130,23 +140,23 @@ __device__ __forceinline__ void plain_panel(const PlainArgs& g, const uint4 a, c
   for (uint32_t j = 0; j < K; ++j) acc[j] = INF;
   while (c0 < nu) {
     const uint32_t m = min(ch, nu - c0), next = c0 + step;
-    uint32_t d[PP_CH];
+    uint32_t d[PP_CH / SIDE];
 #pragma unroll
-    for (uint32_t s = 0; s < PP_CH; ++s) {
-      const uint32_t r = __shfl_sync(0xFFFFFFFFu, id, s);
-      d[s] = s < m ? __ldcg(g.dist + (size_t)r * PLAIN_K + lane) : INF;
+    for (uint32_t q = 0; q < PP_CH / SIDE; ++q) {
+      const uint32_t s = q * SIDE + side, r = __shfl_sync(0xFFFFFFFFu, id, s);
+      d[q] = s < m ? __ldcg(g.dist + (size_t)r * PLAIN_K + at) : INF;
     }
     if (next < nu) load_chunk<K>(g, b, next, min(ch, nu - next), lane, &id, wv);
 #pragma unroll
-    for (uint32_t s = 0; s < PP_CH; ++s) {
-      if (s >= m) break;
+    for (uint32_t q = 0; q < PP_CH / SIDE; ++q) {
+      if (q * SIDE >= m) break;
 #pragma unroll
       for (uint32_t j = 0; j < K; j += 4) {
-        const uint4 x = *reinterpret_cast<const uint4*>(ws + s * K + j);
-        acc[j] = min_plus(d[s], x.x, acc[j]);
-        acc[j + 1] = min_plus(d[s], x.y, acc[j + 1]);
-        acc[j + 2] = min_plus(d[s], x.z, acc[j + 2]);
-        acc[j + 3] = min_plus(d[s], x.w, acc[j + 3]);
+        const uint4 x = *reinterpret_cast<const uint4*>(ws + (q * SIDE + side) * K + j);
+        acc[j] = min_plus(d[q], x.x, acc[j]);
+        acc[j + 1] = min_plus(d[q], x.y, acc[j + 1]);
+        acc[j + 2] = min_plus(d[q], x.z, acc[j + 2]);
+        acc[j + 3] = min_plus(d[q], x.w, acc[j + 3]);
       }
     }
     __syncwarp();
@@ -162,6 +172,7 @@ __device__ __forceinline__ void plain_panel(const PlainArgs& g, const uint4 a, c
       uint32_t v = sm.seed[j][lane];
 #pragma unroll
       for (uint32_t q = 0; q < PP_WARPS; ++q) v = min(v, sm.red[q][j][lane]);
+      if (NARROW) v = across(v);
       sm.red[0][j][lane] = v;
     }
     __syncthreads();
@@ -171,6 +182,9 @@ __device__ __forceinline__ void plain_panel(const PlainArgs& g, const uint4 a, c
 #pragma unroll
       for (uint32_t j = 0; j < K; ++j) acc[j] = sm.red[0][j][lane];
     } else {
+      if (NARROW)
+#pragma unroll
+        for (uint32_t j = 0; j < K; ++j) acc[j] = across(acc[j]);
       const uint32_t w0 = (a.x + 1 - rows) >> 5, w1 = a.x >> 5;
       const uint32_t f0 = __ldcg(g.flag + w0), f1 = w1 == w0 ? f0 : __ldcg(g.flag + w1);
 #pragma unroll
@@ -192,30 +206,32 @@ __device__ __forceinline__ void plain_panel(const PlainArgs& g, const uint4 a, c
       }
 #pragma unroll
     for (uint32_t j = 0; j < K; ++j)
-      if (j < rows)
-        g.dist[(size_t)(a.x - j) * PLAIN_K + lane] = acc[j] > g.threshold ? INF : acc[j];
+      if (j < rows && side == 0)
+        g.dist[(size_t)(a.x - j) * PLAIN_K + at] = acc[j] > g.threshold ? INF : acc[j];
     __syncwarp();  // (the warp's next panel writes the shared tile and triangle)
   }
   if (SHARED) __syncthreads();
 }
 
-// A panel of up to four rows by eight threads, four lanes each (m8: their bits
-// of the warp): four panels of a warp at a time, and rows, weights and seeds move
-// 16 bytes a load.
+// A panel of up to four rows by G threads, four lanes each (eight, or two where
+// at most 8 lanes hold sources; mg: their bits of the warp): several panels of a
+// warp at a time, and rows, weights and seeds move 16 bytes a load.
 __device__ __forceinline__ uint4 min_plus4(const uint4 d, uint32_t w, const uint4 acc) {
   return make_uint4(min_plus(d.x, w, acc.x), min_plus(d.y, w, acc.y), min_plus(d.z, w, acc.z),
                     min_plus(d.w, w, acc.w));
 }
 
-__device__ __forceinline__ void plain_small(const PlainArgs& g, uint32_t p, unsigned m8) {
+template <uint32_t G>
+__device__ __forceinline__ void plain_small(const PlainArgs& g, uint32_t p) {
+  const unsigned mg = ((1u << G) - 1) << (threadIdx.x & 31 & ~(G - 1));
   constexpr uint32_t K = 4, U = 4;  // source rows in flight
   const uint4 a = g.a[p];
   const uint2 b = g.b[p];
-  const uint32_t rows = a.y & 0xFF, nu = a.z, l4 = (threadIdx.x & 7) * 4;
+  const uint32_t rows = a.y & 0xFF, nu = a.z, l4 = (threadIdx.x & (G - 1)) * 4;
   const uint32_t* tile = g.w + b.y;
   const uint32_t w0 = (a.x + 1 - rows) >> 5, w1 = a.x >> 5;
   const uint32_t f0 = __ldcg(g.flag + w0), f1 = w1 == w0 ? f0 : __ldcg(g.flag + w1);
-  __syncwarp(m8);  // (all have read the bits before one clears them)
+  __syncwarp(mg);  // (all have read the bits before one clears them)
   uint4 acc[K];
 #pragma unroll
   for (uint32_t j = 0; j < K; ++j) {
@@ -282,17 +298,18 @@ __device__ __forceinline__ void plain_small(const PlainArgs& g, uint32_t p, unsi
 
 // Bound by the chain of levels: a grid barrier and the dependent reads of
 // each. A level with few panels has a block share each one, what no earlier
-// level writes staged between its arrival at the barrier and its wait; else every warp takes panels of its
-// own: once a block's turn comes round more than four times, its warps do
-// better apart (twice or once: within 3 %). `withhold` (a test hook, NONE otherwise) names a block that leaves
-// before its first barrier arrival.
+// level writes staged between its arrival at the barrier and its wait; else
+// every warp takes panels of its own: once a block's turn comes round more than
+// four times, its warps do better apart (twice or once: within 3 %). `withhold`
+// (a test hook, NONE otherwise) names a block that leaves before its first
+// barrier arrival.
 //
-// Eight sources to all of the town's 119,249 nodes: sweep 615 -> 220 us, whole
-// call 849 -> 335 (348 with the staging before the arrival); one source on grid100
-// 2250 -> 550 us; a batch's sweep on the 1000 x 1250 region 2.99 -> 1.35 ms, on
-// the country graph 6.73 -> 4.55 (9.1 with a warp for panels of up to four rows
-// too).
-template <int PER_SM>
+// 29 sources to all of the town's 119,249 nodes: sweep 615 -> 220 us, whole call
+// 849 -> 335 (348 with the staging before the arrival). A batch's sweep on the
+// 1000 x 1250 region 2.99 -> 1.36 ms, on the country graph 6.73 -> 4.58 (9.1 with
+// a warp for panels of up to four rows too). NARROW, eight sources: 0.93 and 2.73
+// ms there; one source on grid100, whole call: 546 -> 452 us (2250 by rows).
+template <int PER_SM, bool NARROW>
 __global__ void __launch_bounds__(32 * PP_WARPS, PER_SM)
     k_plain_panels(const PlainArgs g, uint32_t* __restrict__ bar, long long timeout,
                    uint32_t withhold, uint32_t* __restrict__ err) {
@@ -317,7 +334,7 @@ __global__ void __launch_bounds__(32 * PP_WARPS, PER_SM)
       for (uint32_t p = p0 + blockIdx.x; p < p1; p += gridDim.x) {
         if (!staged) stage(p);
         staged = false;
-#define BF_SOLVE(K) plain_panel<K, true>(g, a, b, id, sm)
+#define BF_SOLVE(K) plain_panel<K, true, NARROW>(g, a, b, id, sm)
         BF_BY_STRIDE(a, BF_SOLVE)
 #undef BF_SOLVE
       }
@@ -327,13 +344,14 @@ __global__ void __launch_bounds__(32 * PP_WARPS, PER_SM)
            p += gridDim.x * PP_WARPS) {
         const uint4 wa = g.a[p];
         const uint2 wb = g.b[p];
-#define BF_SOLVE(K) plain_panel<K, false>(g, wa, wb, 0, sm)
+#define BF_SOLVE(K) plain_panel<K, false, NARROW>(g, wa, wb, 0, sm)
         BF_BY_STRIDE(wa, BF_SOLVE)
 #undef BF_SOLVE
       }
-      for (uint32_t p = ps + (blockIdx.x * PP_WARPS * 32 + threadIdx.x) / 8; p < p1;
-           p += gridDim.x * PP_WARPS * 4)
-        plain_small(g, p, 0xFFu << (threadIdx.x & 24));
+      constexpr uint32_t G = NARROW ? 2 : 8;
+      for (uint32_t p = ps + (blockIdx.x * PP_WARPS * 32 + threadIdx.x) / G; p < p1;
+           p += gridDim.x * PP_WARPS * 32 / G)
+        plain_small<G>(g, p);
       __syncthreads();
     }
     if (l + 1 == g.n_levels) break;
@@ -351,7 +369,8 @@ __global__ void __launch_bounds__(32 * PP_WARPS, PER_SM)
 
 }  // namespace
 
-bf_status plain_sweep_panels(Graph* g, uint32_t threshold, cudaStream_t st, uint64_t* launches) {
+bf_status plain_sweep_panels(Graph* g, uint32_t k, uint32_t threshold, cudaStream_t st,
+                             uint64_t* launches) {
   bf_status s;
   if ((s = ensure_barrier(g))) return s;
   const Panels& P = g->panels;
@@ -362,7 +381,9 @@ bf_status plain_sweep_panels(Graph* g, uint32_t threshold, cudaStream_t st, uint
   // their kernel spills (country graph 4.7 ms a batch against 5.45 with two an
   // SM, the town 400 us a call against 361)
   const bool wide = (uint64_t)g->n * PLAIN_K * 4 > (128ull << 20);
-  const auto kern = wide ? k_plain_panels<4> : k_plain_panels<2>;
+  const bool narrow = k <= 8;
+  const auto kern = wide ? narrow ? k_plain_panels<4, true> : k_plain_panels<4, false>
+                         : narrow ? k_plain_panels<2, true> : k_plain_panels<2, false>;
   const unsigned blocks = persistent_blocks(g, (const void*)kern, 32 * PP_WARPS,
                                             (wide ? 4 : 2) * g->sm_count);
   BF_CUDA(cudaMemsetAsync(g->d_bar, 0, 8, st));

@@ -261,7 +261,7 @@ def test_plain_sweep_by_panels(built, name):
     g.set_engine(bfphast.ENGINE_PLAIN)
     rng = np.random.default_rng(n)
     every = np.arange(n, dtype=np.uint32)
-    for k in (1, 31, 32, 33, 100):
+    for k in (1, 8, 9, 31, 32, 33, 100):
         src = rng.integers(0, n, k).astype(np.uint32)
         tgt = rng.integers(0, n, 7).astype(np.uint32)
         want, _ = c.matrix(src, every)
