@@ -1390,6 +1390,9 @@ __global__ void __launch_bounds__(32 * (RING_WARPS + 1), 3)
   }
 }
 
+// Units per SM from which a wave of 68 to 128 lanes takes the ring form.
+constexpr uint64_t RING_NARROW = 8;
+
 template <bool SAT>
 cudaError_t launch_panels(const Graph* g, const Sched& sc, uint32_t i0, uint32_t m, uint32_t* slab,
                           uint32_t Kp, const uint32_t* seeded, bool pdl, cudaStream_t st) {
@@ -1398,9 +1401,13 @@ cudaError_t launch_panels(const Graph* g, const Sched& sc, uint32_t i0, uint32_t
   // A thread of the ring form walks all sources of its panel (up to a few
   // hundred at the top of the tree): with few units in a level that chain is
   // the level's time, so the split form takes levels of fewer than two units
-  // per SM, and narrow waves, whose tile would be mostly empty.
-  if ((uint64_t)m * tiles >= 2ull * g->sm_count && (uint64_t)m * tiles < 0x80000000ull &&
-      Kp > 128) {
+  // per SM (fewer than eight at up to 128 lanes, whose tile is mostly empty; at
+  // up to 64 it wins in any level). 100 sources: to 10,000 ends on the country
+  // graph 1.29 ms against 1.49 by the split form alone, to 5000 on the region
+  // 0.60 against 0.68, on grid100 0.38 either way (0.40 from two units).
+  const uint64_t units = (uint64_t)m * tiles;
+  const uint64_t enough = (Kp > 128 ? 2ull : RING_NARROW) * g->sm_count;
+  if (units >= enough && units < 0x80000000ull && Kp > 64) {
     const uint32_t grid = std::min<uint32_t>(m * tiles, 3 * g->sm_count);
     return launch_level_smem(k_sweep_panels_ring<SAT>, dim3(grid), 32 * (RING_WARPS + 1),
                              sizeof(RingSmem), pdl, st, (const uint4*)sc.d_pitem, i0, m, tiles, (const uint32_t*)sc.d_prow,

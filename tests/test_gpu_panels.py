@@ -104,7 +104,7 @@ def test_upward_by_panels_with_thresholds(built, name):
             assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), (o, t)
 
 
-@pytest.mark.parametrize("S", [130, 512, 516, 1030])
+@pytest.mark.parametrize("S", [64, 68, 100, 128, 130, 512, 516, 1030])
 def test_panels_wide_levels(built, grid100, S):
     """Every node a target: levels of thousands of panels, lane blocks of 512
     and what is left of them, every block size."""
