@@ -568,7 +568,8 @@ bf_status build_schedule_device(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_t
                                 const uint32_t* d_tgt, uint64_t T, uint64_t key, cudaStream_t st);
 // Rows and edges that reach the schedule's targets (a panel schedule sweeps a
 // few more), counted on the context's side stream from here; finish_counts
-// waits for them and stores them in the schedule.
+// waits for them and stores them in the schedule, or reports that the count's
+// own bounded wait ran out (the graph's error word is not touched).
 bf_status start_counts(Graph* g, Ctx& c, Sched& sc, cudaStream_t st);
 bf_status finish_counts(Ctx& c, Sched& sc);
 // Per-level item, edge and row tables of a schedule in the panel form.

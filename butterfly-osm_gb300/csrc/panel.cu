@@ -652,10 +652,11 @@ struct PanelScratch {
   uint32_t* pre = nullptr;    // [W + 1] and [PW + 1] bit counts before each word
   uint32_t* bsum = nullptr;
   uint32_t* list = nullptr;   // [panels] opened panels
-  // [W + 1] rows that reach a target; two counters, the grid-barrier words
+  // [W + 1] rows that reach a target; two counters, the grid-barrier words, the
+  // count's own error bits (COUNT_WORDS together)
   uint32_t* live = nullptr;
   uint32_t* tgt = nullptr;    // uploaded targets
-  unsigned long long* h_counts = nullptr;  // page-locked: rows, edges
+  unsigned long long* h_counts = nullptr;  // page-locked: rows, edges, barrier, error bits
   bool counting = false;      // start_counts has work on the side stream
   uint64_t bytes = 0;         // device memory of the graph-sized arrays and the targets
   uint32_t* h_back = nullptr;  // page-locked: sources, cursor, rows, level table
@@ -717,6 +718,7 @@ void drop_panel_schedule(Graph* g, Ctx& c, Sched& sc) {
 
 // Words of the live bitmap, even: two 64-bit counters lie behind it.
 static size_t live_words(uint32_t n) { return (((size_t)n + 31) / 32 + 2) & ~(size_t)1; }
+constexpr size_t COUNT_WORDS = 8, COUNT_ERR = 6;
 
 bf_status start_counts(Graph* g, Ctx& c, Sched& sc, cudaStream_t st) {
   if (!sc.panel) {
@@ -731,7 +733,7 @@ bf_status start_counts(Graph* g, Ctx& c, Sched& sc, cudaStream_t st) {
   uint32_t* tot = s.live + live_words(g->n);
   if (sc.uses) {  // (a reused schedule: the counters are those of its build)
     BF_CUDA(cudaStreamSynchronize(c.cnt));
-    BF_CUDA(cudaMemsetAsync(tot, 0, 24, st));
+    BF_CUDA(cudaMemsetAsync(tot, 0, COUNT_WORDS * 4, st));
   }
   BF_CUDA(cudaEventRecord(c.cnt_fork, st));
   BF_CUDA(cudaStreamWaitEvent(c.cnt, c.cnt_fork, 0));
@@ -744,8 +746,9 @@ bf_status start_counts(Graph* g, Ctx& c, Sched& sc, cudaStream_t st) {
                             (const uint16_t*)P.d_em, (const uint16_t*)P.d_tm,
                             (const uint32_t*)g->d_pos_of, (const uint64_t*)g->d_in_off, s.live,
                             reinterpret_cast<unsigned long long*>(tot), tot + 4,
-                            hook ? 2000000ll : BARRIER_TIMEOUT_CYCLES, hook ? 1u : NONE, g->d_err));
-  BF_CUDA(cudaMemcpyAsync(s.h_counts, tot, 16, cudaMemcpyDeviceToHost, c.cnt));
+                            hook ? 2000000ll : BARRIER_TIMEOUT_CYCLES, hook ? 1u : NONE,
+                            tot + COUNT_ERR));
+  BF_CUDA(cudaMemcpyAsync(s.h_counts, tot, COUNT_WORDS * 4, cudaMemcpyDeviceToHost, c.cnt));
   s.counting = true;
   return BF_OK;
 }
@@ -754,6 +757,11 @@ bf_status finish_counts(Ctx& c, Sched& sc) {
   if (!c.ps || !c.ps->counting) return BF_OK;
   c.ps->counting = false;
   BF_CUDA(cudaStreamSynchronize(c.cnt));
+  // (a count that gave up is partial: the next call counts again)
+  if (reinterpret_cast<const uint32_t*>(c.ps->h_counts)[COUNT_ERR]) {
+    set_error("a bounded device wait ran out (row counts)");
+    return BF_ERR_TIMEOUT;
+  }
   sc.n_live = (uint32_t)c.ps->h_counts[0];
   sc.n_edges = c.ps->h_counts[1];
   sc.counted = true;
@@ -792,11 +800,12 @@ bf_status build_schedule_panels(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_t
     if ((rc = grow(&s.bits, none = 0, meta + 3 + L + 1, g, false)) ||
         (rc = grow(&s.pre, none = 0, meta, g, false)) ||
         (rc = grow(&s.bsum, none = 0, 2 * (size_t)nb, g, false)) ||
-        (rc = grow(&s.live, none = 0, live_words(n) + 6, g, false)) ||
+        (rc = grow(&s.live, none = 0, live_words(n) + COUNT_WORDS, g, false)) ||
         (rc = grow(&s.list, none = 0, P.n, g, false)))
       return rc;
     s.bytes = g->device_bytes - before;
-    if (!s.h_counts && cudaHostAlloc((void**)&s.h_counts, 16, cudaHostAllocDefault) != cudaSuccess) {
+    if (!s.h_counts && cudaHostAlloc((void**)&s.h_counts, COUNT_WORDS * 4,
+                                      cudaHostAllocDefault) != cudaSuccess) {
       cudaGetLastError();
       s.h_counts = nullptr;
       set_error("cannot allocate the row-count read-back buffer");
@@ -844,7 +853,7 @@ bf_status build_schedule_panels(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_t
   if ((rc = grow(&sc.d_pitem, sc.cap_pitem, m, g, true)) ||
       (rc = grow(&sc.d_prow, sc.cap_prow, n_rows, g, true)))
     return rc;
-  BF_CUDA(cudaMemsetAsync(s.live, 0, (live_words(n) + 6) * 4, st));
+  BF_CUDA(cudaMemsetAsync(s.live, 0, (live_words(n) + COUNT_WORDS) * 4, st));
   const uint64_t threads = std::max<uint64_t>((uint64_t)m * 32, T);
   k_pn_items<<<(unsigned)std::min<uint64_t>((threads + 255) / 256, 152 * 32), 256, 0, st>>>(
       s.list, m, P.d_a, P.d_b, P.d_src, rows, wpre, sc.d_cidx, n_src + 1, sc.d_pitem,

@@ -231,6 +231,7 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
   }
   trim_call_buffer(c);
   if ((rc = check_device_error(g, s))) return rc;
+  if (st && (rc = finish_counts(c, sc))) return rc;
   // same-rank pairs belong to the caller's bucket engine (bucket_ch.rs:6786-6845)
   std::unordered_map<uint32_t, std::vector<uint32_t>> src_at;
   for (uint64_t si = 0; si < S; ++si)
@@ -249,7 +250,6 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
   if (n_conflicts) *n_conflicts = cells.size();
   for (uint64_t i = 0; i < cells.size() && i < conflict_cap; ++i) conflicts[i] = cells[i];
   if (st) {
-    if ((rc = finish_counts(c, sc))) return rc;
     st->n_batches += (S + wave - 1) / wave;
     st->waves += (S + wave - 1) / wave;
     st->kernel_launches += launches;

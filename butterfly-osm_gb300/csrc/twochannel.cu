@@ -478,6 +478,7 @@ bf_status matrix_seeded_2ch(Graph* g, Ctx& c, const bf_seed2* src_seeds, const u
   }
   trim_call_buffer(c);
   if ((rc = check_device_error(g, s))) return rc;
+  if (st && (rc = finish_counts(c, sc))) return rc;
   // same-rank pairs belong to the caller's two-channel bucket engine
   // (bucket_ch.rs:6460-6463, :6497-6516)
   std::unordered_map<uint32_t, std::vector<uint32_t>> src_at;
@@ -499,7 +500,6 @@ bf_status matrix_seeded_2ch(Graph* g, Ctx& c, const bf_seed2* src_seeds, const u
   if (n_conflicts) *n_conflicts = cells.size();
   for (uint64_t i = 0; i < cells.size() && i < conflict_cap; ++i) conflicts[i] = cells[i];
   if (st) {
-    if ((rc = finish_counts(c, sc))) return rc;
     st->n_batches += (S + wave - 1) / wave;
     st->waves += (S + wave - 1) / wave;
     st->kernel_launches += launches;
