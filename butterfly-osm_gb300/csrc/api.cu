@@ -415,7 +415,10 @@ bf_status bf_schedule_levels(const bf_graph* h, uint32_t cap, uint64_t* items, u
       return cuda_status(cudaGetLastError(), "cudaSetDevice");
     bf_status rc = schedule_tables(g, g->ctx, sc, g->stream);
     if (rc == BF_OK) rc = check_device_error(g, g->stream);
-    if (rc) return rc;
+    if (rc) {  // (a selection that gave up names too many rows)
+      sc.lvl_item.clear();
+      return rc;
+    }
   }
   if (!sc.valid || sc.lvl_item.size() < 2 || sc.lvl_row.size() != sc.lvl_item.size() ||
       sc.lvl_edge.size() != sc.lvl_item.size()) {

@@ -71,3 +71,18 @@ def test_seeded_calls_report_a_timeout(built, country_small):
         _timeout(lambda: call(g))
         assert np.array_equal(g.matrix(src, tgt), want)
         assert np.array_equal(call(g), call(host))
+
+
+def test_level_table_after_a_timeout(built, country_small):
+    """bf_schedule_levels of a schedule over panels selects the rows on its own."""
+    _, cch = country_small
+    g, host = _graphs(cch)
+    rng = np.random.default_rng(5)
+    src = rng.integers(0, cch["n"], 4).astype(np.uint32)
+    tgt = rng.choice(cch["n"], 400, replace=False).astype(np.uint32)
+    want = host.matrix(src, tgt)
+    assert np.array_equal(g.matrix(src, tgt), want)
+    _timeout(g.schedule_levels)
+    for a, b in zip(g.schedule_levels(), host.schedule_levels()):
+        assert np.array_equal(a, b)
+    assert np.array_equal(g.matrix(src, tgt), want)
