@@ -427,6 +427,10 @@ inline std::vector<uint2> level_program(const std::vector<uint32_t>& first, uint
 // millisecond, so the call must report BF_ERR_TIMEOUT.
 bool test_withhold_arrival();
 
+// Test hook of allocations that may fail: those named by BF_TEST_FAIL_ALLOC in the
+// environment fail as if the device's memory had run out.
+bool test_fail_alloc(const char* what);
+
 // f(i) for i in [0, n) on up to 64 host threads (dynamic assignment).
 template <class F>
 inline void parallel_for(uint64_t n, F&& f) {

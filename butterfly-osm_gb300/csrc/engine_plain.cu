@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <cstring>
 
 #include "engine.cuh"
 
@@ -415,6 +416,11 @@ bf_status check_device_error(Graph* g, cudaStream_t st) {
 }
 
 bool test_withhold_arrival() { return std::getenv("BF_TEST_WITHHOLD_ARRIVAL") != nullptr; }
+
+bool test_fail_alloc(const char* what) {
+  const char* v = std::getenv("BF_TEST_FAIL_ALLOC");
+  return v && std::strcmp(v, what) == 0;
+}
 
 // The seed rows and bits start clear on `st`, before the call's own work there (a
 // memset on the default stream would run beside a stream that does not wait for it).

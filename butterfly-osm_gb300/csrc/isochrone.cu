@@ -986,12 +986,15 @@ bf_status isochrone_bitsets(Graph* g, Ctx& c, const uint32_t* d_orig, const uint
   // by panels (isopanel.cu), in tiles of 64 lanes, unless another form is asked
   // for or the budget holds no tile
   const uint64_t tile_bytes = rows * 128, words_bytes = 2 * rows * 4 + 2048 * 2 + 32;
+  auto scratch = [&](bool by_panels) {
+    return pk.size() * 4 + (by_panels ? words_bytes : 2 * aw * 4) + 32;
+  };
   const bool panels = half && upward_by_panels(g) && !(g->tune.persist & 2u) && !g->tune.staged &&
-                      ctx_budget(g, c) >= tile_bytes + words_bytes + pk.size() * 4 + 16;
+                      ctx_budget(g, c) >= tile_bytes + scratch(true);
   Sched* sc = c.shared_full ? c.shared_full : &c.full;
   if (!panels && !c.shared_full && (s = build_schedule(g, c, c.full, nullptr, 0, true, st)))
     return s;
-  const size_t need = pk.size() * 4 + (panels ? words_bytes : 2 * aw * 4) + 32;
+  const size_t need = scratch(panels);
   if (need > c.iso_tmp_bytes) {
     if (c.d_iso_tmp) {
       cudaFree(c.d_iso_tmp);

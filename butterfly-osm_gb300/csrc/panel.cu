@@ -178,7 +178,7 @@ void emit_panels(uint32_t lo, uint32_t hi, uint32_t ci, const Edges& dn, const E
 template <class T>
 bf_status upload(T** d, const std::vector<T>& h, Panels& P) {
   const size_t bytes = std::max<size_t>(h.size(), 1) * sizeof(T);
-  if (cudaMalloc((void**)d, bytes) != cudaSuccess) {
+  if (test_fail_alloc("panels") || cudaMalloc((void**)d, bytes) != cudaSuccess) {
     cudaGetLastError();
     *d = nullptr;
     return BF_ERR_OOM;

@@ -1,0 +1,53 @@
+"""Device memory: the budget a graph is created with, allocations that fail,
+and buffers kept between calls. Failures are made by BF_TEST_FAIL_ALLOC (the
+named allocation reports that the device's memory has run out)."""
+import contextlib
+import os
+
+import numpy as np
+import pytest
+
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+INF = 0xFFFFFFFF
+
+
+@contextlib.contextmanager
+def _env(name, value):
+    os.environ[name] = value
+    try:
+        yield
+    finally:
+        del os.environ[name]
+
+
+def _fails(what, call):
+    import bfphast
+    with _env("BF_TEST_FAIL_ALLOC", what), pytest.raises(bfphast.BfError) as e:
+        call()
+    assert e.value.status == bfphast.BF_ERR_OOM
+
+
+def _without_panels(cch, **kw):
+    import bfphast
+    with _env("BF_TEST_FAIL_ALLOC", "panels"):
+        return bfphast.Graph.from_cch(cch, **kw)
+
+
+def test_isochrones_of_a_budget_at_one_tile(built):
+    """Budgets around what a tile of 64 lanes and its scratch take: each is
+    served, by the tile or by items."""
+    import bfphast
+    from test_gpu_panels import _band, _cch
+    n, count = 180, 5
+    cch = _cch(n, _band(n, 1), 3, 1, 60, 0.2)  # (its items take less than a tile)
+    c = orc.Cch.from_dict(cch)
+    org = np.arange(0, count * 30, 30, dtype=np.uint32)
+    thr = np.full(count, 300, np.uint32)
+    want, _ = c.isochrone_bitsets(org, thr)
+    own = _without_panels(cch).info()["device_bytes"]
+    tile = own + 128 * n + 2 * 4 * n + 4096 + 32 + 12 * count
+    for budget in [tile + k for k in range(-4, 400, 4)] + [1 << 20, 4 << 20]:
+        g = bfphast.Graph.from_cch(cch, hbm_budget=budget)
+        assert np.array_equal(g.isochrone_bitsets(org, thr)[0], want), budget - tile
