@@ -428,17 +428,25 @@ inline std::vector<uint2> level_program(const std::vector<uint32_t>& first, uint
 bool test_withhold_arrival();
 
 // Test hook of allocations that may fail: those named by BF_TEST_FAIL_ALLOC in the
-// environment fail as if the device's memory had run out.
+// environment fail as if the device's (or the host's) memory had run out.
 bool test_fail_alloc(const char* what);
 
-// f(i) for i in [0, n) on up to 64 host threads (dynamic assignment).
+// f(i) for i in [0, n) on up to 64 host threads (dynamic assignment). An exception
+// of f stops the others at their next i and is thrown here.
 template <class F>
 inline void parallel_for(uint64_t n, F&& f) {
   const unsigned nt = std::max(1u, std::min<unsigned>(std::thread::hardware_concurrency(),
                                                       (unsigned)std::min<uint64_t>(n, 64)));
   std::atomic<uint64_t> next{0};
+  std::atomic<bool> failed{false};
+  std::exception_ptr what;
   auto work = [&]() {
-    for (uint64_t i; (i = next.fetch_add(1)) < n;) f(i);
+    try {
+      for (uint64_t i; (i = next.fetch_add(1)) < n;) f(i);
+    } catch (...) {
+      next = n;
+      if (!failed.exchange(true)) what = std::current_exception();
+    }
   };
   std::vector<std::thread> pool;
   try {
@@ -448,6 +456,7 @@ inline void parallel_for(uint64_t n, F&& f) {
   }
   work();
   for (auto& th : pool) th.join();
+  if (what) std::rethrow_exception(what);
 }
 
 // One level launch; with `pdl` it is a programmatic dependent of the

@@ -225,22 +225,15 @@ void free_panels(Panels& P) {
   P = Panels();
 }
 
-// Panels of the DOWN edges by target rank (in-edges of v: off, src, w; src > v)
-// and the UP edges by source rank (records {depth difference, w}), on runs given
-// by run_end. Leaves P empty (items and paths then serve every call) when the
-// tiles do not fit 32-bit offsets or the device.
-bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
-                       const std::vector<uint32_t>& parent, const std::vector<uint32_t>& depth,
-                       const std::vector<uint64_t>& off, const std::vector<uint32_t>& src,
-                       const std::vector<uint32_t>& w, const std::vector<uint64_t>& up_off,
-                       const std::vector<uint2>& up_rec, uint64_t max_up, const uint32_t* len,
-                       const uint32_t* up_len) {
+static bf_status make_panels(Graph* g, const std::vector<uint32_t>& run_end,
+                             const std::vector<uint32_t>& parent,
+                             const std::vector<uint32_t>& depth, const std::vector<uint64_t>& off,
+                             const std::vector<uint32_t>& src, const std::vector<uint32_t>& w,
+                             const std::vector<uint64_t>& up_off, const std::vector<uint2>& up_rec,
+                             uint64_t max_up, const uint32_t* len, const uint32_t* up_len) {
   Panels& P = g->panels;
   const uint32_t n = g->n;
   bf_status rc;
-  if ((rc = panel_kernels_init()) || (rc = upward_kernel_init()) ||
-      (rc = upward_2ch_kernel_init()))
-    return rc;
   if (!n || off[n] >= 0x20000000ull || up_off[n] >= 0x20000000ull) return BF_OK;
   std::vector<uint32_t> up_end(up_off[n]), up_w(up_off[n]);
   parallel_for((n + 65535) / 65536, [&](uint64_t c) {
@@ -263,6 +256,7 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
   std::vector<Chunk> ch(nc);
   std::vector<uint16_t> tm(n, 0);  // by rank: the rows of its panel it has an edge into
   parallel_for(nc, [&](uint64_t c) {
+    if (test_fail_alloc("panel_tiles")) throw std::bad_alloc();
     std::vector<uint32_t> uni[2];
     // runs from the highest rank down; a run's panels from its end down
     for (uint32_t v = cut[c + 1]; v > cut[c];) {
@@ -394,6 +388,29 @@ bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
     return rc == BF_ERR_OOM ? BF_OK : rc;
   }
   return BF_OK;
+}
+
+// Panels of the DOWN edges by target rank (in-edges of v: off, src, w; src > v)
+// and the UP edges by source rank (records {depth difference, w}), on runs given
+// by run_end. Leaves P empty (items and paths then serve every call) when the
+// tiles do not fit 32-bit offsets, the device or the host's memory.
+bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
+                       const std::vector<uint32_t>& parent, const std::vector<uint32_t>& depth,
+                       const std::vector<uint64_t>& off, const std::vector<uint32_t>& src,
+                       const std::vector<uint32_t>& w, const std::vector<uint64_t>& up_off,
+                       const std::vector<uint2>& up_rec, uint64_t max_up, const uint32_t* len,
+                       const uint32_t* up_len) {
+  bf_status rc;
+  if ((rc = panel_kernels_init()) || (rc = upward_kernel_init()) ||
+      (rc = upward_2ch_kernel_init()))
+    return rc;
+  try {
+    return make_panels(g, run_end, parent, depth, off, src, w, up_off, up_rec, max_up, len,
+                       up_len);
+  } catch (const std::bad_alloc&) {
+    free_panels(g->panels);
+    return BF_OK;
+  }
 }
 
 namespace {

@@ -51,3 +51,15 @@ def test_isochrones_of_a_budget_at_one_tile(built):
     for budget in [tile + k for k in range(-4, 400, 4)] + [1 << 20, 4 << 20]:
         g = bfphast.Graph.from_cch(cch, hbm_budget=budget)
         assert np.array_equal(g.isochrone_bitsets(org, thr)[0], want), budget - tile
+
+
+def test_graph_without_host_memory_for_panels(built, grid100):
+    """Building the tiles runs out of host memory on worker threads: the graph is
+    served without panels."""
+    import bfphast
+    _, cch = grid100
+    with _env("BF_TEST_FAIL_ALLOC", "panel_tiles"):
+        g = bfphast.Graph.from_cch(cch)
+    assert g.info()["device_bytes"] == _without_panels(cch).info()["device_bytes"]
+    src, tgt = (np.arange(k, cch["n"], 900, dtype=np.uint32) for k in (1, 5))
+    assert np.array_equal(g.matrix(src, tgt), orc.Cch.from_dict(cch).matrix(src, tgt)[0])
