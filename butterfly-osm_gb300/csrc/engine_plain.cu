@@ -165,6 +165,165 @@ __global__ void __launch_bounds__(UPWARD_WARPS * 32, 4)
 }
 #undef PN
 
+// Path node at path index idx of a warp's ancestor path held as runs of
+// consecutive ranks: lane r holds run r's first node (r_node) and first path
+// index (r_idx; ~0 on lanes past the last run). Called by all lanes.
+__device__ __forceinline__ uint32_t path_node(uint32_t idx, uint32_t r_node, uint32_t r_idx) {
+  uint32_t lo = 0;
+#pragma unroll
+  for (uint32_t b = 16; b; b >>= 1) {
+    const uint32_t c = __shfl_sync(0xFFFFFFFFu, r_idx, lo + b);
+    if (c <= idx) lo += b;
+  }
+  return __shfl_sync(0xFFFFFFFFu, r_node, lo) + (idx - __shfl_sync(0xFFFFFFFFu, r_idx, lo));
+}
+
+// Upward pass of graphs without panels (upward.cu's otherwise) for ancestor paths
+// of at most 32 runs (the common case: paths are chains of separator runs; the
+// country graph's have 12 on average and 21 at most). The same walk as k_upward_fast, with three changes that cut its
+// instructions per relaxation and raise occupancy:
+//   - the path's nodes are not stored: lane r keeps run r, and the node at a
+//     path index is found by a 5-step shuffle search (once per 32 steps for
+//     the UP-edge ranges, and in the output), so shared memory holds only the
+//     path distances (dcap words per warp: 10 blocks per SM instead of 5);
+//   - a node's UP edges are walked in exact 32-edge chunks (four loads issued
+//     before their relaxations) with 32-bit offsets, instead of groups of
+//     eight chunks with sentinel records;
+//   - the UP-edge ranges of the next 32 path nodes are loaded 32 steps
+//     ahead, so the range loads never stall a step.
+// Every UP edge u -> v has v on u's root path (elimination-tree ancestors),
+// so t = i + rec.x < D; the bound is still checked before each atomic.
+__global__ void __launch_bounds__(UPWARD_WARPS * 32, 10)
+    k_upward_runs(const uint32_t* __restrict__ src, uint32_t k, uint32_t threshold,
+                  const uint32_t* __restrict__ parent, const uint32_t* __restrict__ run_end,
+                  const uint32_t* __restrict__ depth, const uint64_t* __restrict__ up_off,
+                  const uint2* __restrict__ up_rec, const uint32_t* __restrict__ pos_of,
+                  uint32_t n, uint32_t* __restrict__ seed, uint32_t seed_stride,
+                  uint32_t* __restrict__ flag, uint32_t dcap, uint32_t* __restrict__ err,
+                  const uint32_t* __restrict__ lane_thr, const uint32_t* __restrict__ unit_cost,
+                  const uint32_t* __restrict__ unit_lane, uint32_t mode) {
+  extern __shared__ uint32_t smem[];
+  constexpr unsigned FULL = 0xFFFFFFFFu;
+  const uint32_t wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t w = blockIdx.x * UPWARD_WARPS + wib;
+  if (w >= k) return;
+  const uint32_t s = src[w];
+  if (s >= n) {
+    if (lane == 0) atomicOr(err, DEVERR_PATH);
+    return;
+  }
+  const uint32_t D = depth[s] + 1;
+  uint32_t* pd = smem + wib * dcap;
+  // the path as runs [x, run_end[x]], each continuing at the parent of its end
+  uint32_t r_node = 0, r_idx = 0xFFFFFFFFu;
+  {
+    uint32_t x = s, i = 0, r = 0;
+    for (; x != NONE && r < 32 && i < D; ++r) {
+      const uint32_t e = run_end[x];
+      if (e < x || e >= n) break;
+      if (lane == r) {
+        r_node = x;
+        r_idx = i;
+      }
+      i += e - x + 1;
+      x = parent[e];
+    }
+    if (x != NONE || i != D || D > dcap) {
+      if (lane == 0) atomicOr(err, DEVERR_PATH);
+      return;
+    }
+  }
+  const uint32_t c0 = unit_cost ? unit_cost[w] : 0u;
+  const uint32_t out_lane = unit_lane ? unit_lane[w] : w;
+  if (lane_thr) threshold = min(threshold, lane_thr[out_lane]);
+  const uint32_t thr1 = min(threshold, INF - 1);  // d must also be finite
+  for (uint32_t l = lane; l < D; l += 32) pd[l] = (l == 0) ? c0 : INF;
+  __syncwarp();
+  // UP-edge ranges of path nodes [j0, j0 + 32): lane l holds node j0 + l's
+  uint64_t cb, nb;
+  uint32_t cn, nn;
+  {
+    const uint32_t x = path_node(min(lane, D - 1), r_node, r_idx);
+    cb = up_off[x];
+    cn = lane < D ? (uint32_t)(up_off[x + 1] - cb) : 0u;
+    const uint32_t x2 = path_node(min(32 + lane, D - 1), r_node, r_idx);
+    nb = up_off[x2];
+    nn = 32 + lane < D ? (uint32_t)(up_off[x2 + 1] - nb) : 0u;
+  }
+  uint64_t b_cur = __shfl_sync(FULL, cb, 0);
+  uint32_t n_cur = __shfl_sync(FULL, cn, 0);
+  uint2 rec = lane < n_cur ? up_rec[b_cur + lane] : make_uint2(0, 0);
+  for (uint32_t i = 0; i < D; ++i) {
+    const uint32_t j = i + 1;
+    if ((j & 31) == 0) {
+      cb = nb;
+      cn = nn;
+      const uint32_t jn = j + 32 + lane;
+      const uint32_t x = path_node(min(jn, D - 1), r_node, r_idx);
+      if (j + 32 < D) {
+        nb = up_off[x];
+        nn = jn < D ? (uint32_t)(up_off[x + 1] - nb) : 0u;
+      } else {
+        nb = 0;
+        nn = 0;
+      }
+    }
+    const uint64_t b_nx = __shfl_sync(FULL, cb, j & 31);
+    const uint32_t n_nx = __shfl_sync(FULL, cn, j & 31);
+    const uint2 nrec = lane < n_nx ? up_rec[b_nx + lane] : make_uint2(0, 0);
+    const uint32_t d = *(volatile const uint32_t*)&pd[i];
+    if (d <= thr1) {
+      if (lane < n_cur) {
+        const uint32_t t = i + rec.x;
+        if (t < D) atomicMin(&pd[t], sat_add(d, rec.y));
+      }
+      const uint2* rp = up_rec + b_cur;
+      for (uint32_t c = 32 + lane; c < n_cur + lane; c += 128) {
+        uint2 r[4];
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q)
+          r[q] = c + q * 32 < n_cur ? rp[c + q * 32] : make_uint2(D, 0);
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+          const uint32_t t = i + r[q].x;
+          if (t < D) atomicMin(&pd[t], sat_add(d, r[q].y));
+        }
+      }
+    }
+    __syncwarp();
+    rec = nrec;
+    b_cur = b_nx;
+    n_cur = n_nx;
+  }
+  const uint32_t lt = lane_thr ? lane_thr[out_lane] : threshold;
+  if (mode == UPWARD_OUT_COMPACT) {
+    uint2* out = reinterpret_cast<uint2*>(seed);
+    for (uint32_t l0 = 0; l0 < D; l0 += 32) {
+      const uint32_t l = l0 + lane;
+      const uint32_t x = path_node(min(l, D - 1), r_node, r_idx);
+      if (l >= D) continue;
+      const uint32_t d = pd[l];
+      const uint32_t p = (d == INF || d > threshold) ? NONE : (pos_of ? pos_of[x] : x);
+      out[(size_t)(D - 1 - l) * seed_stride + w] = make_uint2(p, d);
+    }
+    return;
+  }
+  for (uint32_t l0 = 0; l0 < D; l0 += 32) {
+    const uint32_t l = l0 + lane;
+    const uint32_t x = path_node(min(l, D - 1), r_node, r_idx);
+    if (l >= D) continue;
+    const uint32_t d = pd[l];
+    if (d == INF || d > threshold) continue;
+    const uint32_t p = pos_of[x];
+    if (p == NONE) continue;
+    if (unit_lane) atomicMin(&seed[(size_t)p * seed_stride + out_lane], d);
+    else if (mode == UPWARD_OUT_SLAB16)  // every stored d is within its lane threshold (< 0xFFFF)
+      reinterpret_cast<uint16_t*>(seed)[(size_t)p * seed_stride + w] = (uint16_t)d;
+    else seed[(size_t)p * seed_stride + w] = d;
+    if (flag && d <= lt) atomicOr(&flag[p >> 5], 1u << (p & 31));
+  }
+}
+
 // Compact upward output -> slab: thread (w, i) writes entry i (counted from
 // the root) of source w's ancestor path into lane w of its row. Consecutive
 // threads are consecutive lanes, and near the root their rows coincide, so
@@ -466,6 +625,18 @@ bf_status launch_upward(Graph* g, const uint32_t* d_src, uint64_t k, uint32_t th
   if (upward_by_panels(g))
     return launch_upward_panels(g, d_src, k, threshold, pos_map, seed, stride, flag, st, lane_thr,
                                 unit_cost, unit_lane, mode);
+  const size_t runs_smem = (size_t)UPWARD_WARPS * dcap * 4;
+  if (g->max_runs <= 32 && runs_smem <= 100 * 1024) {
+    BF_CUDA(cudaFuncSetAttribute(k_upward_runs, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)runs_smem));
+    k_upward_runs<<<(unsigned)((k + UPWARD_WARPS - 1) / UPWARD_WARPS), UPWARD_WARPS * 32,
+                    runs_smem, st>>>(d_src, (uint32_t)k, threshold, g->d_parent, g->d_run_end,
+                                     g->d_depth, g->d_up_off, g->d_up_rec, pos_map, g->n, seed,
+                                     stride, flag, dcap, g->d_err, lane_thr, unit_cost,
+                                     unit_lane, mode);
+    BF_CUDA(cudaGetLastError());
+    return BF_OK;
+  }
   const size_t fast_smem = (size_t)UPWARD_WARPS * 2 * dcap * 4;
   if (fast_smem <= 200 * 1024) {
     BF_CUDA(cudaFuncSetAttribute(k_upward_fast<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
