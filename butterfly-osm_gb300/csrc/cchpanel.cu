@@ -223,9 +223,21 @@ __global__ void __launch_bounds__(CP_TILE * CP_TILE)
 }
 
 template <class T>
-cudaError_t put(T** d, const std::vector<T>& h) {
-  const cudaError_t e = cudaMalloc((void**)d, std::max<size_t>(h.size(), 1) * sizeof(T));
-  return e != cudaSuccess ? e : cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
+bf_status room_for(T** d, size_t m) {
+  if (test_fail_alloc("cch_panels") ||
+      cudaMalloc((void**)d, std::max<size_t>(m, 1) * sizeof(T)) != cudaSuccess) {
+    cudaGetLastError();
+    *d = nullptr;
+    return BF_ERR_OOM;
+  }
+  return BF_OK;
+}
+template <class T>
+bf_status put(T** d, const std::vector<T>& h) {
+  const bf_status rc = room_for(d, h.size());
+  if (rc) return rc;
+  BF_CUDA(cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
+  return BF_OK;
 }
 
 }  // namespace
@@ -237,11 +249,11 @@ void free_cch_panels(CchPanels& P) {
   P = CchPanels();
 }
 
-bf_status build_cch_panels(CchPanels& P, uint32_t n, const std::vector<uint64_t>& qo,
-                           const std::vector<uint32_t>& qt, const std::vector<uint8_t>& pf,
-                           const std::vector<uint32_t>& lev, uint32_t n_levels,
-                           const uint64_t* d_qo, const uint32_t* d_qt, const uint8_t* d_pf,
-                           uint64_t room, cudaStream_t s) {
+static bf_status make_cch_panels(CchPanels& P, uint32_t n, const std::vector<uint64_t>& qo,
+                                 const std::vector<uint32_t>& qt, const std::vector<uint8_t>& pf,
+                                 const std::vector<uint32_t>& lev, uint32_t n_levels,
+                                 const uint64_t* d_qo, const uint32_t* d_qt, const uint8_t* d_pf,
+                                 uint64_t room, cudaStream_t s) {
   // the first level whose apexes have CP_MIN candidates in the mean
   std::vector<uint64_t> cand(n_levels, 0), apexes(n_levels, 0);
   for (uint32_t m = 0; m < n; ++m) {
@@ -331,20 +343,34 @@ bf_status build_cch_panels(CchPanels& P, uint32_t n, const std::vector<uint64_t>
     P.lvl_solve.push_back(solve.size());
     P.lvl_push.push_back(push.size());
   }
-  BF_CUDA(put(&P.d_pan, pan));
-  BF_CUDA(put(&P.d_e0, e0));
-  BF_CUDA(put(&P.d_col, cols));
-  BF_CUDA(put(&P.d_ent, ent));
-  BF_CUDA(put(&P.d_solve, solve));
-  BF_CUDA(put(&P.d_push, push));
+  bf_status rc;
+  if ((rc = put(&P.d_pan, pan)) || (rc = put(&P.d_e0, e0)) || (rc = put(&P.d_col, cols)) ||
+      (rc = put(&P.d_ent, ent)) || (rc = put(&P.d_solve, solve)) || (rc = put(&P.d_push, push)) ||
+      (rc = room_for(&P.d_tgt, push.size() * CP_TILE * CP_TILE)))
+    return rc;
   BF_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // (the uploads, before `s`)
-  BF_CUDA(cudaMalloc(&P.d_tgt, std::max<size_t>(push.size(), 1) * CP_TILE * CP_TILE * 4));
   if (!push.empty())
     k_cp_targets<<<(unsigned)push.size(), CP_TILE * CP_TILE, 0, s>>>(P.d_pan, P.d_col, P.d_push,
                                                                      d_qo, d_qt, d_pf, P.d_tgt);
   BF_CUDA(cudaGetLastError());
   BF_CUDA(cudaStreamSynchronize(s));
   P.first_level = first;
+  return BF_OK;
+}
+
+bf_status build_cch_panels(CchPanels& P, uint32_t n, const std::vector<uint64_t>& qo,
+                           const std::vector<uint32_t>& qt, const std::vector<uint8_t>& pf,
+                           const std::vector<uint32_t>& lev, uint32_t n_levels,
+                           const uint64_t* d_qo, const uint32_t* d_qt, const uint8_t* d_pf,
+                           uint64_t room, cudaStream_t s) {
+  bf_status rc;
+  try {
+    rc = make_cch_panels(P, n, qo, qt, pf, lev, n_levels, d_qo, d_qt, d_pf, room, s);
+  } catch (const std::bad_alloc&) {
+    rc = BF_ERR_OOM;
+  }
+  if (rc != BF_ERR_OOM) return rc;
+  free_cch_panels(P);  // no room for them: left to the levels of apexes
   return BF_OK;
 }
 

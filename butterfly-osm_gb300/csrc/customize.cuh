@@ -51,8 +51,8 @@ struct CchPanels {
   uint32_t* d_tgt = nullptr;  // per push unit: T_* words of its 16 x 16 column pairs
 };
 
-// Builds the panels of the rows at or above the level the rule picks (none: P
-// stays empty). qo, qt, pf: pair rows; lev: levels; d_qo .. d_pf: their device
+// Builds the panels of the rows at or above the level the rule picks (none, or no
+// memory for them: P stays empty). qo, qt, pf: pair rows; lev: levels; d_qo .. d_pf: their device
 // copies; room: bytes the panels may take. Synchronises `s`.
 bf_status build_cch_panels(CchPanels& P, uint32_t n, const std::vector<uint64_t>& qo,
                            const std::vector<uint32_t>& qt, const std::vector<uint8_t>& pf,

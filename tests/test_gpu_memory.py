@@ -63,3 +63,16 @@ def test_graph_without_host_memory_for_panels(built, grid100):
     assert g.info()["device_bytes"] == _without_panels(cch).info()["device_bytes"]
     src, tgt = (np.arange(k, cch["n"], 900, dtype=np.uint32) for k in (1, 5))
     assert np.array_equal(g.matrix(src, tgt), orc.Cch.from_dict(cch).matrix(src, tgt)[0])
+
+
+def test_customization_without_room_for_panels(built):
+    import bfphast
+    from test_gpu_cch_panels import CASES, _topo
+    _, n, pairs = CASES["tree"]
+    rng = np.random.default_rng(1)
+    t = _topo(n, pairs, rng, 0.3)
+    with _env("BF_TEST_FAIL_ALLOC", "cch_panels"):
+        g = bfphast.Cch.from_oracle_topo(t)
+    up, dn = (rng.integers(0, 1000, len(x)).astype(np.uint32) for x in (t.up_mid, t.down_mid))
+    got, want = g.relax(up, dn, t.up_mid, t.down_mid), t.relax(up, dn)[:4]
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
