@@ -692,6 +692,10 @@ void free_panel_scratch(PanelScratch* s) {
 
 namespace {
 
+// Words of the live bitmap, even: two 64-bit counters lie behind it.
+size_t live_words(uint32_t n) { return (((size_t)n + 31) / 32 + 2) & ~(size_t)1; }
+constexpr size_t COUNT_WORDS = 8, COUNT_ERR = 6;
+
 template <class T>
 bf_status grow(T** p, size_t& cap, size_t need, Graph* g, bool slack) {
   if (need <= cap && *p) return BF_OK;
@@ -710,6 +714,42 @@ bf_status grow(T** p, size_t& cap, size_t need, Graph* g, bool slack) {
   }
   cap = m;
   g->device_bytes += m * sizeof(T);
+  return BF_OK;
+}
+
+// The graph-sized scratch of a context, all of it or none.
+bf_status make_scratch(Graph* g, Ctx& c) {
+  const Panels& P = g->panels;
+  const uint32_t W = (g->n + 31) / 32, PW = (P.n + 31) / 32, L = P.n_levels;
+  const size_t meta = (size_t)W + PW + 2, nb = (std::max(W, PW) + SCAN_BLOCK - 1) / SCAN_BLOCK;
+  PanelScratch* s = new (std::nothrow) PanelScratch();
+  if (!s) {
+    set_error("out of host memory");
+    return BF_ERR_OOM;
+  }
+  size_t cap[5] = {};
+  bf_status rc;
+  if ((rc = grow(&s->bits, cap[0], meta + 3 + L + 1, g, false)) ||
+      (rc = grow(&s->pre, cap[1], meta, g, false)) ||
+      (rc = grow(&s->bsum, cap[2], 2 * nb, g, false)) ||
+      (rc = grow(&s->live, cap[3], live_words(g->n) + COUNT_WORDS, g, false)) ||
+      (rc = test_fail_alloc("panel_schedule") ? BF_ERR_OOM : BF_OK) ||
+      (rc = grow(&s->list, cap[4], P.n, g, false))) {
+  } else if (cudaHostAlloc((void**)&s->h_counts, COUNT_WORDS * 4, cudaHostAllocDefault) !=
+                 cudaSuccess ||
+             cudaHostAlloc((void**)&s->h_back, ((size_t)L + 5) * 4, cudaHostAllocDefault) !=
+                 cudaSuccess) {
+    cudaGetLastError();
+    set_error("cannot allocate the schedule read-back buffers");
+    rc = BF_ERR_OOM;
+  }
+  for (size_t m : cap) s->bytes += m * 4;
+  if (rc) {
+    g->device_bytes -= s->bytes;
+    free_panel_scratch(s);
+    return rc;
+  }
+  c.ps = s;
   return BF_OK;
 }
 
@@ -732,10 +772,6 @@ void drop_panel_schedule(Graph* g, Ctx& c, Sched& sc) {
   sc.cap_pitem = sc.cap_prow = 0;
   sc.lvl_pan.clear();
 }
-
-// Words of the live bitmap, even: two 64-bit counters lie behind it.
-static size_t live_words(uint32_t n) { return (((size_t)n + 31) / 32 + 2) & ~(size_t)1; }
-constexpr size_t COUNT_WORDS = 8, COUNT_ERR = 6;
 
 bf_status start_counts(Graph* g, Ctx& c, Sched& sc, cudaStream_t st) {
   if (!sc.panel) {
@@ -798,43 +834,12 @@ bf_status build_schedule_panels(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_t
   const unsigned nb = (unsigned)((std::max(W, PW) + SCAN_BLOCK - 1) / SCAN_BLOCK);
   const size_t meta = (size_t)W + PW + 2;  // words of the two bitmaps
   bf_status rc;
-  if (!c.ps) {
-    c.ps = new (std::nothrow) PanelScratch();
-    if (!c.ps) {
-      set_error("out of host memory");
-      return BF_ERR_OOM;
-    }
-  }
+  if (!c.ps && (rc = make_scratch(g, c))) return rc;
   PanelScratch& s = *c.ps;
   // a count of the schedule before may still run (a call that failed midway)
   if (s.counting) {
     BF_CUDA(cudaStreamSynchronize(c.cnt));
     s.counting = false;
-  }
-  size_t none = 0;
-  if (!s.h_back) {
-    const uint64_t before = g->device_bytes;
-    if ((rc = grow(&s.bits, none = 0, meta + 3 + L + 1, g, false)) ||
-        (rc = grow(&s.pre, none = 0, meta, g, false)) ||
-        (rc = grow(&s.bsum, none = 0, 2 * (size_t)nb, g, false)) ||
-        (rc = grow(&s.live, none = 0, live_words(n) + COUNT_WORDS, g, false)) ||
-        (rc = grow(&s.list, none = 0, P.n, g, false)))
-      return rc;
-    s.bytes = g->device_bytes - before;
-    if (!s.h_counts && cudaHostAlloc((void**)&s.h_counts, COUNT_WORDS * 4,
-                                      cudaHostAllocDefault) != cudaSuccess) {
-      cudaGetLastError();
-      s.h_counts = nullptr;
-      set_error("cannot allocate the row-count read-back buffer");
-      return BF_ERR_OOM;
-    }
-    if (cudaHostAlloc((void**)&s.h_back, ((size_t)L + 5) * 4, cudaHostAllocDefault) !=
-        cudaSuccess) {
-      cudaGetLastError();
-      s.h_back = nullptr;
-      set_error("cannot allocate the schedule read-back buffer");
-      return BF_ERR_OOM;
-    }
   }
   if ((rc = grow(&sc.d_cidx, sc.cap_cidx, n, g, false)) ||
       (rc = grow(&sc.d_trow, sc.cap_t, T, g, true)))

@@ -76,3 +76,15 @@ def test_customization_without_room_for_panels(built):
     up, dn = (rng.integers(0, 1000, len(x)).astype(np.uint32) for x in (t.up_mid, t.down_mid))
     got, want = g.relax(up, dn, t.up_mid, t.down_mid), t.relax(up, dn)[:4]
     assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+def test_schedule_allocation_that_fails_is_given_back(built, country_small):
+    import bfphast
+    _, cch = country_small
+    rng = np.random.default_rng(1)
+    src, tgt = (rng.integers(0, cch["n"], k).astype(np.uint32) for k in (20, 300))
+    g, h = bfphast.Graph.from_cch(cch), bfphast.Graph.from_cch(cch)
+    for _ in range(2):
+        _fails("panel_schedule", lambda: g.matrix(src, tgt))
+    assert np.array_equal(g.matrix(src, tgt), h.matrix(src, tgt))
+    assert g.info()["device_bytes"] == h.info()["device_bytes"]
