@@ -586,9 +586,14 @@ bool test_fail_alloc(const char* what) {
 static bf_status plain_buffers(Graph* g, cudaStream_t st) {
   if (g->d_dist) return BF_OK;
   const size_t slab = (size_t)g->n * PLAIN_K * sizeof(uint32_t);
-  if (cudaMalloc(&g->d_dist, slab) != cudaSuccess || cudaMalloc(&g->d_seed, slab) != cudaSuccess ||
+  if (cudaMalloc(&g->d_dist, slab) != cudaSuccess || test_fail_alloc("plain_seeds") ||
+      cudaMalloc(&g->d_seed, slab) != cudaSuccess ||
       cudaMalloc(&g->d_flag, ((g->n + 31) / 32) * 4) != cudaSuccess) {
     cudaGetLastError();
+    for (uint32_t** q : {&g->d_dist, &g->d_seed, &g->d_flag}) {  // all of them or none
+      if (*q) cudaFree(*q);
+      *q = nullptr;
+    }
     set_error("cannot allocate the plain engine's distance slabs");
     return BF_ERR_OOM;
   }

@@ -88,3 +88,15 @@ def test_schedule_allocation_that_fails_is_given_back(built, country_small):
         _fails("panel_schedule", lambda: g.matrix(src, tgt))
     assert np.array_equal(g.matrix(src, tgt), h.matrix(src, tgt))
     assert g.info()["device_bytes"] == h.info()["device_bytes"]
+
+
+def test_plain_slabs_are_allocated_all_or_none(built, grid100):
+    """A call after one whose seed slab could not be allocated starts over."""
+    import bfphast
+    _, cch = grid100
+    g = bfphast.Graph.from_cch(cch)
+    g.set_engine(bfphast.ENGINE_PLAIN)
+    src, tgt = (np.arange(k, cch["n"], 900, dtype=np.uint32) for k in (1, 5))
+    for _ in range(2):
+        _fails("plain_seeds", lambda: g.matrix(src, tgt))
+    assert np.array_equal(g.matrix(src, tgt), orc.Cch.from_dict(cch).matrix(src, tgt)[0])
