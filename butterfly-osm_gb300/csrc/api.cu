@@ -688,6 +688,7 @@ bf_status bf_query_batch(bf_graph* h, const uint32_t* src, uint32_t k, uint32_t 
   if (cudaSetDevice(g->device) != cudaSuccess) return cuda_status(cudaGetLastError(), "cudaSetDevice");
   cudaStream_t s = g->stream;
   void* buf = nullptr;
+  const CallBufferTrim trim{g->ctx};
   const size_t out_bytes = (size_t)k * g->n * 4;
   if ((rc = call_buffer(g->ctx, out_bytes + k * 4, &buf))) return rc;
   uint32_t* d_out = static_cast<uint32_t*>(buf);
@@ -699,7 +700,6 @@ bf_status bf_query_batch(bf_graph* h, const uint32_t* src, uint32_t k, uint32_t 
   if ((rc = check_device_error(g, s))) return rc;
   BF_CUDA(cudaMemcpyAsync(dist_out, d_out, out_bytes, cudaMemcpyDeviceToHost, s));
   BF_CUDA(cudaStreamSynchronize(s));
-  trim_call_buffer(g->ctx);
   return BF_OK;
 }
 

@@ -611,6 +611,10 @@ bf_status hub_rows(Graph* g, Sched& sc, uint64_t row_bytes, cudaStream_t st, con
 // outside the budget, like the call's own allocations were).
 bf_status call_buffer(Ctx& c, size_t bytes, void** out);
 void trim_call_buffer(Ctx& c);
+struct CallBufferTrim {  // on every way out of the call
+  Ctx& c;
+  ~CallBufferTrim() { trim_call_buffer(c); }
+};
 uint64_t ctx_budget(Graph* g, Ctx& c);
 void free_ctx(Ctx& c);
 bf_status init_ctx(Ctx& c);

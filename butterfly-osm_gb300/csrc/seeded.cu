@@ -187,6 +187,7 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
   // device copies: [target offsets | target seeds {rank, part} | units | cells]
   static_assert(sizeof(bf_seed) == 8, "bf_seed is two u32");
   void* buf = nullptr;
+  const CallBufferTrim trim{c};
   if ((rc = call_buffer(c, (T + 1) * 8 + nt * 8 + ns * 12 + std::min<uint64_t>(wave, S) * T * 4,
                         &buf)))
     return rc;
@@ -229,7 +230,6 @@ bf_status matrix_seeded(Graph* g, Ctx& c, const bf_seed* src_seeds, const uint64
     BF_CUDA(cudaMemcpyAsync(out + s0 * T, d_out, kw * T * 4, cudaMemcpyDeviceToHost, s));
     BF_CUDA(cudaStreamSynchronize(s));  // units is rebuilt for the next wave
   }
-  trim_call_buffer(c);
   if ((rc = check_device_error(g, s))) return rc;
   if (st && (rc = finish_counts(c, sc))) return rc;
   // same-rank pairs belong to the caller's bucket engine (bucket_ch.rs:6786-6845)

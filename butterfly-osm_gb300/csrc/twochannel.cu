@@ -422,6 +422,7 @@ bf_status matrix_seeded_2ch(Graph* g, Ctx& c, const bf_seed2* src_seeds, const u
   // [target offsets | target seeds | units | times | lengths]
   const uint64_t out_cells = std::min<uint64_t>(wave, S) * T;
   void* buf = nullptr;
+  const CallBufferTrim trim{c};
   if ((rc = call_buffer(c, (T + 1) * 8 + nt * 12 + src_off[S] * 16 + out_cells * 8, &buf)))
     return rc;
   uint64_t* d_to = static_cast<uint64_t*>(buf);
@@ -476,7 +477,6 @@ bf_status matrix_seeded_2ch(Graph* g, Ctx& c, const bf_seed2* src_seeds, const u
     BF_CUDA(cudaMemcpyAsync(out_len + s0 * T, d_ol, kw * T * 4, cudaMemcpyDeviceToHost, s));
     BF_CUDA(cudaStreamSynchronize(s));  // units is rebuilt for the next wave
   }
-  trim_call_buffer(c);
   if ((rc = check_device_error(g, s))) return rc;
   if (st && (rc = finish_counts(c, sc))) return rc;
   // same-rank pairs belong to the caller's two-channel bucket engine

@@ -100,3 +100,34 @@ def test_plain_slabs_are_allocated_all_or_none(built, grid100):
     for _ in range(2):
         _fails("plain_seeds", lambda: g.matrix(src, tgt))
     assert np.array_equal(g.matrix(src, tgt), orc.Cch.from_dict(cch).matrix(src, tgt)[0])
+
+
+def _runs_graph(n, run=20):
+    """n ranks in runs of 20, each joined to the next three of its run."""
+    u = np.arange(n, dtype=np.int64)
+    up = np.concatenate([np.stack([v := u[(u % run) < run - k], v + k], 1) for k in (1, 2, 3)])
+    up = up[np.lexsort((up[:, 1], up[:, 0]))]
+    w = np.random.default_rng(2).integers(1, 100, (2, len(up))).astype(np.uint32)
+    o = np.lexsort((up[:, 0], up[:, 1]))
+    off = np.zeros((2, n + 1), np.uint64)
+    off[0, 1:] = np.cumsum(np.bincount(up[:, 0], minlength=n))
+    off[1, 1:] = np.cumsum(np.bincount(up[:, 1], minlength=n))
+    return dict(n=n, up_off=off[0], up_tgt=up[:, 1].astype(np.uint32), up_w=w[0],
+                down_off=off[1], down_tgt=up[o, 0].astype(np.uint32), down_w=w[1][o])
+
+
+def test_failed_call_keeps_no_large_buffer(built):
+    """A call's buffer above the kept size is given back when the call fails too."""
+    import torch
+
+    import bfphast
+    cch = _runs_graph(600_000)
+    g = bfphast.Graph.from_cch(cch)
+    src = np.arange(0, 128 * 4000, 4000, dtype=np.uint32)  # 307 MB of distances
+    one = g.query_batch(src[:1])
+    free = torch.cuda.mem_get_info()[0]
+    with _env("BF_TEST_WITHHOLD_ARRIVAL", "1"), pytest.raises(bfphast.BfError) as e:
+        g.query_batch(src)
+    assert e.value.status == bfphast.BF_ERR_TIMEOUT
+    assert free - torch.cuda.mem_get_info()[0] < 4 * cch["n"] * len(src) // 2
+    assert np.array_equal(g.query_batch(src[:1]), one)
