@@ -219,7 +219,7 @@ bf_status bf_graph_info_get(const bf_graph* h, bf_graph_info* o) {
   o->n_down = g.n_down;
   o->max_depth = g.max_depth;
   o->k_lanes = g.k_lanes;
-  o->device_bytes = g.device_bytes + g.panels.bytes;
+  o->device_bytes = g.device_bytes;
   return BF_OK;
 }
 

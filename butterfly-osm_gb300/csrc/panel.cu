@@ -286,6 +286,14 @@ static bf_status make_panels(Graph* g, const std::vector<uint32_t>& run_end,
     up_nw += ch[c].up_w.size();
   }
   if (std::max(nw, up_nw) >= 0xFFFFFFFFull || std::max(ns, up_ns) >= 0xFFFFFFFFull) return BF_OK;
+  // the graph's budget holds the panels beside what its calls take at least
+  // without them (the plain engine's two slabs, 32 lanes of every row, schedules
+  // of work items and their builder's scratch): else a budget that serves a call
+  // without panels would be too small with them
+  const uint64_t bytes = 56 * np + 6ull * n + n / 8 + 8ull * (g->n_levels + 1) + 6 * ns +
+                         12 * nw + 4 * (up_ns + up_nw) + (len ? 4 * (nw + up_nw) : 0) + 65536;
+  const uint64_t beside = n * (2ull * PLAIN_K * 4 + 32 * (len ? 8 : 4) + 128) + 40 * off[n];
+  if (g->device_bytes + bytes + beside > g->hbm_budget) return BF_OK;
   for (const Chunk& c : ch)
     for (const HostPanel& p : c.pan)
       if (p.nu >= MAX_SOURCES) return BF_OK;
@@ -387,13 +395,15 @@ static bf_status make_panels(Graph* g, const std::vector<uint32_t>& run_end,
     free_panels(P);
     return rc == BF_ERR_OOM ? BF_OK : rc;
   }
+  g->device_bytes += P.bytes;
   return BF_OK;
 }
 
 // Panels of the DOWN edges by target rank (in-edges of v: off, src, w; src > v)
 // and the UP edges by source rank (records {depth difference, w}), on runs given
 // by run_end. Leaves P empty (items and paths then serve every call) when the
-// tiles do not fit 32-bit offsets, the device or the host's memory.
+// tiles do not fit 32-bit offsets, the graph's budget, the device or the host's
+// memory.
 bf_status build_panels(Graph* g, const std::vector<uint32_t>& run_end,
                        const std::vector<uint32_t>& parent, const std::vector<uint32_t>& depth,
                        const std::vector<uint64_t>& off, const std::vector<uint32_t>& src,

@@ -105,8 +105,11 @@ typedef struct bf_config {
   uint32_t k_lanes;           /* lanes per batch for the batched engine (0 = autotune;
                                  16, 32, 64 or 128)                                */
   uint32_t flags;             /* BF_FLAG_* bits                                    */
-  uint64_t hbm_budget_bytes;  /* cap on device memory for distance slabs and
-                                 scratch (0 = 85% of free memory at creation)      */
+  uint64_t hbm_budget_bytes;  /* cap on device memory for the graph, distance slabs
+                                 and scratch (0 = 85% of free memory at creation);
+                                 where it does not hold the panels of the sweeps
+                                 beside them, the graph is created without (slower
+                                 calls, the same results)                          */
   uint32_t subtree_nodes;     /* max nodes of a shared-memory subtree (0 = auto)   */
   uint32_t reserved2;
 } bf_config;

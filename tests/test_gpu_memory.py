@@ -131,3 +131,90 @@ def test_failed_call_keeps_no_large_buffer(built):
     assert e.value.status == bfphast.BF_ERR_TIMEOUT
     assert free - torch.cuda.mem_get_info()[0] < 4 * cch["n"] * len(src) // 2
     assert np.array_equal(g.query_batch(src[:1]), one)
+
+
+def _served(make, want):
+    """Whether a graph's calls are served; a budget too small is BF_ERR_OOM."""
+    import bfphast
+    try:
+        g = make()
+        for call, w in want:
+            assert np.array_equal(call(g), w)
+    except bfphast.BfError as e:
+        assert e.status == bfphast.BF_ERR_OOM
+        return None
+    return g
+
+
+@pytest.mark.parametrize("two", [False, True])
+def test_budget_covers_panels(built, country_small, two):
+    """What a graph with a budget holds stays within it, its panels too, and no
+    budget that serves a call without panels is too small with them."""
+    import bfphast
+    _, cch = country_small
+    n = cch["n"]
+    c = orc.Cch.from_dict(cch)
+    rng = np.random.default_rng(2)
+    src = rng.integers(0, n, 40).astype(np.uint32)
+    tgt = rng.choice(n, 500, replace=False).astype(np.uint32)
+    thr = np.full(3, 9000, np.uint32)
+    kw = {}
+    want = [(lambda g: g.matrix(src, tgt), c.matrix(src, tgt)[0]),
+            (lambda g: g.isochrone_bitsets(src[:3], thr)[0], c.isochrone_bitsets(src[:3], thr)[0])]
+    if two:
+        ln = [np.where(cch[k] == INF, cch[k], cch[k] // 2 + 1) for k in ("up_w", "down_w")]
+        kw = dict(up_len=ln[0], down_len=ln[1])
+        sets = [[[(int(r), 1, 2)] for r in x[:40]] for x in (src, tgt)]
+        want.append((lambda g: g.matrix_seeded_2ch(*sets)[1],
+                     orc.table_phast_lopsided_2ch(c, *sets, INF, *ln)[1]))
+    with_panels = 0
+    last = False
+    for mb in list(range(12, 60, 2)) + list(range(64, 400, 16)):
+        budget = mb << 20
+        g = _served(lambda: bfphast.Graph.from_cch(cch, hbm_budget=budget, **kw), want)
+        h = _served(lambda: _without_panels(cch, hbm_budget=budget, **kw), want)
+        assert (g is not None) == (h is not None), mb
+        assert g is not None or not last, mb
+        last = g is not None
+        if g is None:
+            continue
+        assert g.info()["device_bytes"] <= budget, mb
+        fresh = bfphast.Graph.from_cch(cch, hbm_budget=budget, **kw).info()["device_bytes"]
+        with_panels += fresh > _without_panels(cch, hbm_budget=budget, **kw).info()["device_bytes"]
+    assert last and with_panels
+
+
+def test_serving_slot_budgets(built, country_small):
+    """Slots whose budget holds 32 lanes of the rows that reach a target but not
+    of the targets' ancestors sweep items; tables and isochrones, budgets from too
+    small to ample."""
+    import time
+
+    import bfphast
+    _, cch = country_small
+    n = cch["n"]
+    c = orc.Cch.from_dict(cch)
+    rng = np.random.default_rng(2)
+    src = rng.integers(0, n, 40).astype(np.uint32)
+    tgt = rng.choice(n, 500, replace=False).astype(np.uint32)
+    want, _ = c.matrix(src, tgt)
+    want_bits, _ = c.isochrone_bitsets(src[:1], np.array([9000], np.uint32))
+    g = bfphast.Graph.from_cch(cch)
+    served = []
+    for kb in list(range(600, 3000, 100)) + [8000, 20000, 64000]:
+        srv = bfphast.Server(g, hbm_budget=2 * kb << 10, slots=1)
+        t, out = srv.submit_matrix(src, tgt)
+        ti, bits = srv.submit_isochrone(int(src[0]), 9000)
+        done, t0 = {}, time.time()
+        while len(done) < 2 and time.time() - t0 < 60:
+            done.update({x["ticket"]: x["status"] for x in srv.poll(wait_ms=200)})
+        srv.close()
+        assert set(done.values()) <= {bfphast.BF_OK, bfphast.BF_ERR_OOM}, kb
+        if done[t] == bfphast.BF_OK:
+            assert np.array_equal(out, want), kb
+        if done[ti] == bfphast.BF_OK:
+            assert np.array_equal(bits, want_bits[0]), kb
+        served.append((done[t] == bfphast.BF_OK, done[ti] == bfphast.BF_OK))
+    for k in (0, 1):  # from some budget on
+        s = [x[k] for x in served]
+        assert s == sorted(s) and s[-1] and not s[0], (k, s)
