@@ -349,48 +349,50 @@ bf_status bf_autotune(bf_graph* h, const uint32_t* d_src, uint64_t S, const uint
       }
   double best_ms = 1e300;
   Tune best_t = saved;
-  for (const Tune& t : cands) {
+  uint32_t tried = 0;
+  // Times a candidate and keeps it where it is the fastest. A sweep over panels
+  // has its own blocks and no work items: of candidates that differ in those alone
+  // the first is timed, and the graph's settings of them stay.
+  std::vector<uint32_t> lanes_timed;
+  bool panel = false;
+  auto offer = [&](Tune t) -> bf_status {
+    ++tried;
+    if (panel &&
+        std::find(lanes_timed.begin(), lanes_timed.end(), t.max_lanes) != lanes_timed.end())
+      return BF_OK;
     g->tune = t;
     double sum = 0;
     for (uint32_t r = 0; r <= reps; ++r) {
       bf_stats st{};
-      rc = batched_matrix(g, g->ctx, d_src, S, d_tgt, T, BF_INF, out.as<uint32_t>(), s, &st);
-      if (rc == BF_OK) rc = check_device_error(g, s);
-      if (rc != BF_OK) {
+      if ((rc = batched_matrix(g, g->ctx, d_src, S, d_tgt, T, BF_INF, out.as<uint32_t>(), s, &st)) ||
+          (rc = check_device_error(g, s))) {
         g->tune = saved;
         return rc;
       }
       if (r) sum += st.upward_ms + st.downward_ms + st.extract_ms;
     }
-    const double ms = sum / reps;
-    if (ms < best_ms) {
-      best_ms = ms;
+    panel = g->ctx.sc.panel;
+    lanes_timed.push_back(t.max_lanes);
+    if (sum / reps < best_ms) {
+      best_ms = sum / reps;
       best_t = t;
+      if (panel) {
+        best_t.tpb = saved.tpb;
+        best_t.split = saved.split;
+        best_t.small_rows = saved.small_rows;
+        best_t.small_split = saved.small_split;
+      }
     }
-  }
+    return BF_OK;
+  };
+  for (const Tune& t : cands)
+    if ((rc = offer(t))) return rc;
   // second stage: short work items on the small top levels, on the winner
-  uint32_t tried = (uint32_t)cands.size();
   for (uint32_t rows : {0u, 1024u}) {
     Tune t = best_t;
     t.small_rows = rows;
     t.small_split = 8;
-    g->tune = t;
-    double sum = 0;
-    for (uint32_t r = 0; r <= reps; ++r) {
-      bf_stats st{};
-      rc = batched_matrix(g, g->ctx, d_src, S, d_tgt, T, BF_INF, out.as<uint32_t>(), s, &st);
-      if (rc == BF_OK) rc = check_device_error(g, s);
-      if (rc != BF_OK) {
-        g->tune = saved;
-        return rc;
-      }
-      if (r) sum += st.upward_ms + st.downward_ms + st.extract_ms;
-    }
-    ++tried;
-    if (sum / reps < best_ms) {
-      best_ms = sum / reps;
-      best_t = t;
-    }
+    if ((rc = offer(t))) return rc;
   }
   g->tune = best_t;
   *best = to_c(best_t);

@@ -127,11 +127,11 @@ bf_status build_schedule(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt, uin
   const uint32_t SPLIT = std::max<uint32_t>(1, g->tune.split);
   const uint32_t SMALL_ROWS = g->tune.small_rows;
   const uint32_t SMALL_SPLIT = std::max<uint32_t>(1, std::min(SPLIT, g->tune.small_split));
-  const uint64_t key = (all ? 0x9E3779B97F4A7C15ull : hash_targets(h_tgt, T)) ^
-                       ((uint64_t)SPLIT << 56) ^ ((uint64_t)SMALL_SPLIT << 48) ^
+  const uint64_t tkey = all ? 0x9E3779B97F4A7C15ull : hash_targets(h_tgt, T);
+  const uint64_t key = tkey ^ ((uint64_t)SPLIT << 56) ^ ((uint64_t)SMALL_SPLIT << 48) ^
                        ((uint64_t)SMALL_ROWS << 20);
-  // reuse only for the same split settings and exactly the same targets
-  if (sc.valid && sc.key == key && sc.T == T && (sc.panel || sc.fell_back) == panels &&
+  // reuse only for exactly the same targets and, of items, the same split settings
+  if (sc.valid && sc.key == (sc.panel ? tkey : key) && sc.T == T && (sc.panel || sc.fell_back) == panels &&
       (!panels || sc.words == words) &&
       (all || (sc.tgt.size() == T && (T == 0 || std::memcmp(sc.tgt.data(), h_tgt, T * 4) == 0)))) {
     ++sc.uses;
@@ -150,7 +150,7 @@ bf_status build_schedule(Graph* g, Ctx& c, Sched& sc, const uint32_t* h_tgt, uin
   sc.fell_back = false;
   sc.words = words;
   if (panels) {
-    bf_status s = build_schedule_panels(g, c, sc, h_tgt, d_tgt, T, key, st);
+    bf_status s = build_schedule_panels(g, c, sc, h_tgt, d_tgt, T, tkey, st);
     if (s) return s;
     // a budget that holds 32 lanes of the rows that reach a target, but not
     // of the somewhat more rows of the panels: sweep the former
