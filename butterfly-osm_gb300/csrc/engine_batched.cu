@@ -565,12 +565,13 @@ __global__ void __launch_bounds__(128)
 // Mark the slab rows of every origin's ancestor path (the rows the upward
 // pass will seed): one warp per origin, whole runs of consecutive ranks at once.
 __global__ void __launch_bounds__(128)
-    k_mark_paths(const uint32_t* __restrict__ orig, uint32_t k, const uint32_t* __restrict__ parent,
-                 const uint32_t* __restrict__ run_end, const uint32_t* __restrict__ cidx,
-                 uint32_t* __restrict__ seeded) {
+    k_mark_paths(const uint32_t* __restrict__ orig, uint32_t k, uint32_t n,
+                 const uint32_t* __restrict__ parent, const uint32_t* __restrict__ run_end,
+                 const uint32_t* __restrict__ cidx, uint32_t* __restrict__ seeded) {
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= k) return;
   uint32_t x = orig[w];
+  if (x >= n) return;  // (not a node: the upward pass reports it)
   for (uint32_t guard = 0; x != NONE && guard < (1u << 30); ++guard) {
     // ancestors are shared: once a run's first node is marked, the warp that
     // marked it covers the rest of this same path
@@ -914,7 +915,7 @@ void launch_extract_lanes(const uint32_t* slab, uint32_t Kp, const uint32_t* tro
 void launch_mark_paths(Graph* g, const uint32_t* d_src, uint64_t k, const uint32_t* cidx,
                        uint32_t* seeded, cudaStream_t st) {
   if (!k) return;
-  k_mark_paths<<<(unsigned)((k + 3) / 4), 128, 0, st>>>(d_src, (uint32_t)k, g->d_parent,
+  k_mark_paths<<<(unsigned)((k + 3) / 4), 128, 0, st>>>(d_src, (uint32_t)k, g->n, g->d_parent,
                                                         g->d_run_end, cidx, seeded);
 }
 

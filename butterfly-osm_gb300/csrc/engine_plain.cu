@@ -332,10 +332,14 @@ __global__ void __launch_bounds__(UPWARD_WARPS * 32, 10)
 // rank outside the restricted schedule).
 __global__ void __launch_bounds__(256)
     k_scatter_seeds(const uint2* __restrict__ cseed, uint32_t k, const uint32_t* __restrict__ src,
-                    const uint32_t* __restrict__ depth, uint32_t* __restrict__ slab, uint32_t Kp,
-                    uint32_t stride, uint32_t col0, const uint32_t* __restrict__ cidx) {
+                    uint32_t n, const uint32_t* __restrict__ depth, uint32_t* __restrict__ slab,
+                    uint32_t Kp, uint32_t stride, uint32_t col0,
+                    const uint32_t* __restrict__ cidx) {
   const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
-  if (w >= k || i > depth[src[w]]) return;
+  if (w >= k) return;
+  // (a source that is no node has no entries: the upward pass reported it)
+  const uint32_t s = src[w];
+  if (s >= n || i > depth[s]) return;
   const uint2 e = cseed[(size_t)i * stride + col0 + w];
   if (e.x == NONE) return;
   const uint32_t row = cidx ? cidx[e.x] : e.x;
@@ -609,8 +613,8 @@ bf_status launch_scatter_seeds(Graph* g, const void* cseed, uint64_t k, const ui
   if (!k) return BF_OK;
   dim3 grid((unsigned)((k + 255) / 256), g->max_depth + 1);
   k_scatter_seeds<<<grid, 256, 0, st>>>(reinterpret_cast<const uint2*>(cseed), (uint32_t)k, d_src,
-                                       g->d_depth, slab, Kp, (uint32_t)(stride ? stride : k),
-                                       (uint32_t)col0, cidx);
+                                       g->n, g->d_depth, slab, Kp,
+                                       (uint32_t)(stride ? stride : k), (uint32_t)col0, cidx);
   BF_CUDA(cudaGetLastError());
   return BF_OK;
 }
