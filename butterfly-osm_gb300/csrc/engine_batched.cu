@@ -1028,33 +1028,43 @@ bf_status batched_matrix(Graph* g, Ctx& c, const uint32_t* d_src, uint64_t S, co
     BF_CUDA(cudaEventRecord(c.join, c.aux));
     pre_launches = 1;
   }
+  // a call that ends before a wave waits for that pass: it still reads the
+  // caller's sources, and what it reports belongs to this call, not to the next
+  auto give_up = [&](bf_status rc) {
+    if (pre) {
+      const std::string why = bf_last_error();
+      cudaStreamSynchronize(c.aux);
+      if (check_device_error(g, st)) set_error(why);
+    }
+    return rc;
+  };
   std::vector<uint32_t> h_tgt(T);
   BF_CUDA(cudaMemcpyAsync(h_tgt.data(), d_tgt, T * 4, cudaMemcpyDeviceToHost, st));
   BF_CUDA(cudaStreamSynchronize(st));
   for (uint64_t i = 0; i < T; ++i)
     if (h_tgt[i] >= g->n) {
       set_error("targets[" + std::to_string(i) + "] is not a node of the graph");
-      return BF_ERR_INVALID;
+      return give_up(BF_ERR_INVALID);
     }
   const auto tb = std::chrono::steady_clock::now();
-  if ((s = build_schedule(g, c, c.sc, h_tgt.data(), T, false, st, d_tgt))) return s;
+  if ((s = build_schedule(g, c, c.sc, h_tgt.data(), T, false, st, d_tgt))) return give_up(s);
   if (stats)
     stats->schedule_ms +=
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tb).count();
   Sched& sc = c.sc;
-  if (stats && (s = start_counts(g, c, sc, st))) return s;
+  if (stats && (s = start_counts(g, c, sc, st))) return give_up(s);
   const uint64_t rows = std::max<uint32_t>(sc.n_r, 1);
   // lanes per wave: all sources if the slab fits the budget, else waves
   uint64_t max_lanes = ctx_budget(g, c) / (rows * 4);
   max_lanes = max_lanes >= 32 ? max_lanes & ~31ull : 0;
   if (max_lanes == 0) {
     set_error("HBM budget too small for one 32-lane wave of the restricted slab");
-    return BF_ERR_OOM;
+    return give_up(BF_ERR_OOM);
   }
   if (g->tune.max_lanes) max_lanes = std::min<uint64_t>(max_lanes, g->tune.max_lanes);
   const uint64_t wave = std::min<uint64_t>(max_lanes, (S + 3) & ~3ull);
   const uint32_t Kp = (uint32_t)((wave + 3) & ~3ull);
-  if ((s = ensure_slab(g, c, (size_t)rows * Kp * 4))) return s;
+  if ((s = ensure_slab(g, c, (size_t)rows * Kp * 4))) return give_up(s);
   uint64_t launches = pre_launches;
   // cells from the sweep's "unreachable" up become INF like those above the
   // threshold

@@ -44,3 +44,12 @@ def _last(x, bad):
 @pytest.mark.parametrize("engine", [1, 2])  # plain, batched
 def test_invalid_sources(built, grid100, S, overlap, engine):
     _check(grid100[1], S, engine, overlap, lambda s, t, bad: (_last(s, bad), t))
+
+
+@pytest.mark.parametrize("S", [1, 40, 3000])
+@pytest.mark.parametrize("overlap", [1, 0])
+@pytest.mark.parametrize("engine", [1, 2])
+def test_invalid_targets_beside_invalid_sources(built, grid100, S, overlap, engine):
+    """The targets end the call while the sources are still walked."""
+    _check(grid100[1], S, engine, overlap, lambda s, t, bad: (_last(s, bad), _last(t, bad)))
+    _check(grid100[1], S, engine, overlap, lambda s, t, bad: (s, _last(t, bad)))
