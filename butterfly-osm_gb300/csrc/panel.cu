@@ -1295,12 +1295,13 @@ __device__ __forceinline__ bool ring_unit(const uint4 m, RingSmem& sm, RingPos& 
 // labels, and a warp's work per row is one 8-byte shared load, the weights and
 // the add-mins. Bound by the integer pipe (an add-min per weight and lane, 64 a
 // cycle and SM: 4.9 ms for 10k x 10k on the country graph) and HBM (37 GB, 5.4
-// ms) together; a level of 4347 panels at 4000 lanes ran at 57 % of the first
-// and 60 % of the second. 10k x 10k sweep 14.4 -> 9.5 ms against a thread
-// that loads its own rows into registers; measured on the way: four warps of
-// four lanes a thread 11.3 ms (code for 64 labels misses the instruction
-// cache), groups of four rows 11.0, seeds as sources with one-hot weights 10.4,
-// scalar loads of the triangle 10.0.
+// ms: 32 GB of source rows and rows written, the rest seeded rows read back)
+// together; a level of 4347 panels at 4000 lanes ran at 57 % of the first and 60 %
+// of the second. 10k x 10k sweep 14.4 -> 9.5 ms against a thread that loads its
+// own rows into registers; measured on the way: four warps of four lanes a thread
+// 11.3 ms (code for 64 labels misses the instruction cache), groups of four rows
+// 11.0, seeds as sources with one-hot weights 10.4, scalar loads of the triangle
+// 10.0.
 template <bool SAT>
 __global__ void __launch_bounds__(32 * (RING_WARPS + 1), 3)
     k_sweep_panels_ring(const uint4* __restrict__ item, uint32_t i0, uint32_t n_item,

@@ -308,7 +308,9 @@ __device__ __forceinline__ void plain_small(const PlainArgs& g, uint32_t p) {
 // 849 -> 335 (348 with the staging before the arrival). A batch's sweep on the
 // 1000 x 1250 region 2.99 -> 1.36 ms, on the country graph 6.73 -> 4.58 (9.1 with
 // a warp for panels of up to four rows too). NARROW, eight sources: 0.93 and 2.73
-// ms there; one source on grid100, whole call: 546 -> 452 us (2250 by rows).
+// ms there; one source on grid100, whole call: 546 -> 452 us (2250 by rows). On
+// the region the schedulers issue in a fifth of the cycles: the warps wait at the
+// barriers and for rows.
 template <int PER_SM, bool NARROW>
 __global__ void __launch_bounds__(32 * PP_WARPS, PER_SM)
     k_plain_panels(const PlainArgs g, uint32_t* __restrict__ bar, long long timeout,
@@ -378,9 +380,9 @@ bf_status plain_sweep_panels(Graph* g, uint32_t k, uint32_t threshold, cudaStrea
                     P.absent, g->d_dist, g->d_seed, g->d_flag,  threshold};
   const bool hook = test_withhold_arrival();
   // a slab beyond L2: rows come from HBM, and more blocks hide that although
-  // their kernel spills (country graph 4.7 ms a batch against 5.45 with two an
-  // SM, the town 400 us a call against 361)
-  const bool wide = (uint64_t)g->n * PLAIN_K * 4 > (128ull << 20);
+  // their kernel spills more (630 bytes a thread against 160; country graph 4.7 ms
+  // a batch against 5.45 with two an SM, the town 400 us a call against 361)
+  const bool wide = (uint64_t)g->n * PLAIN_K * 4 > g->l2_bytes;
   const bool narrow = k <= 8;
   const auto kern = wide ? narrow ? k_plain_panels<4, true> : k_plain_panels<4, false>
                          : narrow ? k_plain_panels<2, true> : k_plain_panels<2, false>;

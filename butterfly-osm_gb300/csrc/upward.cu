@@ -14,7 +14,8 @@
 // bound by the chain of panels, many by the L2 reads of the tiles (64 bytes a
 // target and panel). Against the walk of single ranks: the wait for the pass of
 // 37 sources on the 1000 x 1250 region 0.16 -> 0.03 ms (it runs beside the
-// schedule's build), 10 000 sources on the country graph 2.1 -> 1.2 ms.
+// schedule's build), 10 000 sources on the country graph 2.07 -> 1.46 ms (the
+// kernel alone, cold).
 
 #include "engine.cuh"
 
