@@ -65,7 +65,8 @@ def parse():
                     help="plain-engine matrix side (sources = targets, K = 32)")
     ap.add_argument("--level-table", default="",
                     help="write the matrix schedule's per-level items / edges / rows (JSON) "
-                         "to this path, to attribute profiled sweep launches to levels")
+                         "to this path, to attribute profiled launches of a sweep of single "
+                         "rows to levels (a sweep over panels has fewer)")
     ap.add_argument("--isochrones", type=int, default=100000,
                     help="bulk isochrone origins (0 = skip)")
     ap.add_argument("--no-tiles", action="store_true",
@@ -583,9 +584,9 @@ def run_isochrones(g, cch, count, seed=42):
                          "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": None,
                          "peak_kind": peak_kind, "kernel": "k_iso_panels, k_iso_split (all waves)",
                          "alg_bytes": int(sweep_bytes), "sweep_ms": round(sweep_ms, 3),
-                         "bytes_rule": "per wave: 16 B per work item + 8 B per edge record "
-                                       "scanned, 2 B x lanes per active source row gathered "
-                                       "and per row written"},
+                         "bytes_rule": "per wave: 24 B per panel + 8 B per panel source "
+                                       "scanned, 128 B per active source row of a tile of "
+                                       "64 lanes gathered and per such row written"},
             "e2e": e2e,
             "bit_exact_sample": {"origins": len(pick), "equal": exact},
             "cpu_baseline": {"value": round(cpu_n / cpu_s, 2), "unit": "isochrones/s",
@@ -849,7 +850,7 @@ def run_customize(cch, steps, warmup, with_cpu):
            "target_index": info["target_index"], "steps": steps,
            "e2e": {"value": round(tot_ms, 3), "unit": "ms", "h2d_bytes_per_step": 4 * E,
                    "d2h_bytes_per_step": 16 * E},
-           "gpu_launches": info["levels"] + 4, "roofline": roof,
+           "roofline": roof,
            "bit_exact_vs_builder": exact}
     if with_cpu:
         threads = os.cpu_count() or 1
