@@ -1170,9 +1170,10 @@ bf_status isochrone_bitsets(Graph* g, Ctx& c, const uint32_t* d_orig, const uint
       BF_CUDA(cudaEventRecord(c.ev[3], st));
       // outside the timed phases: count the wave's algorithmic sweep bytes (the
       // panel form counts as it sweeps)
-      if (!panels) k_iso_count<<<(unsigned)std::min<uint64_t>((sc->n_items + 255) / 256, 152 * 8), 256, 0, st>>>(
-          (const uint4*)sc->d_item, sc->n_items, (const uint2*)sc->d_erec, d_active, Kp * lb,
-          reinterpret_cast<unsigned long long*>(c.d_count));
+      if (!panels && sc->n_items)
+        k_iso_count<<<(unsigned)std::min<uint64_t>((sc->n_items + 255) / 256, 152 * 8), 256, 0,
+                      st>>>((const uint4*)sc->d_item, sc->n_items, (const uint2*)sc->d_erec,
+                            d_active, Kp * lb, reinterpret_cast<unsigned long long*>(c.d_count));
       BF_CUDA(cudaGetLastError());
       BF_CUDA(cudaEventSynchronize(c.ev[3]));
       float ea, eb, ec;
