@@ -179,7 +179,7 @@ typedef struct bf_tune {
   uint32_t graph_capture;      /* replay the level schedule from a CUDA graph   */
   uint32_t lanes_per_wave;     /* 0 = as many lanes as the HBM budget allows     */
   double step_ms;              /* device time of the sample under this choice    */
-  uint32_t tried;              /* candidates timed by bf_autotune               */
+  uint32_t tried;              /* candidates compared by bf_autotune            */
   uint32_t isochrone_lanes;    /* origins per isochrone wave (0 = budget-limited;
                                   small waves keep the gated active set compact) */
   uint32_t small_level_rows;   /* levels with fewer rows than this use ...        */
@@ -218,7 +218,9 @@ typedef struct bf_tune {
 
 /* Time candidate tunables on a sample matrix (device buffers: d_sources,
  * d_targets) and keep the fastest for this graph; *best receives it. reps
- * timed repetitions per candidate (after one warm-up). */
+ * timed repetitions per candidate (after one warm-up). Candidates that a sweep
+ * over panels cannot tell apart (block size, work items) are timed as one, and
+ * those settings stay. */
 bf_status bf_autotune(bf_graph* g, const uint32_t* d_sources, uint64_t n_sources,
                       const uint32_t* d_targets, uint64_t n_targets, uint32_t reps,
                       bf_tune* best);
